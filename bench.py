@@ -655,19 +655,21 @@ def main():
 
     groups = sorted(W.sigma.keys()) if isinstance(W.sigma, dict) else [0]
     volterra = {str(gid): b.volterra_choice(gid) for gid in groups}
-    # own kernels launched per timed step, from the launch structure of one Dyson step per group:
-    # k_prep_problem, k_prep_group, k_mat_operator, k_zgemm (Matsubara part), ret, k_les_operands_t,
-    # k_zgemm (les*adv), k_tv, k_les_operands_t, k_zgemm (tv*vt), les; ret / les are two kernels
-    # (k_*_start + k_volterra_cl) on the cluster path and one otherwise.  A lattice step adds
-    # k_extrapolate, per corrector k_gloc + k_gloc_final + k_sigma_2b, and the final k-average.
-    per_group = [10 + (2 if v[0] == 100 else 1) + (2 if v[1] == 100 else 1) for v in volterra.values()]
+    # own kernels launched per timed step, from the launch structure of one Dyson step n of a group:
+    # k_prep_problem, k_prep_group, k_mat_operator, the Matsubara product, les*adv, k_tv,
+    # k_les_operands_t, tv*vt; ret and les: the start rows, a diagonal kernel per block of 128 // size1
+    # time rows and a trailing product between blocks.  A lattice step adds k_extrapolate, per corrector
+    # k_gloc + k_gloc_final + k_sigma_2b, and the final k-average.
+    def dyson_launches(n, s):
+        return 8 + 2 * (2 * ((n - k + 128 // s - 1) // (128 // s)))
     if W.lattice:
-        gpu_launches = (nt - k) * (1 + W.ncorr * (3 + sum(per_group)) + 2) * args.steps
+        gpu_launches = sum(1 + W.ncorr * (3 + dyson_launches(n, 1)) + 2 for n in range(k + 1, nt + 1)) * args.steps
     else:
-        nts = {}
+        top = {}
         for d in W.descs:
-            nts.setdefault(d.get("sigma_group", 0), []).append(d["nt"])
-        gpu_launches = sum((max(nts[int(g)]) - k) * c for g, c in zip(volterra.keys(), per_group)) * args.steps
+            g = d.get("sigma_group", 0)
+            top[g] = max(top.get(g, (0, 0)), (d["nt"], d["size1"]))
+        gpu_launches = sum(dyson_launches(n, s) for m, s in top.values() for n in range(k + 1, m + 1)) * args.steps
     mixed_err = None
     if args.mixed_error and args.precision == "mixed":
         mixed_err = compare_with_fp64(b, W, run_step, nt, k)

@@ -349,11 +349,9 @@ int nessi_gpu_gw_polarization_timestep(int tstp, int nk, const nessi_hm_ptrs *G,
 int nessi_gpu_gw_sigma_timestep(int tstp, int nk, const nessi_hm_ptrs *G, const nessi_hm_ptrs *W, const nessi_hm_ptrs *S,
                                 const double *w, int nt, int ntau, int size1, void *stream);
 
-/* Volterra kernels in use for a group: -1 = one problem per CTA, 2/4/8 = problems per CTA of the
- * tensor-core kernels, 100 = the group-wide blocked recursion by thread-block clusters (trailing
- * updates on the FP64 tensor cores), 0 = not chosen yet (the autotuner decides at the first eager
- * step with n >= max(min(128, nt), 3 nt / 4); the environment variable NESSI_VOLTERRA_PP read at
- * batch creation fixes the choice).  No reference counterpart. */
+/* Volterra kernels in use for a group: 102 = the blocked recursion (a diagonal kernel per block of
+ * 128 scalar rows, trailing updates on the FP64 tensor cores), the only form; ret and les alike.  No
+ * reference counterpart. */
 int nessi_gpu_get_volterra_choice(nessi_batch *b, int group, int *pp_ret, int *pp_les);
 
 /* ---- CUDA graphs of the per-step launch sequence ---------------------------------------------

@@ -5,12 +5,12 @@
 // One time step n > k runs as
 //   k_prep_problem   s x s inverses of the step matrices (dyson_impl :179-213, :693-706, :983-1011)
 //   k_prep_group     history coefficients for tv, dense copies of Sigma^< and Sigma^tv
-//   k_ret            G^R(n, 0..n): k-block start + Volterra recursion in t'   (:80-222)
+//   ret recursion    G^R(n, 0..n): k-block start + Volterra recursion in t'   (:80-222)
 //   k_tv             G^tv(n, 0..ntau): history stream + Matsubara integral + solve (:651-741)
 //   k_les_operands_t right-hand operands of the Sigma-shared products
-//   2 x k_zgemm      tv*vt + les*adv convolutions for all problems at once (conv_impl :1075-1394)
-//   k_les            G^<(0..n, n): k-block start + Volterra recursion in t (:893-1056)
-// The Volterra recursions also run group-wide (k_ret_start / k_les_start + k_volterra_cl).
+//   k_zgemm products     tv*vt + les*adv convolutions for all problems at once (conv_impl :1075-1394)
+//   les recursion    G^<(0..n, n): k-block start + Volterra recursion in t (:893-1056)
+// The recursions are in kernels_recursion.cuh.
 #pragma once
 #include "device_common.cuh"
 
@@ -38,6 +38,8 @@ struct GroupDev {
     double2 *Gmat_all; // ((ntau+1)s) x ldc: every problem's G^mat as columns
     double2 *Cmat;     // ((ntau+1)s) x ldc: Matsubara part of the tv right-hand side
     const double2 *fccmat;  // Fcc^mat of a VIE2 group (steepest-descent vie2_mat), or null
+    double2 *vy, *vacc;     // ((ntmax+1)s) x ldc: solved rows and far sums of the blocked recursion
+    const ProbDev *probs;   // the group's problems, nt descending
     int ntmax, ntau, s, sig, k;
     int ldc;           // >= nprob * s
     double h, beta;
@@ -564,13 +566,12 @@ __global__ void k_gmat_stack(GroupDev g, const ProbDev *__restrict__ probs) {
 }
 
 // ---------------------------------------------------------------------------------------
-// k_les_operands_t: right-hand operands of the Sigma-shared products (conv_impl :1075-1394)
-//   badv[(m,c)][(col,d)] = h w(n,m) G^R(n,m)^dagger[c][d],                 m = 0..n
+// k_les_operands_t: right-hand operand of the Sigma-shared product tv*vt (conv_impl :1075-1242)
 //   btv [(m,c)][(col,d)] = w(ntau,m) (-i dtau)(-sig) G^tv(n,ntau-m)^dagger[c][d]
-// badv / btv are row-major with the problems side by side in a row, so one problem's column is
-// a strided write; a CTA takes a tile of LOT problems x LOR time indices, reads each problem's
-// contiguous slice into shared memory and writes whole row segments (coalesced).
-//   which = 1: badv rows m = 0..n (from G^R(n, m)); which = 2: btv rows m = 0..ntau (from G^tv(n, .))
+// (badv[(m,c)][(col,d)] = h w(n,m) G^R(n,m)^dagger[c][d] comes from the retarded recursion).  btv is
+// row-major with the problems side by side in a row, so one problem's column is a strided write; a
+// CTA takes a tile of LOT problems x LOR time indices, reads each problem's contiguous slice into
+// shared memory and writes whole row segments (coalesced).
 // ---------------------------------------------------------------------------------------
 #define LOT 32
 template <int S> struct LoCfg {
@@ -578,33 +579,26 @@ template <int S> struct LoCfg {
 };
 
 template <int S>
-__global__ void __launch_bounds__(256) k_les_operands_t(GroupDev g, const ProbDev *__restrict__ probs, int n,
-                                                        int which, int nact) {
+__global__ void __launch_bounds__(256) k_les_operands_t(GroupDev g, const ProbDev *__restrict__ probs, int n, int nact) {
     constexpr int s2 = S * S, LOR = LoCfg<S>::LOR;
     __shared__ double2 buf[LOT * LOR * s2 + LOT];
     __shared__ const double2 *src[LOT];
     __shared__ int colid[LOT];
     const int k = g.k, ntau = g.ntau, M = ntau + 1;
-    const double h = g.h, dtau = g.beta / ntau;
+    const double dtau = g.beta / ntau;
     const long ldc = g.ldc;
     const int q0 = blockIdx.y * LOT, nq = min(LOT, nact - q0);
-    const int m0 = blockIdx.x * LOR, rows = which == 1 ? n + 1 : M, nm = min(LOR, rows - m0);
+    const int m0 = blockIdx.x * LOR, nm = min(LOR, M - m0);
     if (threadIdx.x < LOT) {
         const int q = threadIdx.x;
-        src[q] = q < nq ? (which == 1 ? probs[q0 + q].gret + tri(n) * s2 : probs[q0 + q].gtv + (long)n * s2 * M)
-                        : nullptr;
+        src[q] = q < nq ? probs[q0 + q].gtv + (long)n * s2 * M : nullptr;
         colid[q] = q < nq ? probs[q0 + q].col : 0;
     }
     __syncthreads();
-    // gather: buf[(q*LOR + mm)*s2 + e] = G element e of problem q at time index m0+mm
+    // gather: buf[(q*LOR + mm)*s2 + e] = G^tv element e of problem q at tau index ntau - (m0+mm)
     for (int i = threadIdx.x; i < nq * nm * s2; i += blockDim.x) {
-        if (which == 1) {
-            const int q = i / (nm * s2), rem = i % (nm * s2), mm = rem / s2, e = rem % s2;
-            buf[(q * LOR + mm) * s2 + e] = src[q][(long)(m0 + mm) * s2 + e];     // ret row n, contiguous
-        } else {
-            const int q = i / (nm * s2), rem = i % (nm * s2), e = rem / nm, mm = rem % nm;
-            buf[(q * LOR + mm) * s2 + e] = src[q][(long)e * M + (ntau - (m0 + mm))];  // tv planes
-        }
+        const int q = i / (nm * s2), rem = i % (nm * s2), e = rem / nm, mm = rem % nm;
+        buf[(q * LOR + mm) * s2 + e] = src[q][(long)e * M + (ntau - (m0 + mm))];  // tv planes
     }
     __syncthreads();
     // scatter: row (m, c), columns (col, d) of this tile
@@ -612,12 +606,7 @@ __global__ void __launch_bounds__(256) k_les_operands_t(GroupDev g, const ProbDe
         const int r = i / (nq * S), cc = i % (nq * S), mm = r / S, c = r % S, q = cc / S, d = cc % S;
         const int m = m0 + mm;
         const double2 v = cconj(buf[(q * LOR + mm) * s2 + d * S + c]);
-        const long dst = ((long)m * S + c) * ldc + (long)colid[q] * S + d;
-        if (which == 1) g.badv[dst] = cscale(v, h * greg_w(k, n, m));
-        else g.btv[dst] = cmul(cmk(0.0, dtau * (double)g.sig * greg_w(k, ntau, m)), v);
+        g.btv[((long)m * S + c) * ldc + (long)colid[q] * S + d] =
+            cmul(cmk(0.0, dtau * (double)g.sig * greg_w(k, ntau, m)), v);
     }
 }
-
-#include "kernels_volterra.cuh"
-#include "kernels_volterra_mp.cuh"
-#include "kernels_volterra_cl.cuh"

@@ -16,6 +16,7 @@
 
 #include "../../include/nessi_gpu.h"
 #include "kernels_dyson.cuh"
+#include "kernels_recursion.cuh"
 #include "kernels_tv_stream.cuh"
 #include "kernels_start.cuh"
 #include "kernels_mat.cuh"
@@ -131,11 +132,10 @@ struct Group {
     double2 *gloc_part = nullptr;    // partial sums of G_loc over chunks of problems
     long gloc_ld = 0;
     bool vie = false;                // VIE2 group: s* hold F, fcc* hold Fcc (nessi_gpu_set_F)
-    int pp_ret = 0, pp_les = 0;      // Volterra kernel chosen by the autotuner (0: not yet)
     double2 *fccret = nullptr, *fccles = nullptr;
     double2 *fccmat = nullptr;       // Fcc^mat of a VIE2 group (nessi_gpu_set_Fcc_mat; steepest descent)
     double2 *U = nullptr;            // diagonal interaction U(t), (ntmax+2) x s, t = -1 first
-    double2 *accr = nullptr, *accl = nullptr, *panel = nullptr;  // cluster Volterra path
+    double2 *vy = nullptr, *vacc = nullptr;  // blocked recursion: solved rows, far sums of the rows to come
     std::vector<int> members;        // problem indices, nt descending
     std::vector<ProbDev> h_probs;    // same order; col = position
     ProbDev *d_probs = nullptr;
@@ -165,11 +165,7 @@ struct nessi_batch {
     std::vector<Group> groups;
     std::vector<void *> allocs;
     long long bytes = 0;
-    // Volterra kernels for size1 <= 2: 0 (default) = chosen per group by the autotuner in
-    // volterra_step; -1 = the one-problem-per-CTA kernels k_ret / k_les, which overlap the next
-    // block's sums with the current block's solve; 1, 2, 4, 8 = problems per CTA of the tensor-core
-    // kernels k_ret_mp / k_les_mp, which read each shared Sigma tile once for all of them.
-    int volterra_pp = 0;
+    GroupDev *d_groups = nullptr;  // the groups' device descriptors, refreshed by sync_groups
     double2 *scratch = nullptr;  // G^tv in libcntr layout during layout conversion (size1 > 1)
     long scratch_n = 0;
     // kernel of the tv row: 1 (default) = k_tv (register loads, every size1), 0 = k_tv_stream
@@ -177,7 +173,6 @@ struct nessi_batch {
     int tv_kernel = 1;
     int nsm = 0;                        // SMs of the device
     int *d_err = nullptr;               // set by a device wait that gave up (NESSI_ERR_TIMEOUT)
-    unsigned *d_gbar = nullptr;         // grid barrier of k_volterra_grid: count, generation, abort
     long long wait_ns = 2000000000LL;   // bound of every mbarrier wait in the batch's kernels
 
     void prof_mark(int id, cudaStream_t st = nullptr) {
@@ -227,7 +222,17 @@ GroupDev group_dev(const Group &g) {
     d.fccmat = g.fccmat;
     d.ntmax = g.ntmax; d.ntau = g.ntau; d.s = g.s; d.sig = g.sig; d.k = g.k;
     d.ldc = g.ldc; d.h = g.h; d.beta = g.beta;
+    d.vy = g.vy; d.vacc = g.vacc; d.probs = g.d_probs;
     return d;
+}
+
+// The device table of the groups' descriptors, after any of their pointers changed
+int sync_groups(nessi_batch *b) {
+    std::vector<GroupDev> h;
+    for (const Group &g : b->groups) h.push_back(group_dev(g));
+    CK(cudaMemcpyAsync(b->d_groups, h.data(), h.size() * sizeof(GroupDev), cudaMemcpyHostToDevice, b->stream));
+    CK(cudaStreamSynchronize(b->stream));
+    return NESSI_OK;
 }
 
 int check_batch(nessi_batch *b) {
@@ -249,18 +254,6 @@ int find_group(nessi_batch *b, int user_id) {
 }
 
 // ---- per-size kernel launch table ----------------------------------------------------
-template <int S> size_t ret_smem(int k) {
-    size_t start = (size_t)(k * k * S * S + k * S * S + (k * S) * (k * S) + k * S * S) * 16 + 16;
-    size_t phase = (size_t)VolLayout<S>::total * 16;
-    return std::max(start, phase);
-}
-template <int S> size_t les_smem(int k) {
-    const int K1 = k + 1;  // the VIE2 start block has k+1 unknowns
-    size_t start = (size_t)((K1 * S) * (K1 * S) + K1 * S * S) * 16 + 16;
-    size_t phase = (size_t)VolLayout<S>::total * 16;
-    return std::max(start, phase);
-}
-
 // C (M x N) = A (M x K) B (K x N) on the repo's DMMA GEMM (kernels_gemm.cuh).
 template <int BM, int BN, class LA, class LB, class ST>
 int zgemm_launch_tiles(const LA &la, const LB &lb, const ST &st, int M, int N, int K, cudaStream_t s) {
@@ -273,11 +266,13 @@ int zgemm_launch_tiles(const LA &la, const LB &lb, const ST &st, int M, int N, i
 }
 // Long K, or too few 32 x 32 tiles for the 148 SMs: the k-split kernel; else the tiled one (both
 // sides measured at the kernels).
+bool zgemm_use_split(long M, long N, long K, int count = 1) {
+    return K >= 256 || ((M + 31) / 32) * ((N + 31) / 32) * count < 148;
+}
 template <class LA, class LB, class ST>
 int zgemm_launch(const LA &la, const LB &lb, const ST &st, int M, int N, int K, cudaStream_t s) {
     if (M <= 0 || N <= 0) return NESSI_OK;
-    const long tiles32 = (long)((M + 31) / 32) * ((N + 31) / 32);
-    if (K >= 256 || tiles32 < 148) {
+    if (zgemm_use_split(M, N, K)) {
         k_zgemm_split<<<dim3((unsigned)((N + 7) / 8), (unsigned)((M + 31) / 32)), 256, 0, s>>>(la, lb, st, K);
         CK(cudaGetLastError());
         return NESSI_OK;
@@ -285,243 +280,64 @@ int zgemm_launch(const LA &la, const LB &lb, const ST &st, int M, int N, int K, 
     return zgemm_launch_tiles<32, 32>(la, lb, st, M, N, K, s);
 }
 
-// Volterra choice code of the group-wide cluster path (k_ret_start / k_les_start + k_volterra_cl)
-#define NESSI_VOLTERRA_CLUSTER 100
-#define NESSI_VOLTERRA_GRID 101  // the blocked recursion by one cooperative launch over all SMs
-#define NESSI_CL 8  // CTAs per cluster (portable cluster size)
+// Volterra kernels reported by nessi_gpu_get_volterra_choice: the blocked recursion
+#define NESSI_VOLTERRA_BLOCKED 102
 
 template <int S> size_t ret_start_smem(int k) {
     return (size_t)(k * k * S * S + k * S * S + (k * S) * (k * S) + k * S * S) * 16 + 16;
 }
 template <int S> size_t les_start_smem(int k) {
-    const int K1 = k + 1;
+    const int K1 = k + 1;  // the VIE2 start block has k+1 unknowns
     return (size_t)((K1 * S) * (K1 * S) + K1 * S * S) * 16 + 16;
 }
 
-// Clusters of k_volterra_cl that can be resident at once (8 CTAs of one SM each must fit in a
-// GPC), asked once per instantiation; the recursion uses at most that many, so that no cluster
-// waits for another to finish.
-template <int S, bool VIE, bool RET, int BN> int max_active_clusters() {
-    static int cached = -1;
-    if (cached > 0) return cached;
-    const size_t sm = (size_t)std::max(ClSmem<S>::diag, ClGemm<BN>::smem) * sizeof(double2);
-    auto kern = k_volterra_cl<S, VIE, RET, BN>;
-    int num = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(NESSI_CL * 32));
-        cfg.blockDim = dim3(256);
-        cfg.dynamicSmemBytes = sm;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = NESSI_CL;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&num, kern, &cfg) != cudaSuccess) {
-            cudaGetLastError();  // a failed query leaves no error behind; the launch reports its own
-            num = 0;
-        }
-    } else {
-        cudaGetLastError();
+// One Volterra recursion (ret or les) of a step for the selected groups (same size1 and kind): the
+// start rows, then per block of VbCfg<S>::NBT time rows the diagonal kernel and the GEMM into the
+// later rows.  Columns per CTA of the diagonal kernel: as many as put one CTA on every SM, at most 8.
+template <int S, bool VIE, bool RET>
+int volterra_class(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) {
+    using C = VbCfg<S>;
+    int kmin = NESSI_K1MAX, kmax = 0, maxact = 0;
+    long cols = 0;
+    for (int i = 0; i < sel.ng; i++) {
+        kmin = std::min(kmin, b->groups[sel.gid[i]].k);
+        kmax = std::max(kmax, b->groups[sel.gid[i]].k);
+        maxact = std::max(maxact, sel.nact[i]);
+        cols += (long)sel.nact[i] * S;
     }
-    cached = num > 0 ? num : 16;
-    return cached;
-}
-
-template <int S, bool VIE, bool RET, int BN>
-int cluster_kernel_launch(const GroupDev &gd, const Group &g, int n, int nact, int PT, int ncl, double2 *acc,
-                          double2 *panel, cudaStream_t st) {
-    const size_t sm = (size_t)std::max(ClSmem<S>::diag, ClGemm<BN>::smem) * sizeof(double2);
-    auto kern = k_volterra_cl<S, VIE, RET, BN>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(NESSI_CL * ncl));
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = sm;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = NESSI_CL;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, kern, gd, (const ProbDev *)g.d_probs, n, nact, PT, acc, panel));
-    return NESSI_OK;
-}
-
-// Group-wide recursion: the start block of every problem (one CTA each), then the blocked
-// recursion by clusters of NESSI_CL CTAs, each owning PT problems (at most NESSI_CL x
-// ClCfg::DWMAX problems, one chain warp each).
-template <int S, bool VIE>
-int cluster_launch(const GroupDev &gd, const Group &g, int n, int nact, bool ret, cudaStream_t st) {
-    if (ret) {
-        const size_t sm = ret_start_smem<S>(gd.k);
+    const GroupDev *gt = b->d_groups;
+    if (RET) {
+        const size_t sm = ret_start_smem<S>(kmax);
         CK(cudaFuncSetAttribute(k_ret_start<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_ret_start<S, VIE><<<nact, 256, sm, st>>>(gd, g.d_probs, n);
+        k_ret_start<S, VIE><<<dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st>>>(gt, sel, n);
     } else {
-        const size_t sm = les_start_smem<S>(gd.k);
+        const size_t sm = les_start_smem<S>(kmax);
         CK(cudaFuncSetAttribute(k_les_start<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_les_start<S, VIE><<<nact, 256, sm, st>>>(gd, g.d_probs, n);
+        k_les_start<S, VIE><<<dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st>>>(gt, sel, n);
     }
     CK(cudaGetLastError());
-    if (n - gd.k <= 0) return NESSI_OK;  // no unknowns below / above the start block
-    // as many clusters as fit at once (about 16 on 148 SMs), each with PT problems
-    int nfit = ret ? max_active_clusters<S, VIE, true, 32>() : max_active_clusters<S, VIE, false, 32>();
-    if constexpr (S <= 2)
-        nfit = std::min(nfit, ret ? max_active_clusters<S, VIE, true, 64>() : max_active_clusters<S, VIE, false, 64>());
-    int PT = (nact + nfit - 1) / nfit;
-    PT = std::max(1, std::min(PT, NESSI_CL * ClCfg<S>::DWMAX));
-    const int ncl = (nact + PT - 1) / PT;
-    double2 *acc = ret ? g.accr : g.accl;
-    if constexpr (S <= 2) {
-        if (PT * S > 32) {
-            if (ret) return cluster_kernel_launch<S, VIE, true, 64>(gd, g, n, nact, PT, ncl, acc, g.panel, st);
-            return cluster_kernel_launch<S, VIE, false, 64>(gd, g, n, nact, PT, ncl, acc, g.panel, st);
-        }
-    }
-    if (ret) return cluster_kernel_launch<S, VIE, true, 32>(gd, g, n, nact, PT, ncl, acc, g.panel, st);
-    return cluster_kernel_launch<S, VIE, false, 32>(gd, g, n, nact, PT, ncl, acc, g.panel, st);
-}
-
-template <int S, bool VIE, bool RET, int BN>
-int grid_kernel_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, int p0, int np, double2 *acc,
-                       cudaStream_t st) {
-    const size_t sm = (size_t)std::max(ClSmem<S>::diag, ClGemm<BN>::smem) * sizeof(double2);
-    auto kern = k_volterra_grid<S, VIE, RET, BN>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    int per = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm));
-    if (per < 1) { set_err("k_volterra_grid: no CTA fits on an SM"); return NESSI_ERR_CUDA; }
-    // barrier words: arrival counter, generation, abort flag (cleared before every launch)
-    CK(cudaMemsetAsync(b->d_gbar, 0, 4 * sizeof(unsigned), st));
-    GridSync gs{b->d_gbar, b->d_gbar + 1, (int *)(b->d_gbar + 2), b->d_err, b->wait_ns};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)b->nsm);  // one CTA per SM, all resident (cooperative launch)
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = sm;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, kern, gd, (const ProbDev *)g.d_probs, n, p0, np, acc, g.panel, gs));
-    return NESSI_OK;
-}
-
-// Group-wide recursion by the whole GPU: the start block of every problem (one CTA each), then
-// the blocked recursion with every block's trailing GEMM over all SMs, in chunks of at most
-// nsm x ClCfg::DWMAX problems (one chain warp each).
-template <int S, bool VIE>
-int grid_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, int nact, bool ret, cudaStream_t st) {
-    if (ret) {
-        const size_t sm = ret_start_smem<S>(gd.k);
-        CK(cudaFuncSetAttribute(k_ret_start<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_ret_start<S, VIE><<<nact, 256, sm, st>>>(gd, g.d_probs, n);
-    } else {
-        const size_t sm = les_start_smem<S>(gd.k);
-        CK(cudaFuncSetAttribute(k_les_start<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_les_start<S, VIE><<<nact, 256, sm, st>>>(gd, g.d_probs, n);
-    }
-    CK(cudaGetLastError());
-    if (n - gd.k <= 0) return NESSI_OK;
-    double2 *acc = ret ? g.accr : g.accl;
-    const int chunk = b->nsm * ClCfg<S>::DWMAX;
-    for (int p0 = 0; p0 < nact; p0 += chunk) {
-        const int np = std::min(chunk, nact - p0);
-        if (np * S > 32) {
-            if (ret) CKR((grid_kernel_launch<S, VIE, true, 64>(b, gd, g, n, p0, np, acc, st)));
-            else CKR((grid_kernel_launch<S, VIE, false, 64>(b, gd, g, n, p0, np, acc, st)));
-        } else {
-            if (ret) CKR((grid_kernel_launch<S, VIE, true, 32>(b, gd, g, n, p0, np, acc, st)));
-            else CKR((grid_kernel_launch<S, VIE, false, 32>(b, gd, g, n, p0, np, acc, st)));
-        }
+    int wc = 1;
+    while (wc < C::WMAX && cols > (long)wc * b->nsm) wc *= 2;
+    const dim3 gd((unsigned)((maxact * S + wc - 1) / wc), (unsigned)sel.ng);
+    const size_t smb = (size_t)C::total * sizeof(double2);
+    CK(cudaFuncSetAttribute(k_vol_block<S, VIE, RET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
+    using P = zg::Pipe<32, 32, LdVolT<S, RET>, LdRowN>;
+    const size_t smt = (size_t)P::total * sizeof(double2);
+    CK(cudaFuncSetAttribute(k_vol_trail<S, RET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt));
+    const int nblk = (n - kmin + C::NBT - 1) / C::NBT;
+    for (int blk = 0; blk < nblk; blk++) {
+        k_vol_block<S, VIE, RET><<<gd, 256, smb, st>>>(gt, sel, n, blk, wc);
+        CK(cudaGetLastError());
+        const int M = (n - kmin - (blk + 1) * C::NBT) * S;  // rows after the block (largest group)
+        if (M <= 0) break;
+        const unsigned rt = (unsigned)((M + 31) / 32), N = (unsigned)(maxact * S);
+        if (zgemm_use_split(M, N, C::NR, sel.ng))
+            k_vol_trail_split<S, RET><<<dim3((N + 7) / 8, rt, (unsigned)sel.ng), 256, 0, st>>>(gt, sel, n, blk);
+        else
+            k_vol_trail<S, RET><<<dim3((N + 31) / 32, rt, (unsigned)sel.ng), 128, smt, st>>>(gt, sel, n, blk);
+        CK(cudaGetLastError());
     }
     return NESSI_OK;
-}
-
-// One Volterra recursion (ret or les) of a step: the one-problem kernels (pp = -1), the
-// multi-problem tensor-core kernels with pp problems per CTA (size1 <= 2), or the blocked
-// recursion by clusters (pp = NESSI_VOLTERRA_CLUSTER) or by the whole GPU (NESSI_VOLTERRA_GRID).
-template <int S, bool VIE> int volterra_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, int nact,
-                                               bool ret, int pp, cudaStream_t st) {
-    if (pp == NESSI_VOLTERRA_CLUSTER) return cluster_launch<S, VIE>(gd, g, n, nact, ret, st);
-    if (pp == NESSI_VOLTERRA_GRID) return grid_launch<S, VIE>(b, gd, g, n, nact, ret, st);
-    if constexpr (S <= 2) {
-        if (pp > 0) {
-            const size_t sm = (size_t)MpCfg<S>::total * sizeof(double2);
-            const unsigned grid = (unsigned)((nact + pp - 1) / pp);
-            if (ret) {
-                CK(cudaFuncSetAttribute(k_ret_mp<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                k_ret_mp<S, VIE><<<grid, MP_NW * 32, sm, st>>>(gd, g.d_probs, n, nact, pp);
-            } else {
-                CK(cudaFuncSetAttribute(k_les_mp<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                k_les_mp<S, VIE><<<grid, MP_NW * 32, sm, st>>>(gd, g.d_probs, n, nact, pp);
-            }
-            CK(cudaGetLastError());
-            return NESSI_OK;
-        }
-    }
-    const size_t sm = ret ? ret_smem<S>(gd.k) : les_smem<S>(gd.k);
-    if (ret) {
-        CK(cudaFuncSetAttribute(k_ret<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_ret<S, VIE><<<nact, 256, sm, st>>>(gd, g.d_probs, n);
-    } else {
-        CK(cudaFuncSetAttribute(k_les<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_les<S, VIE><<<nact, 256, sm, st>>>(gd, g.d_probs, n);
-    }
-    CK(cudaGetLastError());
-    return NESSI_OK;
-}
-
-// Autotuner of the Volterra kernels.  With volterra_pp = 0 (default), the first eager step of a
-// group with n >= the tuning step launches every candidate (one-problem kernels, for size1 <= 2
-// the multi-problem kernels with 2, 4, 8 problems per CTA, and the group-wide cluster recursion)
-// on the step itself -- each launch recomputes the same row / column from the same inputs, so the
-// last one leaves the step's result -- times them with CUDA events and keeps the fastest for the
-// group.  The tuning step is 3/4 of the group's longest history (at least min(128, ntmax)): the
-// cost of a step grows as n^2, so the late steps carry most of a propagation and the kernels'
-// ranking there is the one that counts.  Until then, and while a graph is being recorded, the
-// one-problem kernels run.
-template <int S, bool VIE> int volterra_step(nessi_batch *b, Group &g, const GroupDev &gd, int n, int nact, bool ret,
-                                             cudaStream_t st) {
-    int &choice = ret ? g.pp_ret : g.pp_les;
-    if (b->volterra_pp != 0) return volterra_launch<S, VIE>(b, gd, g, n, nact, ret, b->volterra_pp, st);
-    if (choice != 0) return volterra_launch<S, VIE>(b, gd, g, n, nact, ret, choice, st);
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cap));
-    const int tune_n = std::max(std::min(128, g.ntmax), (3 * g.ntmax) / 4);
-    if (cap != cudaStreamCaptureStatusNone || n < tune_n)
-        return volterra_launch<S, VIE>(b, gd, g, n, nact, ret, -1, st);
-    // candidates: one problem per CTA, the per-CTA tensor-core kernels (size1 <= 2), the cluster
-    // path; for size1 >= 3 also the whole-GPU path
-    const int cand_small[5] = {-1, 2, 4, 8, NESSI_VOLTERRA_CLUSTER};
-    const int cand_big[3] = {-1, NESSI_VOLTERRA_CLUSTER, NESSI_VOLTERRA_GRID};
-    const int *cand = S <= 2 ? cand_small : cand_big;
-    const int ncand = S <= 2 ? 5 : 3;
-    cudaEvent_t e0, e1;
-    CK(cudaEventCreate(&e0));
-    CK(cudaEventCreate(&e1));
-    float best = 1e30f;
-    int bestc = -1;
-    for (int pass = 0; pass < 2; pass++)  // the first pass warms up every variant
-        for (int ic = 0; ic < ncand; ic++) {
-            const int c = cand[ic];
-            CK(cudaEventRecord(e0, st));
-            CKR((volterra_launch<S, VIE>(b, gd, g, n, nact, ret, c, st)));
-            CK(cudaEventRecord(e1, st));
-            CK(cudaEventSynchronize(e1));
-            float ms = 0;
-            CK(cudaEventElapsedTime(&ms, e0, e1));
-            if (pass == 1 && ms < best) { best = ms; bestc = c; }
-        }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    choice = bestc;
-    return volterra_launch<S, VIE>(b, gd, g, n, nact, ret, choice, st);  // the kept variant writes last
 }
 
 // Decomposition of k_tv_stream: tau chunk width tw <= TWMAX chosen to balance the items
@@ -575,6 +391,10 @@ int tv_stream_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, 
 
 template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int nact) {
     const GroupDev gd = group_dev(g);
+    GroupSel sel;
+    sel.ng = 1;
+    sel.gid[0] = (int)(&g - b->groups.data());
+    sel.nact[0] = nact;
     cudaStream_t st = b->stream;
     const int k = g.k;
     // step-matrix inverses
@@ -623,14 +443,9 @@ template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int n
     CK(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
     {
         b->prof_mark(NESSI_KERNEL_RET, b->side);
-        CKR((volterra_step<S, VIE>(b, g, gd, n, nact, true, b->side)));
+        CKR((volterra_class<S, VIE, true>(b, sel, n, b->side)));
         // flops: every pair m > j of the row, an s x s complex product (8 s^3) per problem
         b->prof_end(NESSI_KERNEL_RET, 8.0 * S * S * S * (double)nact * tri_h(n), b->side);
-        b->prof_mark(NESSI_KERNEL_LES_OPERANDS, b->side);
-        dim3 grid((unsigned)((n + 1 + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR), (unsigned)((nact + LOT - 1) / LOT));
-        k_les_operands_t<S><<<grid, 256, 0, b->side>>>(gd, g.d_probs, n, 1, nact);
-        CK(cudaGetLastError());
-        b->prof_end(NESSI_KERNEL_LES_OPERANDS, 32.0 * S * S * (double)nact * (n + 1), b->side);
         b->prof_mark(NESSI_KERNEL_GEMM, b->side);
         CKR(zgemm_launch(LdRowK{g.Ldense, ldL, nn, nn}, LdRowN{g.badv, g.ldc, nn, m},
                          StRow{g.gles, g.ldc, nn, m, alpha, 0}, nn, m, nn, b->side));
@@ -663,7 +478,7 @@ template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int n
                                                                  (mixed ? 8.0 * M : 0.0)) + 16.0 * n));
         b->prof_mark(NESSI_KERNEL_LES_OPERANDS);
         dim3 grid2((unsigned)((g.ntau + 1 + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR), (unsigned)((nact + LOT - 1) / LOT));
-        k_les_operands_t<S><<<grid2, 256, 0, st>>>(gd, g.d_probs, n, 2, nact);
+        k_les_operands_t<S><<<grid2, 256, 0, st>>>(gd, g.d_probs, n, nact);
         CK(cudaGetLastError());
         b->prof_end(NESSI_KERNEL_LES_OPERANDS, 32.0 * S * S * (double)nact * (g.ntau + 1));
     }
@@ -680,7 +495,7 @@ template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int n
     // lesser column
     {
         b->prof_mark(NESSI_KERNEL_LES);
-        CKR((volterra_step<S, VIE>(b, g, gd, n, nact, false, st)));
+        CKR((volterra_class<S, VIE, false>(b, sel, n, st)));
         b->prof_end(NESSI_KERNEL_LES, 8.0 * S * S * S * (double)nact * tri_h(n));
     }
     return NESSI_OK;
@@ -879,12 +694,6 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
     g_live_batches++;
     b->device = g_device;
     b->precision = precision;
-    if (const char *v = getenv("NESSI_VOLTERRA_PP")) {
-        const int pp = atoi(v);
-        if (pp == -1 || pp == 0 || pp == 1 || pp == 2 || pp == 4 || pp == 8 || pp == NESSI_VOLTERRA_CLUSTER ||
-            pp == NESSI_VOLTERRA_GRID)
-            b->volterra_pp = pp;
-    }
     if (const char *v = getenv("NESSI_TV_KERNEL")) b->tv_kernel = strcmp(v, "stream") == 0 ? 0 : 1;
     auto fail = [&](int r) { nessi_gpu_batch_destroy(b); return r; };
     if (cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || b->nsm <= 0) {
@@ -899,13 +708,6 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
         }
         b->allocs.push_back(q);
         b->d_err = (int *)q;
-        q = nullptr;
-        if (cudaMalloc(&q, 4 * sizeof(unsigned)) != cudaSuccess || cudaMemset(q, 0, 4 * sizeof(unsigned)) != cudaSuccess) {
-            set_err("cudaMalloc of the grid barrier failed");
-            return fail(NESSI_ERR_OOM);
-        }
-        b->allocs.push_back(q);
-        b->d_gbar = (unsigned *)q;
     }
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
         set_err("stream creation failed");
@@ -978,8 +780,8 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
             (r = b->alloc(&g.tvcoef, N * s2)) || (r = b->alloc(&g.badv, N * S * g.ldc)) ||
             (r = b->alloc(&g.btv, M * S * g.ldc)) || (r = b->alloc(&g.gles, N * S * g.ldc)) ||
             (r = b->alloc(&g.Kmat, M * S * M * S)) || (r = b->alloc(&g.Gmat_all, M * S * g.ldc)) ||
-            (r = b->alloc(&g.Cmat, M * S * g.ldc)) || (r = b->alloc(&g.accr, N * S * g.ldc)) ||
-            (r = b->alloc(&g.accl, N * S * g.ldc)) || (r = b->alloc(&g.panel, (32 + NESSI_K1MAX) * S * g.ldc)))
+            (r = b->alloc(&g.Cmat, M * S * g.ldc)) || (r = b->alloc(&g.vy, N * S * g.ldc)) ||
+            (r = b->alloc(&g.vacc, N * S * g.ldc)))
             return fail(r);
         for (size_t c = 0; c < g.members.size(); c++) {
             const Prob &p = b->probs[g.members[c]];
@@ -1000,7 +802,14 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
             return fail(NESSI_ERR_CUDA);
         }
     }
-    if (cudaStreamSynchronize(b->stream) != cudaSuccess) { set_err("stream sync failed"); return fail(NESSI_ERR_CUDA); }
+    {
+        void *q = nullptr;
+        if (cudaMalloc(&q, b->groups.size() * sizeof(GroupDev)) != cudaSuccess) { set_err("cudaMalloc failed"); return fail(NESSI_ERR_OOM); }
+        b->allocs.push_back(q);
+        b->d_groups = (GroupDev *)q;
+        const int r = sync_groups(b);
+        if (r) return fail(r);
+    }
     *out = b;
     return NESSI_OK;
 }
@@ -1385,7 +1194,7 @@ static int ensure_fcc(nessi_batch *b, Group &g) {
     const long s2 = (long)g.s * g.s, N = g.ntmax + 1;
     CKR(b->alloc(&g.fccret, tri_h(N) * s2));
     CKR(b->alloc(&g.fccles, tri_h(N) * s2));
-    return NESSI_OK;
+    return sync_groups(b);
 }
 
 int nessi_gpu_set_F(nessi_batch *b, int group, const void *ret, const void *les, const void *tv, const void *mat,
@@ -1413,7 +1222,10 @@ int nessi_gpu_set_Fcc_mat(nessi_batch *b, int group, const void *cc_mat) {
     if (!cc_mat) { set_err("set_Fcc_mat: null Fcc^mat"); return NESSI_ERR_ARG; }
     CKR(ensure_fcc(b, *g));
     const long M = g->ntau + 1, s2 = (long)g->s * g->s;
-    if (!g->fccmat) CKR(b->alloc(&g->fccmat, M * s2));
+    if (!g->fccmat) {
+        CKR(b->alloc(&g->fccmat, M * s2));
+        CKR(sync_groups(b));
+    }
     CKR(copy_cplx(b, g->fccmat, cc_mat, M * s2, cudaMemcpyHostToDevice));
     CK(cudaStreamSynchronize(b->stream));
     return NESSI_OK;
@@ -1642,9 +1454,8 @@ int nessi_gpu_lattice_2b_timestep(nessi_batch *b, int n, int corrector_steps) {
 int nessi_gpu_get_volterra_choice(nessi_batch *b, int group, int *pp_ret, int *pp_les) {
     Group *g;
     CKR(find_group_checked(b, group, &g));
-    const int fixed = b->volterra_pp;
-    if (pp_ret) *pp_ret = fixed != 0 ? fixed : g->pp_ret;
-    if (pp_les) *pp_les = fixed != 0 ? fixed : g->pp_les;
+    if (pp_ret) *pp_ret = NESSI_VOLTERRA_BLOCKED;
+    if (pp_les) *pp_les = NESSI_VOLTERRA_BLOCKED;
     return NESSI_OK;
 }
 

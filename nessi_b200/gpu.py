@@ -296,7 +296,7 @@ class Batch:
         _check(load_library().nessi_gpu_graph_record(self._h, kind, n0, n1, corrector_steps))
 
     def volterra_choice(self, group=0):
-        """(ret, les) Volterra kernels of a group: -1 one problem per CTA, 2/4/8 problems per CTA."""
+        """(ret, les) Volterra kernels of a group: 102, the blocked recursion."""
         r, l = ctypes.c_int(), ctypes.c_int()
         _check(load_library().nessi_gpu_get_volterra_choice(self._h, group, ctypes.byref(r), ctypes.byref(l)))
         return r.value, l.value
