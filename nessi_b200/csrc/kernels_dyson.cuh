@@ -13,6 +13,7 @@
 // The recursions are in kernels_recursion.cuh.
 #pragma once
 #include "device_common.cuh"
+#include "kernels_gemm.cuh"
 
 struct ProbDev {
     double2 *gret, *gles, *gtv, *gmat;  // this problem's G (libcntr layout)
@@ -39,10 +40,18 @@ struct GroupDev {
     double2 *Cmat;     // ((ntau+1)s) x ldc: Matsubara part of the tv right-hand side
     const double2 *fccmat;  // Fcc^mat of a VIE2 group (steepest-descent vie2_mat), or null
     double2 *vy, *vacc;     // ((ntmax+1)s) x ldc: solved rows and far sums of the blocked recursion
+    double2 *vst;           // ((k+1)s) x ldc: its start rows
     const ProbDev *probs;   // the group's problems, nt descending
     int ntmax, ntau, s, sig, k;
     int ldc;           // >= nprob * s
     double h, beta;
+};
+
+#define NESSI_GSEL 64  // groups per launch
+// The groups of a launch (blockIdx.y or .z): index into the batch's group table, active problems
+struct GroupSel {
+    int ng;
+    int gid[NESSI_GSEL], nact[NESSI_GSEL];
 };
 
 __device__ __forceinline__ long tri(long t) { return t * (t + 1) / 2; }
@@ -366,28 +375,173 @@ __device__ void les_start_block(const GroupDev &g, const ProbDev &p, int n, cons
 }
 
 // ---------------------------------------------------------------------------------------
-// k_tv: G^tv(n, tau) for one problem and a tile of tau (dyson_impl :651-741):
+// The tv row: G^tv(n, tau) of every problem (dyson_impl :651-741):
 //   Q(tau) = sum_{j<n} a_j G^tv(j,tau) + dtau * matsubara_integral_2(Sigma^tv(n,.), G^mat)(tau)
 //   G^tv(n,tau) = Minv_les[n] Q(tau)
 // The Matsubara integral is linear in G^mat with an operator K_n built from Sigma^tv(n,.)
 // alone (k_mat_operator), so for a group sharing Sigma it is one GEMM over all problems
-// (Cmat = K_n Gmat_all); this kernel streams the history and adds Cmat.
-// Thread per (tau, column d); the history G^tv(0..n-1, tile) is streamed once.
+// (Cmat = K_n Gmat_all); these kernels stream the history and add Cmat.  Both work on the device
+// layout of G^tv: element planes, (t*s^2 + e)*(ntau+1) + tau, so a warp reading 32 consecutive tau
+// of one plane moves 512 contiguous bytes.
+// k_tv_ring (FP64 history) and k_tv_mixed (FP32 copy of the history).
 // ---------------------------------------------------------------------------------------
-// k_tv works on the device layout of G^tv: element planes, (t*s^2 + e)*(ntau+1) + tau, so a
-// warp reading 32 consecutive tau of one plane issues one contiguous 512-byte access.
+// k_tv_ring.  Bound: HBM, the history G^tv(0..n-1) once (size1 >= 6: the FP64 pipe, 8 s flops per
+// 16 bytes).  Persistent, one CTA of 16 warps per SM.  A work item is (problem, 32 tau, column d of
+// the s x s blocks); warp w takes rows j = w, w + 16, ...  Each warp keeps DEPTH plane rows of 512
+// bytes in flight in its own ring in shared memory: a lane copies its 16 bytes with cp.async and
+// reads only those, so the ring needs no barrier, and the copies of the next item are issued while
+// the current one is still summed.  The coefficients a_j, shared by all items of a group, are
+// double-buffered in shared memory and the next chunk waits in registers.  16 x 6 x 512 bytes in
+// flight per SM are enough for the full HBM rate; with 64 registers a thread the kernel holds half
+// of an SM's registers and a quarter of its shared memory, so that the retarded recursion runs
+// beside it (size1 4, 32 problems, n 1200: stream, recursion and les*adv together 3.2 ms, one after
+// the other 4.1 ms; size1 1, 1024 problems, n 1000: 2.6 and 2.8 ms).  Alone: size1 1, 2 6210, 5680
+// GB/s, size1 4 4260 (register loads, a CTA per 32 tau: 3900), size1 8 2060 (1270).  (Loads into registers go through L1 lines, which a shared-memory heavy neighbour takes
+// away: 6592 -> 5064 GB/s for size1 1 with the carve-out the recursion needs, and without it the two
+// kernels cannot share an SM at all.)
 template <int S> struct TvCfg {
+    static constexpr int NW = 16, NTH = NW * 32;                       // warps, threads per CTA
+    static constexpr int DEPTH = 6;                                    // plane rows in flight per warp
+    static constexpr int CHW = S == 1 ? 16 : (S == 2 ? 4 : (S == 3 ? 2 : 1));  // rows per warp and chunk
+    static constexpr int CH = CHW * NW, CE = CH * S * S;               // rows, complex of a chunk
+    static constexpr int CR = (CE + NTH - 1) / NTH;                    // complex a thread carries to the next
+    static constexpr int ring = 0, coef = NW * DEPTH * 32;             // shared memory (complex)
+    static constexpr int red = 8 * 32;                                 // partial sums (share the coefficients' place)
+    static constexpr int total = coef + (2 * CE > red ? 2 * CE : red);
+};
+__device__ __forceinline__ void cp16g(double2 *dst, const double2 *src) {  // past L1
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+// Grid (persistent CTAs, groups).  Copies are not predicated on tau: a lane past ntau reads the next
+// plane or the next row, and row n of every problem exists (n <= nt).
+template <int S, bool VIE>
+__global__ void __launch_bounds__(TvCfg<S>::NTH, 2) k_tv_ring(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
+    using C = TvCfg<S>;
+    constexpr int s2 = S * S, D = C::DEPTH;
+    extern __shared__ double2 rsm_[];
+    const GroupDev &g = gt[sel.gid[blockIdx.y]];
+    const int M = g.ntau + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
+    const long rowstride = (long)s2 * M;
+    const int ntile = (M + 31) / 32, items = sel.nact[blockIdx.y] * ntile * S;
+    if ((int)blockIdx.x >= items) return;
+    const int R = n > warp ? (n - warp + C::NW - 1) / C::NW : 0;  // rows of this warp per item
+    double2 *ring = rsm_ + C::ring + warp * D * 32 + lane, *cbuf = rsm_ + C::coef;
+    const double2 *cf = g.tvcoef;
+    // ---- the copy stream of this warp: planes b = 0..S-1 of its rows, item after item
+    auto item_base = [&](int it) {
+        return g.probs[it / (S * ntile)].gtv + (long)warp * rowstride + (long)(it % S) * M + (it / S) % ntile * 32 + lane;
+    };
+    int lit = blockIdx.x, lrow = 0, lb = 0, lslot = 0;
+    const double2 *lptr = R > 0 ? item_base(lit) : nullptr;
+    auto copy_next = [&]() {
+        if (lptr) {
+            cp16g(ring + lslot * 32, lptr);
+            if (S > 1 && lb < S - 1) {
+                lb++;
+                lptr += (long)S * M;
+            } else {
+                lb = 0;
+                lptr += C::NW * rowstride - (long)(S - 1) * S * M;
+                if (++lrow == R) {
+                    lrow = 0;
+                    lit += gridDim.x;
+                    lptr = lit < items ? item_base(lit) : nullptr;
+                }
+            }
+        }
+        lslot = lslot + 1 == D ? 0 : lslot + 1;
+        cp_commit();  // one group per plane row, empty past the end
+    };
+#pragma unroll 1
+    for (int q = 0; q < D; q++) copy_next();
+    int cslot = 0;
+    const int nch = (n + C::CH - 1) / C::CH;
+    auto coef_at = [&](int ch, int i) {  // complex i of this thread in chunk ch
+        const long e = (long)ch * C::CE + tid + (long)i * C::NTH;
+        return (tid + i * C::NTH < C::CE && e < (long)n * s2) ? __ldg(cf + e) : cmk(0, 0);
+    };
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        double2 acc[S], nx[C::CR];
+#pragma unroll
+        for (int a = 0; a < S; a++) acc[a] = cmk(0, 0);
+#pragma unroll
+        for (int i = 0; i < C::CR; i++) nx[i] = coef_at(0, i);
+        for (int ch = 0; ch < nch; ch++) {
+            double2 *cb = cbuf + (ch & 1) * C::CE;
+#pragma unroll
+            for (int i = 0; i < C::CR; i++)
+                if (tid + i * C::NTH < C::CE) cb[tid + i * C::NTH] = nx[i];
+            __syncthreads();  // chunk ch is in place; the other buffer was read before the last barrier
+            if (ch + 1 < nch)
+#pragma unroll
+                for (int i = 0; i < C::CR; i++) nx[i] = coef_at(ch + 1, i);
+            const int rows = min(C::CHW, R - ch * C::CHW);
+#pragma unroll 1
+            for (int r = 0; r < rows; r++) {
+                const double2 *cj = cb + (r * C::NW + warp) * s2;
+#pragma unroll
+                for (int b = 0; b < S; b++) {
+                    cp_wait<D - 1>();
+                    const double2 x = ring[cslot * 32];
+                    cslot = cslot + 1 == D ? 0 : cslot + 1;
+#pragma unroll
+                    for (int a = 0; a < S; a++) acc[a] = cfma(cj[a * S + b], x, acc[a]);
+                    copy_next();
+                }
+            }
+        }
+        // sum over the warps, in the place of the coefficients
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < S; a++)
+#pragma unroll
+            for (int half = 8; half > 0; half >>= 1) {
+                if (warp >= half && warp < 2 * half) cbuf[(warp - half) * 32 + lane] = acc[a];
+                __syncthreads();
+                if (warp < half) acc[a] = cadd(acc[a], cbuf[warp * 32 + lane]);
+                __syncthreads();
+            }
+        const int tau = (it / S) % ntile * 32 + lane, d = it % S;
+        if (warp == 0 && tau < M) {
+            const ProbDev &p = g.probs[it / (S * ntile)];
+            // Matsubara part dtau*[c2 + sig c1] from the group GEMM (k_mat_operator)
+            const double2 *cm = g.Cmat + (long)tau * S * g.ldc + (long)p.col * S + d;
+#pragma unroll
+            for (int a = 0; a < S; a++) acc[a] = cadd(acc[a], cm[(long)a * g.ldc]);
+            // VIE2 (vie2_timestep_tv, cntr_vie2_impl.hpp:645-725): a_j and Cmat carry the minus sign of
+            // the convolution; + Q^tv(n, tau) before the solve with (1 + h w0 F^R(n,n))^-1
+            if (VIE) {
+                const double2 *qt = p.qtv + (long)n * rowstride + tau;
+#pragma unroll
+                for (int a = 0; a < S; a++) acc[a] = cadd(acc[a], qt[(long)(a * S + d) * M]);
+            }
+            const double2 *mi = p.minv_les + (long)n * s2;
+#pragma unroll
+            for (int a = 0; a < S; a++) {
+                double2 x = cmk(0, 0);
+#pragma unroll
+                for (int b = 0; b < S; b++) x = cfma(mi[a * S + b], acc[b], x);
+                p.gtv[(long)n * rowstride + (long)(a * S + d) * M + tau] = x;
+            }
+        }
+    }
+    cp_wait<0>();
+}
+
+// k_tv_mixed: thread per (tau, column d), a CTA per 32 tau of a problem, 8 warps splitting the rows.
+template <int S> struct TvmCfg {
     static constexpr int DCH = S <= 2 ? S : (S <= 4 ? 2 : 1);  // block columns per pass
     static constexpr int NW = 8;                // warps per CTA, splitting the history sum over j
 };
 
-// MIXED: history rows j < n-k-1 are read from the FP32 copy (half the bytes); the k+1 rows
+// History rows j < n-k-1 are read from the FP32 copy (half the bytes); the k+1 rows
 // that carry the backward-difference terms, and all sums, stay in FP64.
 // VIE2 (vie2_timestep_tv, cntr_vie2_impl.hpp:645-725): a_j and Cmat carry the minus sign of
 // the convolution and Q^tv(n, tau) is added before the solve with (1 + h w0 F^R(n,n))^-1.
-template <int S, bool MIXED, bool VIE = false>
-__global__ void __launch_bounds__(256) k_tv(GroupDev g, const ProbDev *__restrict__ probs, int n) {
-    constexpr int s2 = S * S, DCH = TvCfg<S>::DCH, NW = TvCfg<S>::NW;
+template <int S, bool VIE = false>
+__global__ void __launch_bounds__(256) k_tv_mixed(GroupDev g, const ProbDev *__restrict__ probs, int n) {
+    constexpr int s2 = S * S, DCH = TvmCfg<S>::DCH, NW = TvmCfg<S>::NW;
     __shared__ double2 red[NW * 32 * S * DCH];
     const ProbDev p = probs[blockIdx.y];
     const int ntau = g.ntau, M = ntau + 1;
@@ -404,8 +558,8 @@ __global__ void __launch_bounds__(256) k_tv(GroupDev g, const ProbDev *__restric
         if (live) {
             const double2 *gb = p.gtv + tau;
             const double2 *cf = g.tvcoef;
-            const int j64 = MIXED ? (n - g.k - 1 > 0 ? n - g.k - 1 : 0) : 0;  // first FP64 row
-            if (MIXED) {
+            const int j64 = n - g.k - 1 > 0 ? n - g.k - 1 : 0;  // first FP64 row
+            {
                 const float2 *gb32 = p.gtv32 + tau;
                 // 8-byte loads: twice the rows in flight of the FP64 loop keep as many bytes in flight
 #pragma unroll 8
@@ -492,7 +646,7 @@ __global__ void __launch_bounds__(256) k_tv(GroupDev g, const ProbDev *__restric
 #pragma unroll
                     for (int b = 0; b < S; b++) x = cfma(mi[a * S + b], acc[b][c], x);
                     out[(long)(a * S + c0 + c) * M] = x;
-                    if (MIXED) p.gtv32[(long)n * rowstride + tau + (long)(a * S + c0 + c) * M] =
+                    p.gtv32[(long)n * rowstride + tau + (long)(a * S + c0 + c) * M] =
                         make_float2((float)x.x, (float)x.y);
                 }
         }

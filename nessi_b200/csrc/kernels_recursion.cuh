@@ -20,47 +20,55 @@
 // (integration.hpp:382-390, and the overlap rows k < i < 2k+2 below it).  So in the far field
 // (i - l > k) it is a_l, a factor of the column l, and the block's contribution to all later rows
 // is ONE complex GEMM over the group's columns (k_vol_trail, on the FP64 tensor cores) with the
-// columns stored as a_l Y_l (`vy`); the k rows next to a block get (a_{i-l} - 1) T(i, l) Y_l added
-// by the next diagonal kernel, which also adds the backward differences across the block edge.
+// columns stored as a_l Y_l (`vy`; the start rows 0..k first); the k rows next to a block get
+// (a_{i-l} - 1) T(i, l) Y_l added by the next diagonal kernel, which also adds the backward
+// differences across the block edge.
 //
-// k_vol_block, one launch per block: the CTA stages the block's triangle g h a_{i-l} T(i, l) (128
-// scalar rows, 130 KB) and the step inverses in shared memory; then one warp per column (p, d)
-// solves the 128 rows right-looking from registers: a lane holds 4 scalar rows (lane + 32 t), and
-// after a time row is solved every lane folds it into its own rows.  Per time row the critical path
-// is the solve with D_l, the broadcast and the update of the next row.  128 scalar rows: the widest
-// triangle that fits in shared memory, so that a step of n rows is n s / 128 launch pairs.
+// k_vol_block, one launch per block: the CTA stages the block's triangle a_{i-l} T(i, l) (128
+// scalar rows, 130 KB) and the step inverses in shared memory with asynchronous copies; then a warp
+// (s >= 3: four warps, a slot of 32 rows each) solves one or two columns (p, d), 128 rows
+// right-looking from registers: a lane holds scalar rows lane + 32 t of a column, and after a time
+// row is solved every lane folds it into its own rows.
+// Bound: the chain of 128 / s dependent rows; per row the solve with D_l, the broadcast and the update
+// of the next row (a dependent FP64 FMA takes 9 cycles, a shared-memory round trip 33), with the
+// triangle's column of the next row loaded one row ahead.  Two columns per warp share those loads.
+// 128 scalar rows: the widest triangle that fits in shared memory beside the tv stream's ring, so
+// that a step of n rows is n s / 128 launch pairs.  The kernels of a recursion are launched with
+// programmatic stream serialization: what does not depend on the solution (triangle, near block,
+// step inverses) is staged while the previous kernel still runs.
 //
-// Measured (ret + les of a step, ms; before = the best of the one-problem, multi-problem, cluster
-// and whole-GPU forms that this replaces, which solved blocks of 8-32 rows and either kept a whole
-// recursion on one SM or met at a barrier of all SMs 2 n s / 32 times): size1 2, 256 problems,
-// n 1000: 3.4 (with the tv stream beside the retarded half), before 5.3; size1 4, 32 problems,
-// n 1200: 5.7, before 13.2; sizes 1-8, 96 problems, n 600: 12.8, before 31; size1 2, 32 problems,
-// n 500 (VIE2): 0.63, before 1.27; size1 1, one problem, n 200: 0.13, before 0.14.
+// Measured on a B200, alone, ret + les of a step in us (blocks / trailing products / start rows):
+// size1 1, 1024 problems, n 1000: 853 (477 / 391 / 46); size1 2, 256 problems, n 1000: 1419 (688 /
+// 781 / 47); size1 4, 32 problems, n 1200: 2607 (1244 / 1456 / 81); size1 8, 18 problems, n 600: 3177
+// (1275 / 1626 / 226); size1 1, one problem, n 400: 141.  Synchronous staging, without the overlap of
+// launches, one warp per column for s >= 3: 957, 1842, 3774, 4175 and 238.
 #pragma once
-#include "kernels_gemm.cuh"
-
-#define NESSI_GSEL 64  // groups per launch
-// The groups of a launch (blockIdx.z, or .y): index into the batch's group table, active problems
-struct GroupSel {
-    int ng;
-    int gid[NESSI_GSEL], nact[NESSI_GSEL];
-};
+#include "kernels_dyson.cuh"
 
 template <int S> struct VbCfg {
-    static constexpr int NBT = 128 / S;              // time rows per block
+    static constexpr int TPS = 32 / S;               // time rows per slot (the 32 lanes of a warp)
+    static constexpr int SR = TPS * S;               // scalar rows per slot
+    static constexpr int NBT = 4 * TPS;              // time rows per block: four slots
     static constexpr int NR = NBT * S;               // scalar rows, at most 128
     static constexpr int NRP = NR | 1;               // odd stride of a column buffer
     static constexpr int TRI = S * S * (NBT * (NBT - 1) / 2);
     static constexpr int NEAR = NESSI_K1MAX * S;     // rows next to the block above, and their sources
-    static constexpr int WMAX = 8;                   // columns (chain warps) per CTA
-    static constexpr int SLOTS = (WMAX - 1 + S - 1) / S + 1;  // problems those columns can touch
-    // shared memory in double2: triangle, near block, near values, step inverses, columns, q of a row
-    static constexpr int near_ = TRI, ynear = near_ + NEAR * NEAR, dm = ynear + WMAX * NEAR, buf = dm + SLOTS * NR * S,
-                         qs = buf + WMAX * NRP, total = qs + WMAX * S;
-    static_assert(total * 16 <= 227 * 1024, "one CTA per SM");
+    // s <= 2: a warp solves one or two columns, all four slots; s >= 3: four warps per column, a slot each
+    static constexpr int NTH = S <= 4 ? 256 : 512, NW = NTH / 32, WMAX = S <= 2 ? 8 : NTH / 128, NC = S <= 2 ? 2 : 1;
+    // shared memory in double2: 32 of padding (unpredicated loads of solved rows), triangle, near
+    // block, then per column the near values, the column and (s >= 3) the row being solved, then the
+    // step inverses of the problems touched
+    static constexpr int coef = 32, near_ = coef + TRI, cols = near_ + NEAR * NEAR, QS = S >= 3 ? S : 0;
+    static __host__ __device__ constexpr int slots(int wc) { return (wc - 1 + S - 1) / S + 1 < wc ? (wc - 1 + S - 1) / S + 1 : wc; }
+    static __host__ __device__ constexpr int buf(int wc) { return cols + wc * NEAR; }
+    static __host__ __device__ constexpr int qs(int wc) { return buf(wc) + wc * NRP; }
+    static __host__ __device__ constexpr int dm(int wc) { return qs(wc) + wc * QS; }
+    static __host__ __device__ constexpr int total(int wc) { return dm(wc) + (S == 1 ? 0 : slots(wc) * NR * S); }
     // packed column-major triangle: column l (s scalar columns) holds rows (l+1) s .. NR-1
     static __device__ __forceinline__ int off(int l) { return S * (l * NR - S * (l * (l + 1) / 2)); }
 };
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // T(i, l)[a][b]
 template <int S, bool RET>
@@ -75,269 +83,314 @@ __device__ __forceinline__ double2 sub_ib(double2 acc, double b, double2 x) {
     return cmk(fma(b, x.y, acc.x), fma(-b, x.x, acc.y));
 }
 
-// One column of a block, solved by a warp: acc[t] = right-hand side of scalar row lane + 32 t on
-// entry.  xs (shared, NR): the solved rows on exit.  bdx[delta] = bd / h for delta <= k+1, else 0.
-template <int S, bool VIE>
-__device__ __forceinline__ void vol_chain(double2 *acc, const double2 *coef, const double2 *D, const double *bdx, int K1,
-                                          int nb, double2 *xs, double2 *qs, int lane) {
-    using C = VbCfg<S>;
-    if constexpr (S == 1) {
-        double2 Dr[4];
+// s <= 2: NC columns of a block, solved by a warp.  acc[c][t] = right-hand side of scalar row
+// lane + 32 t of column c on entry; xs (shared, stride NRP) receives the solved rows.  D: step
+// inverses (s = 1: registers, rows lane + 32 t; s = 2: shared).  bdp[32 + delta] = bd / h for
+// 1 <= delta <= k+1, else 0.  The accumulators of solved rows are not used again.
+template <bool VIE, int NC>
+__device__ __forceinline__ void vol_chain1(double2 (*acc)[4], const double2 *coef, double2 (*D)[4], const double *bdp,
+                                           double gh, int K1, int nb, double2 *xs, int lane) {
+    using C = VbCfg<1>;
+    const double2 *cl = coef - 1 + lane;  // column l: row lane + 32 t at cl[32 t]
+    double2 cv[4];
 #pragma unroll
-        for (int t = 0; t < 4; t++) Dr[t] = lane + 32 * t < nb ? D[lane + 32 * t] : cmk(0, 0);
+    for (int t = 0; t < 4; t++) cv[t] = t > 0 || lane > 0 ? cl[32 * t] : cmk(0, 0);
 #pragma unroll
-        for (int ph = 0; ph < 4; ph++) {
-            const int lend = min(nb, 32 * ph + 32);
-            for (int l = 32 * ph; l < lend; l++) {
-                const int ll = l - 32 * ph;
-                const double2 *cl = coef + C::off(l) - (l + 1);
-                double2 cv[4];
+    for (int ph = 0; ph < 4; ph++) {
+        const int lend = min(32, nb - 32 * ph);
+        const double *bp = bdp + 32 + lane;
+#pragma unroll 2
+        for (int ll = 0; ll < lend; ll++) {
+            const double b0 = VIE ? 0.0 : bp[-ll], b1 = VIE ? 0.0 : bp[32 - ll];
+            double2 nv[4];  // the next column of the triangle, one row ahead
+            cl += C::NR - 2 - (32 * ph + ll);
 #pragma unroll
-                for (int t = ph; t < 4; t++) cv[t] = (t > ph || lane > ll) ? cl[lane + 32 * t] : cmk(0, 0);
-                const double b0 = lane > ll ? bdx[lane - ll] : 0.0;
-                const double2 x = shfl2(cmul(Dr[ph], acc[ph]), ll);
-                if (lane > ll) {
-                    acc[ph] = cfma(cv[ph], x, acc[ph]);
-                    if (!VIE) acc[ph] = sub_ib(acc[ph], b0, x);
-                }
-                if (lane == ll) acc[ph] = x;
+            for (int t = ph; t < 4; t++) nv[t] = 32 * t + lane > 32 * ph + ll + 1 ? cl[32 * t] : cmk(0, 0);
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const double2 x = shfl2(cmul(D[c][ph], acc[c][ph]), ll), xg = cscale(x, gh);
+                if (lane == ll) xs[c * C::NRP + 32 * ph + ll] = x;
+                double2 u = acc[c][ph];
+                if (!VIE) u = sub_ib(u, b0, x);
+                acc[c][ph] = cfma(cv[ph], xg, u);
 #pragma unroll
                 for (int t = ph + 1; t < 4; t++) {
-                    acc[t] = cfma(cv[t], x, acc[t]);
-                    if (!VIE && t == ph + 1 && ll + K1 >= 32) acc[t] = sub_ib(acc[t], bdx[lane + 32 * t - l], x);
+                    if (!VIE && t == ph + 1 && ll + K1 >= 32) acc[c][t] = sub_ib(acc[c][t], b1, x);
+                    acc[c][t] = cfma(cv[t], xg, acc[c][t]);
                 }
             }
+#pragma unroll
+            for (int t = ph; t < 4; t++) cv[t] = nv[t];
         }
+    }
+}
+
+template <bool VIE, int NC>
+__device__ __forceinline__ void vol_chain2(double2 (*acc)[4], const double2 *coef, const double2 *D, const double *bdp,
+                                           double gh, int K1, int nb, double2 *xs, int lane) {
+    using C = VbCfg<2>;
+    const double2 *cl = coef - 2 + lane;  // column (l, 0): row lane + 32 t at cl[32 t]; (l, 1): len further
+    double2 u[4], v[4];
 #pragma unroll
-        for (int t = 0; t < 4; t++)
-            if (lane + 32 * t < nb) xs[lane + 32 * t] = acc[t];
-    } else if constexpr (S == 2) {
+    for (int t = 0; t < 4; t++) {
+        u[t] = t > 0 || lane > 1 ? cl[32 * t] : cmk(0, 0);
+        v[t] = t > 0 || lane > 1 ? cl[C::NR - 2 + 32 * t] : cmk(0, 0);
+    }
 #pragma unroll
-        for (int ph = 0; ph < 4; ph++) {
-            const int lend = min(nb, 16 * ph + 16);
-            for (int l = 16 * ph; l < lend; l++) {
-                const int src = 2 * (l - 16 * ph), len = C::NR - 2 * (l + 1);
-                const double2 *c0 = coef + C::off(l) - 2 * (l + 1), *c1 = c0 + len;
-                double2 u[4], v[4];
+    for (int ph = 0; ph < 4; ph++) {
+        const int lend = min(16, nb - 16 * ph);
+        const double *bp = bdp + 32 + (lane >> 1);
+#pragma unroll 1
+        for (int ll = 0; ll < lend; ll++) {
+            const int l = 16 * ph + ll, src = 2 * ll, len = C::NR - 2 * (l + 2);  // of the next column
+            const double b0 = VIE ? 0.0 : bp[-ll], b1 = VIE ? 0.0 : bp[16 - ll];
+            const double2 d00 = D[l * 4], d01 = D[l * 4 + 1], d10 = D[l * 4 + 2], d11 = D[l * 4 + 3];
+            double2 nu[4], nv[4];
+            cl += 2 * (C::NR - 2 * (l + 1)) - 2;
 #pragma unroll
-                for (int t = ph; t < 4; t++) {
-                    const bool in = t > ph || lane > src + 1;
-                    u[t] = in ? c0[lane + 32 * t] : cmk(0, 0);
-                    v[t] = in ? c1[lane + 32 * t] : cmk(0, 0);
-                }
-                const double2 d00 = D[l * 4], d01 = D[l * 4 + 1], d10 = D[l * 4 + 2], d11 = D[l * 4 + 3];
-                const double b0 = lane > src + 1 ? bdx[(lane >> 1) - (l - 16 * ph)] : 0.0;
-                const double2 q0 = shfl2(acc[ph], src), q1 = shfl2(acc[ph], src + 1);
+            for (int t = ph; t < 4; t++) {
+                const bool open = 32 * t + lane > 32 * ph + src + 3;
+                nu[t] = open ? cl[32 * t] : cmk(0, 0);
+                nv[t] = open ? cl[len + 32 * t] : cmk(0, 0);
+            }
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const double2 q0 = shfl2(acc[c][ph], src), q1 = shfl2(acc[c][ph], src + 1);
                 const double2 x0 = cfma(d01, q1, cmul(d00, q0)), x1 = cfma(d11, q1, cmul(d10, q0));
-                const double2 xa = (lane & 1) ? x1 : x0;
-                if (lane > src + 1) {
-                    acc[ph] = cfma(v[ph], x1, cfma(u[ph], x0, acc[ph]));
-                    if (!VIE) acc[ph] = sub_ib(acc[ph], b0, xa);
-                }
-                if ((lane & ~1) == src) acc[ph] = xa;
+                const double2 xa = (lane & 1) ? x1 : x0, g0 = cscale(x0, gh), g1 = cscale(x1, gh);
+                if ((lane & ~1) == src) xs[c * C::NRP + 32 * ph + lane] = xa;
+                double2 w = acc[c][ph];
+                if (!VIE) w = sub_ib(w, b0, xa);
+                acc[c][ph] = cfma(v[ph], g1, cfma(u[ph], g0, w));
 #pragma unroll
                 for (int t = ph + 1; t < 4; t++) {
-                    acc[t] = cfma(v[t], x1, cfma(u[t], x0, acc[t]));
-                    if (!VIE && t == ph + 1 && src / 2 + K1 >= 16)
-                        acc[t] = sub_ib(acc[t], bdx[((lane + 32 * t) >> 1) - l], xa);
+                    if (!VIE && t == ph + 1 && ll + K1 >= 16) acc[c][t] = sub_ib(acc[c][t], b1, xa);
+                    acc[c][t] = cfma(v[t], g1, cfma(u[t], g0, acc[c][t]));
                 }
             }
-        }
 #pragma unroll
-        for (int t = 0; t < 4; t++)
-            if (lane + 32 * t < 2 * nb) xs[lane + 32 * t] = acc[t];
-    } else {
-        for (int l = 0; l < nb; l++) {
-            const int r0 = l * S, r1 = r0 + S, len = C::NR - r1;
-            // the row's right-hand side to shared memory, x = D_l q by lanes 0..s-1, then all lanes
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int r = lane + 32 * t;
-                if (r >= r0 && r < r1) qs[r - r0] = acc[t];
-            }
-            __syncwarp();
-            if (lane < S) {
-                const double2 *dl = D + l * S * S + lane * S;
-                double2 xe = cmk(0, 0), xo = cmk(0, 0);
-#pragma unroll
-                for (int b = 0; b < S; b += 2) xe = cfma(dl[b], qs[b], xe);
-#pragma unroll
-                for (int b = 1; b < S; b += 2) xo = cfma(dl[b], qs[b], xo);
-                xs[r0 + lane] = cadd(xe, xo);
-            }
-            __syncwarp();
-            double2 x[S];
-#pragma unroll
-            for (int b = 0; b < S; b++) x[b] = xs[r0 + b];
-            const double2 *cl = coef + C::off(l) - r1;
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                if (32 * t + 31 < r1 || 32 * t >= C::NR) continue;  // no row of this slot is left
-                const int r = lane + 32 * t;
-                if (r >= r1 && r < C::NR) {
-                    double2 e = cmk(0, 0);
-#pragma unroll
-                    for (int b = 0; b < S; b += 2) acc[t] = cfma(cl[b * len + r], x[b], acc[t]);
-#pragma unroll
-                    for (int b = 1; b < S; b += 2) e = cfma(cl[b * len + r], x[b], e);
-                    acc[t] = cadd(acc[t], e);
-                    if (!VIE && r < r1 + K1 * S) acc[t] = sub_ib(acc[t], bdx[r / S - l], xs[r0 + r % S]);
-                }
+            for (int t = ph; t < 4; t++) {
+                u[t] = nu[t];
+                v[t] = nv[t];
             }
         }
     }
 }
 
-// Grid (ceil(columns / wc), groups), 256 threads; wc = 1, 2, 4 or 8 columns per CTA.
+// s >= 3: one column, solved by four warps, warp `slot` holding the SR scalar rows of its slot.  Per
+// time row the warp that owns it forms x = D_l q (lanes 0..s-1, q through shared memory) and
+// publishes it; one barrier of the warps still at work (named barrier `bar`), then every lane folds
+// it into its row.
+template <int S, bool VIE>
+__device__ __forceinline__ void vol_chain_big(double2 acc, const double2 *coef, const double2 *D, const double *bdp,
+                                              double gh, int nb, double2 *xs, double2 *qs, int slot, int lane, int bar) {
+    using C = VbCfg<S>;
+    const int row = slot * C::TPS + lane / S, ra = lane % S, r = slot * C::SR + lane;
+    const bool live = lane < C::SR;
+    const int lend = min(nb, (slot + 1) * C::TPS);
+#pragma unroll 1
+    for (int l = 0; l < lend; l++) {
+        const int r0 = l * S, len = C::NR - r0 - S, own = l / C::TPS;
+        const bool open = live && row > l;
+        const double2 *cl = coef + C::off(l) - r0 - S + r;
+        double2 cf[S];
+#pragma unroll
+        for (int b = 0; b < S; b++) cf[b] = open ? cl[b * len] : cmk(0, 0);
+        const double bw = VIE || !open ? 0.0 : bdp[32 + min(row - l, NESSI_K1MAX + 1)];
+        if (own == slot) {
+            double2 dv[S];
+            const double2 *dl = D + l * S * S + (lane < S ? lane : 0) * S;
+#pragma unroll
+            for (int b = 0; b < S; b++) dv[b] = dl[b];
+            if (live && row == l) qs[ra] = acc;
+            __syncwarp();
+            double2 xe = cmul(dv[0], qs[0]), xo = cmul(dv[1], qs[1]);
+#pragma unroll
+            for (int b = 2; b < S; b += 2) xe = cfma(dv[b], qs[b], xe);
+#pragma unroll
+            for (int b = 3; b < S; b += 2) xo = cfma(dv[b], qs[b], xo);
+            if (lane < S) xs[r0 + lane] = cadd(xe, xo);
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * (4 - own)) : "memory");
+        double2 e = acc, o = cmk(0, 0);
+        if (!VIE) e = sub_ib(e, bw, xs[r0 + ra]);
+#pragma unroll
+        for (int b = 0; b < S; b += 2) o = cfma(cf[b], cscale(xs[r0 + b], gh), o);
+#pragma unroll
+        for (int b = 1; b < S; b += 2) e = cfma(cf[b], cscale(xs[r0 + b], gh), e);
+        if (open) acc = cadd(e, o);
+    }
+}
+
+// Grid (ceil(columns / wc), groups), VbCfg<S>::NTH threads; wc = 1, 2, 4 or 8 columns per CTA (at most
+// WMAX), VbCfg<S>::total(wc) complex of dynamic shared memory.
 template <int S, bool VIE, bool RET>
-__global__ void __launch_bounds__(256) k_vol_block(const GroupDev *__restrict__ gt, GroupSel sel, int n, int blk, int wc) {
+__global__ void __launch_bounds__(VbCfg<S>::NTH, VbCfg<S>::NTH == 256 ? 2 : 1) k_vol_block(const GroupDev *__restrict__ gt, GroupSel sel, int n, int blk,
+                                                             int wc) {
     extern __shared__ double2 smem[];
     using C = VbCfg<S>;
-    constexpr int s2 = S * S, NR = C::NR;
-    __shared__ double bdx[C::NBT + 1], wdx[C::NBT + 1];  // bd(delta) / h (0 beyond k+1), a_delta
+    constexpr int s2 = S * S, NR = C::NR, NTH = C::NTH;
+    __shared__ double bdp[32 + C::NBT + 1], wdx[NESSI_K1MAX + 1];  // [32 + delta]: bd(delta) / h; a_delta
     const GroupDev &g = gt[sel.gid[blockIdx.y]];
     const int cols = sel.nact[blockIdx.y] * S, c0 = (int)blockIdx.x * wc;
     const int k = g.k, K1 = k + 1, i0 = K1 + blk * C::NBT, nb = min(C::NBT, n - i0 + 1);
     if (c0 >= cols || nb <= 0) return;
     const int ncol = min(wc, cols - c0), NRb = nb * S, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int lw = wc == 8 ? 3 : (wc == 4 ? 2 : (wc == 2 ? 1 : 0)), p0 = c0 / S;
+    const int nc = wc == 8 ? C::NC : 1;  // columns per warp (s <= 2): two share the loads of the triangle
     const double h = g.h, gh = VIE ? -h : h;
     const long ldc = g.ldc;
     const ProbDev *probs = g.probs;
-    double2 *coef = smem, *near_ = smem + C::near_, *ynear = smem + C::ynear, *dm = smem + C::dm, *buf = smem + C::buf;
-    for (int e = tid; e <= C::NBT; e += 256) {
-        bdx[e] = e <= K1 ? bd_w(k, e) / h : 0.0;
-        wdx[e] = e <= k ? greg_omega(k, e) : 1.0;
-    }
-    __syncthreads();
-    // ---- operands that do not depend on the solution: triangle, near block, step inverses
+    double2 *coef = smem + C::coef, *near_ = smem + C::near_, *ynear = smem + C::cols, *dm = smem + C::dm(wc),
+            *buf = smem + C::buf(wc);
+    pdl_trigger();
+    // ---- operands that do not depend on the solution, all copies in flight at once: triangle, near
+    //      block, step inverses
     if (RET) {  // memory is contiguous along the rows of a column
-        for (int l = warp; l < nb - 1; l += 8)
+        for (int l = warp; l < nb - 1; l += C::NW)
             for (int b = 0; b < S; b++) {
-                double2 v[4];
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    const int r = (l + 1) * S + lane + 32 * t;
-                    if (r < NRb) v[t] = *vol_t<S, RET>(g, n, i0 + r / S, i0 + l, r % S, b);
-                }
+                double2 *dst = coef + C::off(l) + b * (NR - (l + 1) * S);
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
                     const int x = lane + 32 * t, r = (l + 1) * S + x;
-                    if (r < NRb) coef[C::off(l) + b * (NR - (l + 1) * S) + x] = cscale(v[t], gh * wdx[r / S - l]);
+                    if (r < NRb) cp16(dst + x, vol_t<S, RET>(g, n, i0 + r / S, i0 + l, r % S, b));
                 }
             }
     } else {  // memory is contiguous along the columns of a row
-        for (int r = S + warp; r < NRb; r += 8) {
+        for (int r = S + warp; r < NRb; r += C::NW) {
             const int rt = r / S, a = r % S;
-            double2 v[4];
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int x = lane + 32 * t;
-                if (x < rt * S) v[t] = *vol_t<S, RET>(g, n, i0 + rt, i0 + x / S, a, x % S);
-            }
 #pragma unroll
             for (int t = 0; t < 4; t++) {
                 const int x = lane + 32 * t, l = x / S, b = x % S;
-                if (x < rt * S) coef[C::off(l) + b * (NR - (l + 1) * S) + r - (l + 1) * S] = cscale(v[t], gh * wdx[rt - l]);
+                if (x < rt * S)
+                    cp16(coef + C::off(l) + b * (NR - (l + 1) * S) + r - (l + 1) * S, vol_t<S, RET>(g, n, i0 + rt, i0 + l, a, b));
             }
         }
     }
-    if (blk > 0)
-        for (int e = tid; e < K1 * S * K1 * S; e += 256) {
-            const int x = RET ? e / (K1 * S) : e % (K1 * S), r = RET ? e % (K1 * S) : e / (K1 * S);
-            const int rt = r / S, l = x / S, delta = rt + K1 - l;
-            double2 v = cmk(0, 0);
-            if (r < NRb && delta <= k)
-                v = cscale(*vol_t<S, RET>(g, n, i0 + rt, i0 - K1 + l, r % S, x % S), gh * (wdx[delta] - 1.0));
-            near_[x * C::NEAR + r] = v;
-        }
-    for (int q = p0; q <= (c0 + ncol - 1) / S; q++) {
-        const double2 *mi = RET ? probs[q].minv_ret : probs[q].minv_les;
-        for (int e = tid; e < nb * s2; e += 256) {
-            const int l = e / s2, a = (e % s2) / S, b = e % S;
-            dm[(q - p0) * NR * S + (RET ? l * s2 + b * S + a : e)] = mi[(long)(RET ? n - i0 - l : i0 + l) * s2 + a * S + b];
+    for (int e = tid; e < K1 * S * K1 * S; e += NTH) {
+        const int x = RET ? e / (K1 * S) : e % (K1 * S), r = RET ? e % (K1 * S) : e / (K1 * S);
+        const bool in = r < NRb && r / S + K1 - x / S <= k;
+        cp16(near_ + x * C::NEAR + r, in ? vol_t<S, RET>(g, n, i0 + r / S, i0 - K1 + x / S, r % S, x % S) : nullptr);
+    }
+    double2 Dr[C::NC][4];  // s = 1: the step inverses of the warp's columns
+    if constexpr (S == 1) {
+#pragma unroll
+        for (int c = 0; c < C::NC; c++)
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int q = c0 + warp * nc + c, i = i0 + lane + 32 * t;
+                Dr[c][t] = cmk(0, 0);
+                if (warp * nc + c < ncol && c < nc && i <= n) Dr[c][t] = RET ? probs[q].minv_ret[n - i] : probs[q].minv_les[i];
+            }
+    } else {
+        for (int q = p0; q <= (c0 + ncol - 1) / S; q++) {
+            const double2 *mi = RET ? probs[q].minv_ret : probs[q].minv_les;
+            for (int e = tid; e < nb * s2; e += NTH) {
+                const int l = e / s2, a = (e % s2) / S, b = e % S;
+                cp16(dm + (q - p0) * NR * S + (RET ? l * s2 + b * S + a : e), mi + (long)(RET ? n - i0 - l : i0 + l) * s2 + a * S + b);
+            }
         }
     }
-    // ---- right-hand sides: q_i + g h (far sum of the blocks above)
-    for (int e = tid; e < NRb << lw; e += 256) {
-        const int w = e & (wc - 1), r = e >> lw, i = i0 + r / S, a = r % S, c = c0 + w;
-        if (w >= ncol) continue;
-        double2 v = cmk(0, 0);
-        if (!RET) v = __ldcg(g.gles + ((long)i * S + a) * ldc + c);
-        if (VIE) {
-            const ProbDev &p = probs[c / S];
-            v = cadd(v, RET ? p.qret[(tri(n) + n - i) * s2 + (c % S) * S + a] : p.qles[(tri(n) + i) * s2 + a * S + c % S]);
-        }
-        if (blk > 0) {
-            const double2 far = __ldcg(g.vacc + ((long)i * S + a) * ldc + c);
-            v = cmk(fma(gh, far.x, v.x), fma(gh, far.y, v.y));
-        }
-        buf[w * C::NRP + r] = v;
-    }
-    if (blk > 0)
-        for (int e = tid; e < (K1 * S) << lw; e += 256) {
-            const int w = e & (wc - 1), x = e >> lw;
-            if (w < ncol) ynear[w * C::NEAR + x] = __ldcg(g.vy + ((long)(i0 - K1) * S + x) * ldc + c0 + w);
-        }
+    cp_commit();
+    for (int e = tid; e < 32 + C::NBT + 1; e += NTH) bdp[e] = e > 32 && e - 32 <= K1 ? bd_w(k, e - 32) / h : 0.0;
+    if (tid <= NESSI_K1MAX) wdx[tid] = tid <= k ? greg_omega(k, tid) : 1.0;
+    cp_wait<0>();
     __syncthreads();
-    if (warp < ncol) {
-        const int c = c0 + warp, d = c % S;
-        double2 *xs = buf + warp * C::NRP;
-        double2 acc[4];
+    // weights: a_delta on the k rows below the diagonal, g h (a_delta - 1) on the near block
+    for (int l = warp; l < nb - 1; l += C::NW) {
+        const int len = NR - (l + 1) * S;
+        double2 *col = coef + C::off(l);
+        for (int b = 0; b < S; b++)
+            for (int x = lane; x < k * S; x += 32)
+                if ((l + 1) * S + x < NRb) col[b * len + x] = cscale(col[b * len + x], wdx[x / S + 1]);
+    }
+    for (int e = tid; e < K1 * S * K1 * S; e += NTH) {
+        const int x = e / (K1 * S), r = e % (K1 * S), delta = r / S + K1 - x / S;
+        if (delta <= k) near_[x * C::NEAR + r] = cscale(near_[x * C::NEAR + r], gh * (wdx[delta] - 1.0));
+    }
+    pdl_wait();  // from here on the results of the kernels before
+    // ---- right-hand sides: q_i + g h (far sum of the rows above)
+    constexpr int RI = (NR * C::WMAX + NTH - 1) / NTH;
+    {
+        double2 far[RI], q[RI];
 #pragma unroll
-        for (int t = 0; t < 4; t++) acc[t] = lane + 32 * t < NRb ? xs[lane + 32 * t] : cmk(0, 0);
-        __syncwarp();
-        if (blk > 0) {
-            const double2 *y = ynear + warp * C::NEAR;
-#pragma unroll
-            for (int t = 0; t < (C::NEAR + 31) / 32; t++) {
-                const int r = lane + 32 * t;
-                if (r >= K1 * S || r >= NRb) continue;
-                for (int x = (r / S) * S; x < K1 * S; x++) acc[t] = cfma(near_[x * C::NEAR + r], y[x], acc[t]);
-                if (!VIE)
-                    for (int l = r / S; l < K1; l++) acc[t] = sub_ib(acc[t], bdx[r / S + K1 - l], y[l * S + r % S]);
-            }
-        } else {
-            // the start rows 0..k with exact weights
-            const ProbDev &p = probs[c / S];
-            for (int l = 0; l <= k; l++) {
-                double2 y[S];
-#pragma unroll
-                for (int b = 0; b < S; b++)
-                    y[b] = RET ? p.gret[(tri(n) + n - l) * s2 + d * S + b] : p.gles[(tri(n) + l) * s2 + b * S + d];
-                const double al = greg_omega(k, l);
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    const int r = lane + 32 * t, i = i0 + r / S, a = r % S, delta = i - l;
-                    if (r >= NRb) continue;
-                    const double w = gh * (al + (delta <= k ? greg_omega(k, delta) : 1.0) - 1.0);
-                    double2 e = cmk(0, 0);
-#pragma unroll
-                    for (int b = 0; b < S; b++) e = cfma(*vol_t<S, RET>(g, n, i, l, a, b), y[b], e);
-                    acc[t] = cmk(fma(w, e.x, acc[t].x), fma(w, e.y, acc[t].y));
-                    if (!VIE && delta <= K1) {
-                        double2 ya = y[0];
-#pragma unroll
-                        for (int b = 1; b < S; b++) ya = a == b ? y[b] : ya;
-                        acc[t] = sub_ib(acc[t], bd_w(k, delta) / h, ya);
-                    }
-                }
+        for (int x = 0; x < RI; x++) {
+            const int e = tid + x * NTH, w = e & (wc - 1), r = e >> lw, i = i0 + r / S, a = r % S, c = c0 + w;
+            far[x] = q[x] = cmk(0, 0);
+            if (r >= NRb || w >= ncol) continue;
+            far[x] = __ldcg(g.vacc + ((long)i * S + a) * ldc + c);
+            if (!RET) q[x] = __ldcg(g.gles + ((long)i * S + a) * ldc + c);
+            if (VIE) {
+                const ProbDev &p = probs[c / S];
+                q[x] = cadd(q[x], RET ? p.qret[(tri(n) + n - i) * s2 + (c % S) * S + a] : p.qles[(tri(n) + i) * s2 + a * S + c % S]);
             }
         }
-        vol_chain<S, VIE>(acc, coef, dm + (c / S - p0) * NR * S, bdx, K1, nb, xs, smem + C::qs + warp * S, lane);
+        const double2 *ysrc = blk > 0 ? g.vy + (long)(i0 - K1) * S * ldc : g.vst;
+        for (int e = tid; e < (K1 * S) << lw; e += NTH) {
+            const int w = e & (wc - 1), x = e >> lw;
+            if (w < ncol) ynear[w * C::NEAR + x] = __ldcg(ysrc + (long)x * ldc + c0 + w);
+        }
+#pragma unroll
+        for (int x = 0; x < RI; x++) {
+            const int e = tid + x * NTH, w = e & (wc - 1), r = e >> lw;
+            if (r < NRb && w < ncol) buf[w * C::NRP + r] = cmk(fma(gh, far[x].x, q[x].x), fma(gh, far[x].y, q[x].y));
+        }
+    }
+    __syncthreads();
+    // row r of column w: the right-hand side with the near rows (weights and backward differences)
+    auto rhs = [&](int w, int r) {
+        double2 v = buf[w * C::NRP + r];
+        if (r < K1 * S) {
+            const double2 *y = ynear + w * C::NEAR;
+            const int l0 = r / S;
+            double2 o = cmk(0, 0);
+            for (int x = l0 * S; x < K1 * S; x++) o = cfma(near_[x * C::NEAR + r], y[x], o);
+            v = cadd(v, o);
+            if (!VIE)
+                for (int l = l0; l < K1; l++) v = sub_ib(v, bdp[32 + l0 + K1 - l], y[l * S + r % S]);
+        }
+        return v;
+    };
+    if constexpr (S <= 2) {
+        if (warp * nc < ncol) {
+            double2 acc[C::NC][4];
+            double2 *xs = buf + warp * nc * C::NRP;
+#pragma unroll
+            for (int cc = 0; cc < C::NC; cc++)
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    acc[cc][t] = cc < nc && warp * nc + cc < ncol && lane + 32 * t < NRb ? rhs(warp * nc + cc, lane + 32 * t) : cmk(0, 0);
+            __syncwarp();
+            if constexpr (S == 1) {
+                if (nc == 2) vol_chain1<VIE, 2>(acc, coef, Dr, bdp, gh, K1, nb, xs, lane);
+                else vol_chain1<VIE, 1>(acc, coef, Dr, bdp, gh, K1, nb, xs, lane);
+            } else {  // two columns of a warp are one problem's
+                const double2 *D = dm + ((c0 + warp * nc) / S - p0) * NR * S;
+                if (nc == 2) vol_chain2<VIE, 2>(acc, coef, D, bdp, gh, K1, nb, xs, lane);
+                else vol_chain2<VIE, 1>(acc, coef, D, bdp, gh, K1, nb, xs, lane);
+            }
+        }
+    } else {
+        const int w = warp >> 2, slot = warp & 3, r = slot * C::SR + lane;
+        double2 acc = w < ncol && lane < C::SR && r < NRb ? rhs(w, r) : cmk(0, 0);
+        __syncthreads();
+        if (w < ncol)
+            vol_chain_big<S, VIE>(acc, coef, dm + ((c0 + w) / S - p0) * NR * S, bdp, gh, nb, buf + w * C::NRP,
+                                  smem + C::qs(wc) + w * S, slot, lane, 1 + w);
     }
     __syncthreads();
     // ---- results: vy (rows x columns, for the trailing GEMM), ret: the operand of les*adv
     //      badv(m) = h w(n, m) G^R(n, m)^dagger, and G's own row / column
     const bool more = i0 + nb <= n;
-    for (int e = tid; e < NRb << lw; e += 256) {
-        const int w = e & (wc - 1), r = e >> lw, i = i0 + r / S, a = r % S;
-        if (w >= ncol) continue;
-        const double2 x = buf[w * C::NRP + r];
-        if (more) g.vy[((long)i * S + a) * ldc + c0 + w] = x;
-        if (RET) g.badv[((long)(n - i) * S + a) * ldc + c0 + w] = cscale(cconj(x), h * greg_w(k, n, n - i));
+#pragma unroll
+    for (int x = 0; x < RI; x++) {
+        const int e = tid + x * NTH, w = e & (wc - 1), r = e >> lw, i = i0 + r / S, a = r % S;
+        if (r >= NRb || w >= ncol) continue;
+        const double2 v = buf[w * C::NRP + r];
+        if (more) g.vy[((long)i * S + a) * ldc + c0 + w] = v;
+        if (RET) g.badv[((long)(n - i) * S + a) * ldc + c0 + w] = cscale(cconj(v), h * greg_w(k, n, n - i));
     }
-    for (int w = warp; w < ncol; w += 8) {
+    for (int w = warp; w < ncol; w += C::NW) {
         const int c = c0 + w, d = c % S;
         double2 *out = RET ? probs[c / S].gret + tri(n) * s2 : probs[c / S].gles + tri(n) * s2;
         for (int r = lane; r < NRb; r += 32) {
@@ -361,13 +414,13 @@ template <int S, bool RET> struct LdVolT {
 template <int S, bool RET>
 __device__ __forceinline__ bool vol_trail_operands(const GroupDev &g, int cols, int n, int blk, LdVolT<S, RET> &la,
                                                    LdRowN &lb, StRow &st, int &K) {
-    using C = VbCfg<S>;
-    const int i0 = g.k + 1 + blk * C::NBT, i1 = i0 + C::NBT, l0 = blk == 0 ? 0 : i0;
+    // blk = -1: the start rows 0..k
+    const int l0 = blk < 0 ? 0 : g.k + 1 + blk * VbCfg<S>::NBT, i1 = g.k + 1 + (blk + 1) * VbCfg<S>::NBT;
     const int M = (n - i1 + 1) * S;
     K = (i1 - l0) * S;
     la = LdVolT<S, RET>{RET ? g.rret : g.sret, n, i1, l0, M, K};
     lb = LdRowN{g.vy + (long)l0 * S * g.ldc, g.ldc, K, cols};
-    st = StRow{g.vacc + (long)i1 * S * g.ldc, g.ldc, M, cols, 1.0, blk > 0};
+    st = StRow{g.vacc + (long)i1 * S * g.ldc, g.ldc, M, cols, 1.0, blk >= 0};
     return M > 0;
 }
 // Grid (column tiles, row tiles, groups)
@@ -380,8 +433,10 @@ __global__ void __launch_bounds__(128, 4) k_vol_trail(const GroupDev *__restrict
     LdRowN lb;
     StRow st;
     int K;
+    pdl_trigger();
     if (!vol_trail_operands<S, RET>(g, cols, n, blk, la, lb, st, K)) return;
     if ((int)blockIdx.x * 32 >= cols || (int)blockIdx.y * 32 >= la.M) return;
+    pdl_wait();
     zgemm_pipe<32, 32>(la, lb, st, blockIdx.y * 32, blockIdx.x * 32, K, smem);
 }
 template <int S, bool RET>
@@ -393,8 +448,10 @@ __global__ void __launch_bounds__(256) k_vol_trail_split(const GroupDev *__restr
     LdRowN lb;
     StRow st;
     int K;
+    pdl_trigger();
     if (!vol_trail_operands<S, RET>(g, cols, n, blk, la, lb, st, K)) return;
     if ((int)blockIdx.x * 8 >= cols || (int)blockIdx.y * 32 >= la.M) return;
+    pdl_wait();
     zgemm_split(la, lb, st, blockIdx.y * 32, blockIdx.x * 8, K, red);
 }
 
@@ -421,6 +478,7 @@ __global__ void __launch_bounds__(256) k_ret_start(const GroupDev *__restrict__ 
         const int l = e / s2, b = (e % s2) / S, d = e % S;  // Y_l[b][d] = G(n, n-l)[d][b]
         const double2 y = grow[(long)(n - l) * s2 + d * S + b];
         g.vy[((long)l * S + b) * ldc + p.col * S + d] = cscale(y, greg_omega(k, l));
+        g.vst[((long)l * S + b) * ldc + p.col * S + d] = y;
         g.badv[((long)(n - l) * S + b) * ldc + p.col * S + d] = cscale(cconj(y), g.h * greg_w(k, n, n - l));
     }
 }
@@ -452,5 +510,6 @@ __global__ void __launch_bounds__(256) k_les_start(const GroupDev *__restrict__ 
     for (int e = threadIdx.x; e < (k + 1) * s2; e += blockDim.x) {
         const int l = e / s2, b = (e % s2) / S, d = e % S;
         g.vy[((long)l * S + b) * ldc + p.col * S + d] = cscale(xcol[e], greg_omega(k, l));
+        g.vst[((long)l * S + b) * ldc + p.col * S + d] = xcol[e];
     }
 }

@@ -135,7 +135,7 @@ struct Group {
     double2 *fccret = nullptr, *fccles = nullptr;
     double2 *fccmat = nullptr;       // Fcc^mat of a VIE2 group (nessi_gpu_set_Fcc_mat; steepest descent)
     double2 *U = nullptr;            // diagonal interaction U(t), (ntmax+2) x s, t = -1 first
-    double2 *vy = nullptr, *vacc = nullptr;  // blocked recursion: solved rows, far sums of the rows to come
+    double2 *vy = nullptr, *vacc = nullptr, *vst = nullptr;  // blocked recursion: solved rows, far sums, start rows
     std::vector<int> members;        // problem indices, nt descending
     std::vector<ProbDev> h_probs;    // same order; col = position
     ProbDev *d_probs = nullptr;
@@ -222,7 +222,7 @@ GroupDev group_dev(const Group &g) {
     d.fccmat = g.fccmat;
     d.ntmax = g.ntmax; d.ntau = g.ntau; d.s = g.s; d.sig = g.sig; d.k = g.k;
     d.ldc = g.ldc; d.h = g.h; d.beta = g.beta;
-    d.vy = g.vy; d.vacc = g.vacc; d.probs = g.d_probs;
+    d.vy = g.vy; d.vacc = g.vacc; d.vst = g.vst; d.probs = g.d_probs;
     return d;
 }
 
@@ -254,6 +254,32 @@ int find_group(nessi_batch *b, int user_id) {
 }
 
 // ---- per-size kernel launch table ----------------------------------------------------
+// Dynamic shared memory of a kernel, with the SM's L1 / shared split set to all shared: kernels of
+// the two streams of a step can share an SM only when they ask for the same split.
+int share_sm(const void *kernel, size_t smem) {
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    return NESSI_OK;
+}
+
+// Launch that may start before the previous kernel of the stream has finished: the kernel waits for
+// it (griddepcontrol.wait) before it touches anything that an earlier kernel of the chain wrote.
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return NESSI_OK;
+}
+
 // C (M x N) = A (M x K) B (K x N) on the repo's DMMA GEMM (kernels_gemm.cuh).
 template <int BM, int BN, class LA, class LB, class ST>
 int zgemm_launch_tiles(const LA &la, const LB &lb, const ST &st, int M, int N, int K, cudaStream_t s) {
@@ -308,34 +334,33 @@ int volterra_class(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) 
     const GroupDev *gt = b->d_groups;
     if (RET) {
         const size_t sm = ret_start_smem<S>(kmax);
-        CK(cudaFuncSetAttribute(k_ret_start<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        CKR(share_sm((const void *)k_ret_start<S, VIE>, sm));
         k_ret_start<S, VIE><<<dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st>>>(gt, sel, n);
     } else {
         const size_t sm = les_start_smem<S>(kmax);
-        CK(cudaFuncSetAttribute(k_les_start<S, VIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        CKR(share_sm((const void *)k_les_start<S, VIE>, sm));
         k_les_start<S, VIE><<<dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st>>>(gt, sel, n);
     }
     CK(cudaGetLastError());
     int wc = 1;
     while (wc < C::WMAX && cols > (long)wc * b->nsm) wc *= 2;
     const dim3 gd((unsigned)((maxact * S + wc - 1) / wc), (unsigned)sel.ng);
-    const size_t smb = (size_t)C::total * sizeof(double2);
-    CK(cudaFuncSetAttribute(k_vol_block<S, VIE, RET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
+    const size_t smb = (size_t)C::total(wc) * sizeof(double2);
+    CKR(share_sm((const void *)k_vol_block<S, VIE, RET>, (size_t)C::total(C::WMAX) * sizeof(double2)));
     using P = zg::Pipe<32, 32, LdVolT<S, RET>, LdRowN>;
     const size_t smt = (size_t)P::total * sizeof(double2);
-    CK(cudaFuncSetAttribute(k_vol_trail<S, RET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt));
+    CKR(share_sm((const void *)k_vol_trail<S, RET>, smt));
+    CKR(share_sm((const void *)k_vol_trail_split<S, RET>, 0));
     const int nblk = (n - kmin + C::NBT - 1) / C::NBT;
-    for (int blk = 0; blk < nblk; blk++) {
-        k_vol_block<S, VIE, RET><<<gd, 256, smb, st>>>(gt, sel, n, blk, wc);
-        CK(cudaGetLastError());
+    for (int blk = -1; blk < nblk; blk++) {  // -1: the start rows, which only enter the later ones
+        if (blk >= 0) CKR(launch_chained(k_vol_block<S, VIE, RET>, gd, C::NTH, smb, st, gt, sel, n, blk, wc));
         const int M = (n - kmin - (blk + 1) * C::NBT) * S;  // rows after the block (largest group)
         if (M <= 0) break;
-        const unsigned rt = (unsigned)((M + 31) / 32), N = (unsigned)(maxact * S);
-        if (zgemm_use_split(M, N, C::NR, sel.ng))
-            k_vol_trail_split<S, RET><<<dim3((N + 7) / 8, rt, (unsigned)sel.ng), 256, 0, st>>>(gt, sel, n, blk);
+        const unsigned rt = (unsigned)((M + 31) / 32), N = (unsigned)(maxact * S), z = (unsigned)sel.ng;
+        if (blk >= 0 && zgemm_use_split(M, N, C::NR, sel.ng))
+            CKR(launch_chained(k_vol_trail_split<S, RET>, dim3((N + 7) / 8, rt, z), 256, 0, st, gt, sel, n, blk));
         else
-            k_vol_trail<S, RET><<<dim3((N + 31) / 32, rt, (unsigned)sel.ng), 128, smt, st>>>(gt, sel, n, blk);
-        CK(cudaGetLastError());
+            CKR(launch_chained(k_vol_trail<S, RET>, dim3((N + 31) / 32, rt, z), 128, smt, st, gt, sel, n, blk));
     }
     return NESSI_OK;
 }
@@ -454,7 +479,6 @@ template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int n
     CK(cudaEventRecord(b->ev_join, b->side));
     // main stream: tv row, then the tv*vt operand
     {
-        dim3 grid((g.ntau + 1 + 31) / 32, nact);
         b->prof_mark(NESSI_KERNEL_TV);
         const bool mixed = b->precision == NESSI_PREC_MIXED;
         bool streamed = false;
@@ -466,8 +490,14 @@ template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int n
             }
         }
         if (!streamed) {
-            if (mixed) k_tv<S, true, VIE><<<grid, 256, 0, st>>>(gd, g.d_probs, n);
-            else k_tv<S, false, VIE><<<grid, 256, 0, st>>>(gd, g.d_probs, n);
+            if (mixed) {
+                k_tv_mixed<S, VIE><<<dim3((g.ntau + 1 + 31) / 32, nact), 256, 0, st>>>(gd, g.d_probs, n);
+            } else {
+                const int items = nact * ((g.ntau + 32) / 32) * S;
+                const size_t smr = (size_t)TvCfg<S>::total * sizeof(double2);
+                CKR(share_sm((const void *)k_tv_ring<S, VIE>, smr));
+                k_tv_ring<S, VIE><<<dim3((unsigned)std::min(items, b->nsm), 1), TvCfg<S>::NTH, smr, st>>>(b->d_groups, sel, n);
+            }
             CK(cudaGetLastError());
         }
         // per problem: G^tv history rows 0..n-1 read (FP32 below the k+1 BDF rows when mixed),
@@ -781,7 +811,7 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
             (r = b->alloc(&g.btv, M * S * g.ldc)) || (r = b->alloc(&g.gles, N * S * g.ldc)) ||
             (r = b->alloc(&g.Kmat, M * S * M * S)) || (r = b->alloc(&g.Gmat_all, M * S * g.ldc)) ||
             (r = b->alloc(&g.Cmat, M * S * g.ldc)) || (r = b->alloc(&g.vy, N * S * g.ldc)) ||
-            (r = b->alloc(&g.vacc, N * S * g.ldc)))
+            (r = b->alloc(&g.vacc, N * S * g.ldc)) || (r = b->alloc(&g.vst, (g.k + 1) * S * g.ldc)))
             return fail(r);
         for (size_t c = 0; c < g.members.size(); c++) {
             const Prob &p = b->probs[g.members[c]];
