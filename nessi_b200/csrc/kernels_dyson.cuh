@@ -45,6 +45,7 @@ struct GroupDev {
     int ntmax, ntau, s, sig, k;
     int ldc;           // >= nprob * s
     double h, beta;
+    double conv_sign;  // sign of the convolutions on the right-hand side: 1 (Dyson), -1 (VIE2)
 };
 
 #define NESSI_GSEL 64  // groups per launch
@@ -52,6 +53,11 @@ struct GroupDev {
 struct GroupSel {
     int ng;
     int gid[NESSI_GSEL], nact[NESSI_GSEL];
+};
+// First time indices a step has to prepare, per group of a GroupSel: step matrices of the lesser / tv
+// and retarded equations, dense rows and columns of Sigma
+struct PrepSel {
+    int les_lo[NESSI_GSEL], ret_lo[NESSI_GSEL], d_lo[NESSI_GSEL];
 };
 
 __device__ __forceinline__ long tri(long t) { return t * (t + 1) / 2; }
@@ -64,9 +70,12 @@ __device__ __forceinline__ long tri(long t) { return t * (t + 1) / 2; }
 // VIE2 ([1 + F] G = Q, cntr_vie2_impl.hpp:60-140, 645-725, 847-990): the step matrices are
 //   tv/les:  mm = 1 + h w0 F^R(j,j);   ret: mm = 1 + h w0 Fcc^R(j,j)
 template <int S, bool VIE = false>
-__global__ void k_prep_problem(GroupDev g, const ProbDev *__restrict__ probs, int n, int les_lo, int r0, int r1) {
-    const ProbDev p = probs[blockIdx.x];
+__global__ void k_prep_problem(const GroupDev *__restrict__ gt, GroupSel sel, PrepSel ps, int n) {
+    if ((int)blockIdx.x >= sel.nact[blockIdx.y]) return;
+    const GroupDev &g = gt[sel.gid[blockIdx.y]];
+    const ProbDev p = g.probs[blockIdx.x];
     const int k = g.k, s2 = S * S;
+    const int les_lo = ps.les_lo[blockIdx.y], r0 = ps.ret_lo[blockIdx.y], r1 = n - k - 1;
     const double h = g.h;
     const double2 ibd0 = cmk(0.0, bd_w(k, 0) / h);
     const double w0 = h * greg_omega(k, 0);
@@ -104,8 +113,9 @@ __global__ void k_prep_problem(GroupDev g, const ProbDev *__restrict__ probs, in
 // ---------------------------------------------------------------------------------------
 // VIE2: a_j = -h w(n,j) F^R(n,j) (conv_tv with A = F, moved to the right-hand side).
 template <int S, bool VIE = false>
-__global__ void k_prep_group(GroupDev g, int n, int d_lo) {
-    const int k = g.k, s2 = S * S;
+__global__ void k_prep_group(const GroupDev *__restrict__ gt, GroupSel sel, PrepSel ps, int n) {
+    const GroupDev &g = gt[sel.gid[blockIdx.y]];
+    const int k = g.k, s2 = S * S, d_lo = ps.d_lo[blockIdx.y];
     const double h = g.h;
     const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
     const long nth = (long)gridDim.x * blockDim.x;
@@ -540,10 +550,12 @@ template <int S> struct TvmCfg {
 // VIE2 (vie2_timestep_tv, cntr_vie2_impl.hpp:645-725): a_j and Cmat carry the minus sign of
 // the convolution and Q^tv(n, tau) is added before the solve with (1 + h w0 F^R(n,n))^-1.
 template <int S, bool VIE = false>
-__global__ void __launch_bounds__(256) k_tv_mixed(GroupDev g, const ProbDev *__restrict__ probs, int n) {
+__global__ void __launch_bounds__(256) k_tv_mixed(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
     constexpr int s2 = S * S, DCH = TvmCfg<S>::DCH, NW = TvmCfg<S>::NW;
     __shared__ double2 red[NW * 32 * S * DCH];
-    const ProbDev p = probs[blockIdx.y];
+    const GroupDev &g = gt[sel.gid[blockIdx.z]];
+    if ((int)blockIdx.y >= sel.nact[blockIdx.z] || (int)blockIdx.x * 32 > g.ntau) return;
+    const ProbDev p = g.probs[blockIdx.y];
     const int ntau = g.ntau, M = ntau + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tau = blockIdx.x * 32 + lane;
@@ -680,9 +692,10 @@ __global__ void k_tv_relayout(double2 *__restrict__ dst, const double2 *__restri
 //   c2 = sum_{l=0}^{r} w(r,l) A(m+l) B(l)           (r = ntau-m >= k; rcorr for 0<r<k)
 //   c1 = sum_{l=0}^{m} w(m,l) A(m-l) B(ntau-l)      (m >= k; rcorr for 0<m<k),  C = c2 + sig c1
 // ---------------------------------------------------------------------------------------
-// sgn = -1 for VIE2, whose Matsubara convolution enters the right-hand side with a minus sign.
+// (conv_sign = -1 for VIE2, whose Matsubara convolution enters the right-hand side with a minus sign.)
 template <int S>
-__global__ void k_mat_operator(GroupDev g, int n, double sgn) {
+__global__ void k_mat_operator(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
+    const GroupDev &g = gt[sel.gid[blockIdx.y]];
     const int k = g.k, s2 = S * S, ntau = g.ntau, M = ntau + 1;
     const long KS = (long)M * S;
     const double2 *A = g.stv + (long)n * M * s2;
@@ -704,7 +717,7 @@ __global__ void k_mat_operator(GroupDev g, int n, double sgn) {
         } else if (m > 0 && l >= 0 && l <= k) {
             for (int jj = 0; jj <= k; jj++) v = cfma(cmk(sg * rcorr_w(k, m, l, jj), 0), A[(long)jj * s2 + ac], v);
         }
-        g.Kmat[((long)m * S + a) * KS + (long)x * S + c] = cscale(v, dtau * sgn);
+        g.Kmat[((long)m * S + a) * KS + (long)x * S + c] = cscale(v, dtau * g.conv_sign);
     }
 }
 
@@ -733,8 +746,12 @@ template <int S> struct LoCfg {
 };
 
 template <int S>
-__global__ void __launch_bounds__(256) k_les_operands_t(GroupDev g, const ProbDev *__restrict__ probs, int n, int nact) {
+__global__ void __launch_bounds__(256) k_les_operands_t(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
     constexpr int s2 = S * S, LOR = LoCfg<S>::LOR;
+    const GroupDev &g = gt[sel.gid[blockIdx.z]];
+    const ProbDev *probs = g.probs;
+    const int nact = sel.nact[blockIdx.z];
+    if ((int)blockIdx.y * LOT >= nact || (int)blockIdx.x * LOR > g.ntau) return;
     __shared__ double2 buf[LOT * LOR * s2 + LOT];
     __shared__ const double2 *src[LOT];
     __shared__ int colid[LOT];
@@ -763,4 +780,64 @@ __global__ void __launch_bounds__(256) k_les_operands_t(GroupDev g, const ProbDe
         g.btv[((long)m * S + c) * ldc + (long)colid[q] * S + d] =
             cmul(cmk(0.0, dtau * (double)g.sig * greg_w(k, ntau, m)), v);
     }
+}
+
+// ---------------------------------------------------------------------------------------
+// The three Sigma-shared products of a step, one launch for all selected groups (grid z):
+//   PROD_MAT     Cmat = K_n Gmat_all                        (Matsubara part of the tv row)
+//   PROD_LESADV  gles = +- Sigma^<_dense badv               (les*adv)
+//   PROD_TVVT    gles += +- Sigma^tv btv                    (tv*vt)
+// ---------------------------------------------------------------------------------------
+enum { PROD_MAT, PROD_LESADV, PROD_TVVT };
+struct ProdDims {
+    int M, N, K;
+};
+template <int OP>
+__host__ __device__ inline ProdDims prod_dims(int s, int ntau, int n, int nact) {
+    const int MS = (ntau + 1) * s, nn = (n + 1) * s;
+    return ProdDims{OP == PROD_MAT ? MS : nn, nact * s, OP == PROD_LESADV ? nn : MS};
+}
+template <int OP>
+__host__ __device__ inline ProdDims prod_operands(const GroupDev &g, int n, int nact, LdRowK &la, LdRowN &lb, StRow &st) {
+    const ProdDims d = prod_dims<OP>(g.s, g.ntau, n, nact);
+    const long ldL = (long)(g.ntmax + 1) * g.s, MS = (long)(g.ntau + 1) * g.s;
+    if (OP == PROD_MAT) {
+        la = LdRowK{g.Kmat, MS, d.M, d.K};
+        lb = LdRowN{g.Gmat_all, g.ldc, d.K, d.N};
+        st = StRow{g.Cmat, g.ldc, d.M, d.N, 1.0, 0};
+    } else if (OP == PROD_LESADV) {
+        la = LdRowK{g.Ldense, ldL, d.M, d.K};
+        lb = LdRowN{g.badv, g.ldc, d.K, d.N};
+        st = StRow{g.gles, g.ldc, d.M, d.N, g.conv_sign, 0};
+    } else {
+        la = LdRowK{g.s == 1 ? g.stv : g.Tdense, MS, d.M, d.K};
+        lb = LdRowN{g.btv, g.ldc, d.K, d.N};
+        st = StRow{g.gles, g.ldc, d.M, d.N, g.conv_sign, 1};
+    }
+    return d;
+}
+template <int OP>
+__global__ void __launch_bounds__(128, 4) k_zgemm(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
+    extern __shared__ double2 zsm[];
+    LdRowK la;
+    LdRowN lb;
+    StRow st;
+    const ProdDims d = prod_operands<OP>(gt[sel.gid[blockIdx.z]], n, sel.nact[blockIdx.z], la, lb, st);
+    if ((int)blockIdx.y * 32 >= d.M || (int)blockIdx.x * 32 >= d.N) return;
+    zgemm_pipe<32, 32>(la, lb, st, blockIdx.y * 32, blockIdx.x * 32, d.K, zsm);
+}
+template <int OP>
+__global__ void __launch_bounds__(256, 2) k_zgemm_split(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
+    __shared__ double2 red[8 * 32 * 8];
+    LdRowK la;
+    LdRowN lb;
+    StRow st;
+    const ProdDims d = prod_operands<OP>(gt[sel.gid[blockIdx.z]], n, sel.nact[blockIdx.z], la, lb, st);
+    if ((int)blockIdx.y * 32 >= d.M || (int)blockIdx.x * 8 >= d.N) return;
+    zgemm_split(la, lb, st, blockIdx.y * 32, blockIdx.x * 8, d.K, red);
+}
+// one group: the operands in the kernel's parameters (2002 x 512 x 2002 521 us, through the table 542)
+__global__ void __launch_bounds__(256, 2) k_zgemm_split1(LdRowK la, LdRowN lb, StRow st, int K) {
+    __shared__ double2 red[8 * 32 * 8];
+    zgemm_split(la, lb, st, blockIdx.y * 32, blockIdx.x * 8, K, red);
 }

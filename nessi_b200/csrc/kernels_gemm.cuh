@@ -104,6 +104,9 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 
 // C tile (m0.., n0..) = A B over k = 0..K-1 by the 128 threads of a CTA: 2 x 2 warps of
 // (16 MT) x (8 NT), operands through a ring of three cp.async stages of 8 k (one barrier per stage).
+// Used with 32 x 32 tiles, four CTAs per SM, for short K (the last factor): 900 x 512 x 128 19.0
+// TFLOP/s, the k-split form 17.5; 400 x 1024 x 128 20.2 against 16.9.  Larger tiles leave too few
+// CTAs (64 x 64: 15.6 TFLOP/s on 400 x 1024 x 128).
 template <int BM, int BN, class LA, class LB, class PUT>
 __device__ __forceinline__ void zgemm_pipe(const LA &la, const LB &lb, const PUT &put, int m0, int n0, int K,
                                            double2 *sm) {
@@ -203,19 +206,10 @@ __device__ __forceinline__ void zgemm_pipe(const LA &la, const LB &lb, const PUT
     }
 }
 
-// grid (ceil(N / BN), ceil(M / BM)), 128 threads, zg::Pipe<...>::total complex of dynamic shared
-// memory.  For short K (the last factor): 900 x 512 x 128 19.0 TFLOP/s, the k-split form 17.5;
-// 400 x 1024 x 128 20.2 against 16.9.  32 x 32 tiles, four CTAs per SM: larger tiles leave too few
-// CTAs (64 x 64 15.6 TFLOP/s on 400 x 1024 x 128).
-template <int BM, int BN, class LA, class LB, class PUT>
-__global__ void __launch_bounds__(128, 4) k_zgemm(LA la, LB lb, PUT put, int K) {
-    extern __shared__ double2 zsm[];
-    zgemm_pipe<BM, BN>(la, lb, put, blockIdx.y * BM, blockIdx.x * BN, K, zsm);
-}
-
 // k-split products: a CTA of 8 warps computes a 32 x 8 tile, the k steps dealt to the warps and
 // summed in warp order; operands straight from L1 / L2 into the fragments.  Grid (ceil(N / 8),
-// ceil(M / 32)).  Bound: the FP64 tensor pipe (16 warps per SM, each with two k steps of loads in
+// ceil(M / 32)); two CTAs per SM (128 registers: with one CTA 812 us for 2002 x 512 x 2002, with three
+// 687, with two 521).  Bound: the FP64 tensor pipe (16 warps per SM, each with two k steps of loads in
 // flight), and for few tiles the K / 64 dependent rounds of loads of a warp.  Measured alone on a
 // B200, complex M x N x K (8 flops each): 4804 x 128 x 4804 31.5 TFLOP/s (32 x 32 tiles through
 // shared memory 25.4, 64 x 64 17.5: too few tiles, uneven last wave), 2002 x 512 x 2002 31.5
@@ -278,9 +272,4 @@ __device__ __forceinline__ void zgemm_split(const LA &la, const LB &lb, const PU
         const int r = m0 + x / BN, c = n0 + x % BN;
         put.store(r, c, put.combine(put.accumulates() ? put.load(r, c) : cmk(0, 0), v));
     }
-}
-template <class LA, class LB, class PUT>
-__global__ void __launch_bounds__(256) k_zgemm_split(LA la, LB lb, PUT put, int K) {
-    __shared__ double2 red[8 * 32 * 8];
-    zgemm_split(la, lb, put, blockIdx.y * 32, blockIdx.x * 8, K, red);
 }

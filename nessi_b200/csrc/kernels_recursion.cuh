@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(128, 4) k_vol_trail(const GroupDev *__restrict
     zgemm_pipe<32, 32>(la, lb, st, blockIdx.y * 32, blockIdx.x * 32, K, smem);
 }
 template <int S, bool RET>
-__global__ void __launch_bounds__(256) k_vol_trail_split(const GroupDev *__restrict__ gt, GroupSel sel, int n, int blk) {
+__global__ void __launch_bounds__(256, 2) k_vol_trail_split(const GroupDev *__restrict__ gt, GroupSel sel, int n, int blk) {
     __shared__ double2 red[8 * 32 * 8];
     const GroupDev &g = gt[sel.gid[blockIdx.z]];
     const int cols = sel.nact[blockIdx.z] * S;

@@ -223,6 +223,7 @@ GroupDev group_dev(const Group &g) {
     d.ntmax = g.ntmax; d.ntau = g.ntau; d.s = g.s; d.sig = g.sig; d.k = g.k;
     d.ldc = g.ldc; d.h = g.h; d.beta = g.beta;
     d.vy = g.vy; d.vacc = g.vacc; d.vst = g.vst; d.probs = g.d_probs;
+    d.conv_sign = g.vie ? -1.0 : 1.0;
     return d;
 }
 
@@ -280,30 +281,38 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
     return NESSI_OK;
 }
 
-// C (M x N) = A (M x K) B (K x N) on the repo's DMMA GEMM (kernels_gemm.cuh).
-template <int BM, int BN, class LA, class LB, class ST>
-int zgemm_launch_tiles(const LA &la, const LB &lb, const ST &st, int M, int N, int K, cudaStream_t s) {
-    const dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM));
-    const size_t sm = (size_t)zg::Pipe<BM, BN, LA, LB>::total * sizeof(double2);
-    CK(cudaFuncSetAttribute(k_zgemm<BM, BN, LA, LB, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_zgemm<BM, BN><<<grid, 128, sm, s>>>(la, lb, st, K);
-    CK(cudaGetLastError());
-    return NESSI_OK;
-}
-// Long K, or too few 32 x 32 tiles for the 148 SMs: the k-split kernel; else the tiled one (both
-// sides measured at the kernels).
+// Products on the repo's DMMA GEMM (kernels_gemm.cuh).  Long K, or too few 32 x 32 tiles for the
+// 148 SMs: the k-split form; else the tiled one (both sides measured at the kernels).
 bool zgemm_use_split(long M, long N, long K, int count = 1) {
     return K >= 256 || ((M + 31) / 32) * ((N + 31) / 32) * count < 148;
 }
-template <class LA, class LB, class ST>
-int zgemm_launch(const LA &la, const LB &lb, const ST &st, int M, int N, int K, cudaStream_t s) {
-    if (M <= 0 || N <= 0) return NESSI_OK;
-    if (zgemm_use_split(M, N, K)) {
-        k_zgemm_split<<<dim3((unsigned)((N + 7) / 8), (unsigned)((M + 31) / 32)), 256, 0, s>>>(la, lb, st, K);
-        CK(cudaGetLastError());
-        return NESSI_OK;
+template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) {
+    ProdDims m{0, 0, 0};
+    for (int i = 0; i < sel.ng; i++) {
+        const Group &g = b->groups[sel.gid[i]];
+        const ProdDims d = prod_dims<OP>(g.s, g.ntau, n, sel.nact[i]);
+        m.M = std::max(m.M, d.M);
+        m.N = std::max(m.N, d.N);
+        m.K = std::max(m.K, d.K);
     }
-    return zgemm_launch_tiles<32, 32>(la, lb, st, M, N, K, s);
+    if (zgemm_use_split(m.M, m.N, m.K, sel.ng)) {
+        const dim3 grid((unsigned)((m.N + 7) / 8), (unsigned)((m.M + 31) / 32), (unsigned)sel.ng);
+        if (sel.ng == 1) {
+            LdRowK la;
+            LdRowN lb;
+            StRow sto;
+            const ProdDims d = prod_operands<OP>(group_dev(b->groups[sel.gid[0]]), n, sel.nact[0], la, lb, sto);
+            k_zgemm_split1<<<grid, 256, 0, st>>>(la, lb, sto, d.K);
+        } else {
+            k_zgemm_split<OP><<<grid, 256, 0, st>>>(b->d_groups, sel, n);
+        }
+    } else {
+        const dim3 grid((unsigned)((m.N + 31) / 32), (unsigned)((m.M + 31) / 32), (unsigned)sel.ng);
+        const size_t sm = (size_t)zg::Pipe<32, 32, LdRowK, LdRowN>::total * sizeof(double2);
+        k_zgemm<OP><<<grid, 128, sm, st>>>(b->d_groups, sel, n);
+    }
+    CK(cudaGetLastError());
+    return NESSI_OK;
 }
 
 // Volterra kernels reported by nessi_gpu_get_volterra_choice: the blocked recursion
@@ -414,120 +423,115 @@ int tv_stream_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, 
     return NESSI_OK;
 }
 
-template <int S, bool VIE> int step_group(nessi_batch *b, Group &g, int n, int nact) {
-    const GroupDev gd = group_dev(g);
-    GroupSel sel;
-    sel.ng = 1;
-    sel.gid[0] = (int)(&g - b->groups.data());
-    sel.nact[0] = nact;
+// Time step n of the selected groups, all of size1 = S and one kind: every kernel is one launch for
+// all of them.
+template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, int n) {
     cudaStream_t st = b->stream;
-    const int k = g.k;
-    // step-matrix inverses
-    int les_lo = std::min(n, std::max(k + 1, g.les_valid + 1));
-    int r0 = g.ret_valid + 1, r1 = n - k - 1;
-    b->prof_mark(NESSI_KERNEL_PREP);
-    k_prep_problem<S, VIE><<<nact, 64, 0, st>>>(gd, g.d_probs, n, les_lo, r0, r1);
-    CK(cudaGetLastError());
-    g.les_valid = n - 1;
-    if (r1 >= r0) g.ret_valid = r1;
-    int d_lo = std::min(n, g.dense_valid + 1);
-    {
-        long work = (long)(n + 1) * S * S * (n - d_lo + 1) + (long)n * S * S;
-        int blocks = (int)std::min<long>(std::max<long>(1, (work + 255) / 256), 1184);
-        k_prep_group<S, VIE><<<blocks, 256, 0, st>>>(gd, n, d_lo);
-        CK(cudaGetLastError());
-        b->prof_end(NESSI_KERNEL_PREP, 0.0);
+    const GroupDev *gt = b->d_groups;
+    const unsigned ng = (unsigned)sel.ng;
+    PrepSel ps;
+    int maxact = 0, M = 0;  // over the groups
+    long prep = 1, nprob = 0;
+    double flop_rec = 0, flop_mat = 0, flop_les = 0, flop_vt = 0, by_mat = 0, by_tv = 0, by_vt = 0;
+    const bool mixed = b->precision == NESSI_PREC_MIXED;
+    for (int i = 0; i < sel.ng; i++) {
+        Group &g = b->groups[sel.gid[i]];
+        const int nact = sel.nact[i], k = g.k;
+        maxact = std::max(maxact, nact);
+        M = std::max(M, g.ntau + 1);
+        nprob += nact;
+        // step-matrix inverses
+        ps.les_lo[i] = std::min(n, std::max(k + 1, g.les_valid + 1));
+        ps.ret_lo[i] = g.ret_valid + 1;
+        ps.d_lo[i] = std::min(n, g.dense_valid + 1);
+        g.les_valid = n - 1;
+        g.ret_valid = std::max(g.ret_valid, n - k - 1);
         g.dense_valid = n - 1;
-    }
-    // VIE2 moves the convolution to the right-hand side: gles = -(tv*vt + les*adv)
-    const double alpha = VIE ? -1.0 : 1.0;
-    // Matsubara part of the tv row: Cmat = K_n Gmat_all (one GEMM for the group)
-    {
-        const long M = g.ntau + 1;
+        prep = std::max(prep, (long)(n + 1) * S * S * (n - ps.d_lo[i] + 1) + (long)n * S * S);
+        const double Mg = g.ntau + 1, s2 = S * S, P = nact, N = n + 1;
+        flop_rec += 8.0 * S * s2 * P * tri_h(n);  // every pair m > j of the row, an s x s complex product (8 s^3)
+        flop_mat += 8.0 * S * s2 * P * Mg * Mg;
+        flop_les += 8.0 * S * s2 * P * N * N;
+        flop_vt += 8.0 * S * s2 * P * N * Mg;
+        by_mat += 16.0 * s2 * (Mg * Mg + Mg);
+        // per problem: G^tv history rows 0..n-1 read (FP32 below the k+1 BDF rows when mixed),
+        // row n written, Cmat column read; shared: the n coefficient blocks
+        const double n32 = mixed ? std::max(0, n - k - 1) : 0, n64 = n - n32;
+        by_tv += s2 * (P * (8.0 * n32 * Mg + 16.0 * n64 * Mg + 32.0 * Mg + (mixed ? 8.0 * Mg : 0.0)) + 16.0 * n);
+        by_vt += 32.0 * s2 * P * Mg;
         if (!g.gmat_valid) {
-            dim3 grid((unsigned)((M * S * S + 255) / 256), (unsigned)g.members.size());
-            k_gmat_stack<S><<<grid, 256, 0, st>>>(gd, g.d_probs);
+            dim3 grid((unsigned)((Mg * s2 + 255) / 256), (unsigned)g.members.size());
+            k_gmat_stack<S><<<grid, 256, 0, st>>>(group_dev(g), g.d_probs);
             CK(cudaGetLastError());
             g.gmat_valid = true;
         }
-        b->prof_mark(NESSI_KERNEL_MATOP);
-        long work = M * M * S * S;
-        k_mat_operator<S><<<(unsigned)std::min<long>((work + 255) / 256, 4736), 256, 0, st>>>(gd, n, VIE ? -1.0 : 1.0);
-        CK(cudaGetLastError());
-        b->prof_end(NESSI_KERNEL_MATOP, 16.0 * (double)work + 16.0 * M * S * S);
-        b->prof_mark(NESSI_KERNEL_GEMM);
-        const int MS = (int)(M * S);
-        CKR(zgemm_launch(LdRowK{g.Kmat, MS, MS, MS}, LdRowN{g.Gmat_all, g.ldc, MS, nact * S},
-                         StRow{g.Cmat, g.ldc, MS, nact * S, 1.0, 0}, MS, nact * S, MS, st));
-        b->prof_end(NESSI_KERNEL_GEMM, 8.0 * (double)nact * S * (M * S) * (M * S));
     }
-    const int m = nact * S, nn = (n + 1) * S;
-    const long ldL = (long)(g.ntmax + 1) * S, ldT = (long)(g.ntau + 1) * S;
-    // side stream: retarded row, then les*adv = Ldense * badv (needs only G^R(n, .))
+    b->prof_mark(NESSI_KERNEL_PREP);
+    k_prep_problem<S, VIE><<<dim3((unsigned)maxact, ng), 64, 0, st>>>(gt, sel, ps, n);
+    CK(cudaGetLastError());
+    k_prep_group<S, VIE><<<dim3((unsigned)std::min<long>((prep + 255) / 256, 1184), ng), 256, 0, st>>>(gt, sel, ps, n);
+    CK(cudaGetLastError());
+    b->prof_end(NESSI_KERNEL_PREP, 0.0);
+    // Matsubara part of the tv row: Cmat = K_n Gmat_all (one GEMM per group)
+    b->prof_mark(NESSI_KERNEL_MATOP);
+    k_mat_operator<S><<<dim3((unsigned)std::min<long>(((long)M * M * S * S + 255) / 256, 4736), ng), 256, 0, st>>>(gt, sel, n);
+    CK(cudaGetLastError());
+    b->prof_end(NESSI_KERNEL_MATOP, by_mat);
+    b->prof_mark(NESSI_KERNEL_GEMM);
+    CKR(product_launch<PROD_MAT>(b, sel, n, st));
+    b->prof_end(NESSI_KERNEL_GEMM, flop_mat);
+    // side stream: retarded row, then les*adv = Ldense * badv (needs only G^R(n, .)); VIE2 moves the
+    // convolution to the right-hand side: gles = -(tv*vt + les*adv)
     CK(cudaEventRecord(b->ev_fork, st));
     CK(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-    {
-        b->prof_mark(NESSI_KERNEL_RET, b->side);
-        CKR((volterra_class<S, VIE, true>(b, sel, n, b->side)));
-        // flops: every pair m > j of the row, an s x s complex product (8 s^3) per problem
-        b->prof_end(NESSI_KERNEL_RET, 8.0 * S * S * S * (double)nact * tri_h(n), b->side);
-        b->prof_mark(NESSI_KERNEL_GEMM, b->side);
-        CKR(zgemm_launch(LdRowK{g.Ldense, ldL, nn, nn}, LdRowN{g.badv, g.ldc, nn, m},
-                         StRow{g.gles, g.ldc, nn, m, alpha, 0}, nn, m, nn, b->side));
-        b->prof_end(NESSI_KERNEL_GEMM, 8.0 * (double)m * nn * ((n + 1) * S), b->side);
-    }
+    b->prof_mark(NESSI_KERNEL_RET, b->side);
+    CKR((volterra_class<S, VIE, true>(b, sel, n, b->side)));
+    b->prof_end(NESSI_KERNEL_RET, flop_rec, b->side);
+    b->prof_mark(NESSI_KERNEL_GEMM, b->side);
+    CKR(product_launch<PROD_LESADV>(b, sel, n, b->side));
+    b->prof_end(NESSI_KERNEL_GEMM, flop_les, b->side);
     CK(cudaEventRecord(b->ev_join, b->side));
     // main stream: tv row, then the tv*vt operand
-    {
-        b->prof_mark(NESSI_KERNEL_TV);
-        const bool mixed = b->precision == NESSI_PREC_MIXED;
-        bool streamed = false;
-        if constexpr (S <= 4) {
-            if (b->tv_kernel == 0) {
-                if (mixed) CKR((tv_stream_launch<S, true, VIE>(b, gd, g, n, nact, st)));
-                else CKR((tv_stream_launch<S, false, VIE>(b, gd, g, n, nact, st)));
-                streamed = true;
+    b->prof_mark(NESSI_KERNEL_TV);
+    bool streamed = false;
+    if constexpr (S <= 4) {
+        if (b->tv_kernel == 0) {
+            for (int i = 0; i < sel.ng; i++) {
+                const Group &g = b->groups[sel.gid[i]];
+                if (mixed) CKR((tv_stream_launch<S, true, VIE>(b, group_dev(g), g, n, sel.nact[i], st)));
+                else CKR((tv_stream_launch<S, false, VIE>(b, group_dev(g), g, n, sel.nact[i], st)));
             }
+            streamed = true;
         }
-        if (!streamed) {
-            if (mixed) {
-                k_tv_mixed<S, VIE><<<dim3((g.ntau + 1 + 31) / 32, nact), 256, 0, st>>>(gd, g.d_probs, n);
-            } else {
-                const int items = nact * ((g.ntau + 32) / 32) * S;
-                const size_t smr = (size_t)TvCfg<S>::total * sizeof(double2);
-                CKR(share_sm((const void *)k_tv_ring<S, VIE>, smr));
-                k_tv_ring<S, VIE><<<dim3((unsigned)std::min(items, b->nsm), 1), TvCfg<S>::NTH, smr, st>>>(b->d_groups, sel, n);
-            }
-            CK(cudaGetLastError());
-        }
-        // per problem: G^tv history rows 0..n-1 read (FP32 below the k+1 BDF rows when mixed),
-        // row n written, Cmat column read; shared: the n coefficient blocks
-        const double M = g.ntau + 1;
-        const double n32 = mixed ? std::max(0, n - k - 1) : 0, n64 = n - n32;
-        b->prof_end(NESSI_KERNEL_TV, S * S * ((double)nact * (8.0 * n32 * M + 16.0 * n64 * M + 32.0 * M +
-                                                                 (mixed ? 8.0 * M : 0.0)) + 16.0 * n));
-        b->prof_mark(NESSI_KERNEL_LES_OPERANDS);
-        dim3 grid2((unsigned)((g.ntau + 1 + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR), (unsigned)((nact + LOT - 1) / LOT));
-        k_les_operands_t<S><<<grid2, 256, 0, st>>>(gd, g.d_probs, n, nact);
-        CK(cudaGetLastError());
-        b->prof_end(NESSI_KERNEL_LES_OPERANDS, 32.0 * S * S * (double)nact * (g.ntau + 1));
     }
+    if (!streamed) {
+        if (mixed) {
+            k_tv_mixed<S, VIE><<<dim3((unsigned)((M + 31) / 32), (unsigned)maxact, ng), 256, 0, st>>>(gt, sel, n);
+        } else {
+            // one CTA per SM, shared among the groups; many groups of few items: at least 8 each
+            const int items = maxact * ((M + 31) / 32) * S;
+            const unsigned x = (unsigned)std::min(items, ng == 1 ? b->nsm : std::max(8, b->nsm / sel.ng));
+            const size_t smr = (size_t)TvCfg<S>::total * sizeof(double2);
+            CKR(share_sm((const void *)k_tv_ring<S, VIE>, smr));
+            k_tv_ring<S, VIE><<<dim3(x, ng), TvCfg<S>::NTH, smr, st>>>(gt, sel, n);
+        }
+        CK(cudaGetLastError());
+    }
+    b->prof_end(NESSI_KERNEL_TV, by_tv);
+    b->prof_mark(NESSI_KERNEL_LES_OPERANDS);
+    k_les_operands_t<S><<<dim3((unsigned)((M + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR), (unsigned)((maxact + LOT - 1) / LOT), ng),
+                          256, 0, st>>>(gt, sel, n);
+    CK(cudaGetLastError());
+    b->prof_end(NESSI_KERNEL_LES_OPERANDS, by_vt);
     CK(cudaStreamWaitEvent(st, b->ev_join, 0));
     // tv*vt: gles += Sigma^tv * btv
-    {
-        b->prof_mark(NESSI_KERNEL_GEMM);
-        const double2 *T = S == 1 ? g.stv : g.Tdense;
-        const int MS = (g.ntau + 1) * S;
-        CKR(zgemm_launch(LdRowK{T, ldT, nn, MS}, LdRowN{g.btv, g.ldc, MS, m}, StRow{g.gles, g.ldc, nn, m, alpha, 1},
-                         nn, m, MS, st));
-        b->prof_end(NESSI_KERNEL_GEMM, 8.0 * (double)m * nn * ((g.ntau + 1) * S));
-    }
+    b->prof_mark(NESSI_KERNEL_GEMM);
+    CKR(product_launch<PROD_TVVT>(b, sel, n, st));
+    b->prof_end(NESSI_KERNEL_GEMM, flop_vt);
     // lesser column
-    {
-        b->prof_mark(NESSI_KERNEL_LES);
-        CKR((volterra_class<S, VIE, false>(b, sel, n, st)));
-        b->prof_end(NESSI_KERNEL_LES, 8.0 * S * S * S * (double)nact * tri_h(n));
-    }
+    b->prof_mark(NESSI_KERNEL_LES);
+    CKR((volterra_class<S, VIE, false>(b, sel, n, st)));
+    b->prof_end(NESSI_KERNEL_LES, flop_rec);
     return NESSI_OK;
 }
 
@@ -668,22 +672,22 @@ int mat_dispatch(nessi_batch *b, Group &g, int method, int force_herm) {
 }
 int vie2_mat_dispatch(nessi_batch *b, Group &g, int method) { NESSI_SIZE_SWITCH(vie2_mat_group, b, g, method) }
 
-template <int S> int step_group_any(nessi_batch *b, Group &g, int n, int nact) {
-    return g.vie ? step_group<S, true>(b, g, n, nact) : step_group<S, false>(b, g, n, nact);
+template <int S> int step_class_any(nessi_batch *b, bool vie, const GroupSel &sel, int n) {
+    return vie ? step_class<S, true>(b, sel, n) : step_class<S, false>(b, sel, n);
 }
 
-int step_dispatch(nessi_batch *b, Group &g, int n, int nact) {
-    switch (g.s) {
-        case 1: return step_group_any<1>(b, g, n, nact);
-        case 2: return step_group_any<2>(b, g, n, nact);
-        case 3: return step_group_any<3>(b, g, n, nact);
-        case 4: return step_group_any<4>(b, g, n, nact);
-        case 5: return step_group_any<5>(b, g, n, nact);
-        case 6: return step_group_any<6>(b, g, n, nact);
-        case 7: return step_group_any<7>(b, g, n, nact);
-        case 8: return step_group_any<8>(b, g, n, nact);
+int step_dispatch(nessi_batch *b, int s, bool vie, const GroupSel &sel, int n) {
+    switch (s) {
+        case 1: return step_class_any<1>(b, vie, sel, n);
+        case 2: return step_class_any<2>(b, vie, sel, n);
+        case 3: return step_class_any<3>(b, vie, sel, n);
+        case 4: return step_class_any<4>(b, vie, sel, n);
+        case 5: return step_class_any<5>(b, vie, sel, n);
+        case 6: return step_class_any<6>(b, vie, sel, n);
+        case 7: return step_class_any<7>(b, vie, sel, n);
+        case 8: return step_class_any<8>(b, vie, sel, n);
     }
-    set_err("size1 = %d not supported (1..8)", g.s);
+    set_err("size1 = %d not supported (1..8)", s);
     return NESSI_ERR_ARG;
 }
 
@@ -1044,15 +1048,29 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
         if (n <= g.k) { set_err("%s: n = %d must exceed the solve order %d", name, n, g.k); return NESSI_ERR_ARG; }
     }
     if (!any) { set_err("%s: the batch has no %s group", name, vie ? "VIE2 (nessi_gpu_set_F)" : "Dyson"); return NESSI_ERR_ARG; }
-    for (Group &g : b->groups) {
+    // groups of one size1 step together, NESSI_GSEL at a time
+    std::vector<int> nact(b->groups.size(), 0);
+    for (size_t gi = 0; gi < b->groups.size(); gi++) {
+        const Group &g = b->groups[gi];
         if (g.vie != vie) continue;
-        int nact = 0;
-        for (int i : g.members) nact += b->probs[i].d.nt >= n ? 1 : 0;
-        if (nact == 0) continue;
+        nact[gi] = active_members(b, g, n);
         if (vie)
-            for (int i = 0; i < nact; i++)
+            for (int i = 0; i < nact[gi]; i++)
                 if (!b->probs[g.members[i]].qret) { set_err("%s: Q of problem %d not set", name, g.members[i]); return NESSI_ERR_ARG; }
-        CKR(step_dispatch(b, g, n, nact));
+    }
+    for (int s = 1; s <= NESSI_MAXS; s++) {
+        GroupSel sel;
+        sel.ng = 0;
+        for (size_t gi = 0; gi < b->groups.size(); gi++) {
+            if (b->groups[gi].s == s && nact[gi] > 0) {
+                sel.gid[sel.ng] = (int)gi;
+                sel.nact[sel.ng++] = nact[gi];
+            }
+            if (sel.ng == NESSI_GSEL || (gi + 1 == b->groups.size() && sel.ng > 0)) {
+                CKR(step_dispatch(b, s, vie, sel, n));
+                sel.ng = 0;
+            }
+        }
     }
     return NESSI_OK;
 }
