@@ -401,17 +401,18 @@ __device__ void les_start_block(const GroupDev &g, const ProbDev &p, int n, cons
 // bytes in flight in its own ring in shared memory: a lane copies its 16 bytes with cp.async and
 // reads only those, so the ring needs no barrier, and the copies of the next item are issued while
 // the current one is still summed.  The coefficients a_j, shared by all items of a group, are
-// double-buffered in shared memory and the next chunk waits in registers.  16 x 6 x 512 bytes in
+// double-buffered in shared memory and the next chunk waits in registers.  16 x 8 x 512 bytes in
 // flight per SM are enough for the full HBM rate; with 64 registers a thread the kernel holds half
 // of an SM's registers and a quarter of its shared memory, so that the retarded recursion runs
 // beside it (size1 4, 32 problems, n 1200: stream, recursion and les*adv together 3.2 ms, one after
-// the other 4.1 ms; size1 1, 1024 problems, n 1000: 2.6 and 2.8 ms).  Alone: size1 1, 2 6210, 5680
-// GB/s, size1 4 4260 (register loads, a CTA per 32 tau: 3900), size1 8 2060 (1270).  (Loads into registers go through L1 lines, which a shared-memory heavy neighbour takes
-// away: 6592 -> 5064 GB/s for size1 1 with the carve-out the recursion needs, and without it the two
-// kernels cannot share an SM at all.)
+// the other 4.1 ms; size1 1, 1024 problems, n 1000: 2.6 and 2.8 ms); size1 >= 5 takes 128 registers
+// and the SM.  Alone: size1 1, 2 6400, 6060 GB/s, size1 4 4280 (register loads, a CTA per 32 tau: 3900),
+// size1 8 4010 (1270).  (Loads into registers go through L1 lines, which a shared-memory heavy
+// neighbour takes away: 6592 -> 5064 GB/s for size1 1 with the carve-out the recursion needs, and
+// without it the two kernels cannot share an SM at all.)
 template <int S> struct TvCfg {
     static constexpr int NW = 16, NTH = NW * 32;                       // warps, threads per CTA
-    static constexpr int DEPTH = 6;                                    // plane rows in flight per warp
+    static constexpr int DEPTH = 8;                                    // plane rows in flight per warp
     static constexpr int CHW = S == 1 ? 16 : (S == 2 ? 4 : (S == 3 ? 2 : 1));  // rows per warp and chunk
     static constexpr int CH = CHW * NW, CE = CH * S * S;               // rows, complex of a chunk
     static constexpr int CR = (CE + NTH - 1) / NTH;                    // complex a thread carries to the next
@@ -423,10 +424,10 @@ __device__ __forceinline__ void cp16g(double2 *dst, const double2 *src) {  // pa
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
-// Grid (persistent CTAs, groups).  Copies are not predicated on tau: a lane past ntau reads the next
-// plane or the next row, and row n of every problem exists (n <= nt).
+// Grid (persistent CTAs, groups).  Lanes past ntau copy the previous 32 tau (copies of one address by
+// many lanes are slow: size1 1, M 801: 5580 GB/s, so 6400).
 template <int S, bool VIE>
-__global__ void __launch_bounds__(TvCfg<S>::NTH, 2) k_tv_ring(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
+__global__ void __launch_bounds__(TvCfg<S>::NTH, S <= 4 ? 2 : 1) k_tv_ring(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
     using C = TvCfg<S>;
     constexpr int s2 = S * S, D = C::DEPTH;
     extern __shared__ double2 rsm_[];
@@ -439,13 +440,17 @@ __global__ void __launch_bounds__(TvCfg<S>::NTH, 2) k_tv_ring(const GroupDev *__
     double2 *ring = rsm_ + C::ring + warp * D * 32 + lane, *cbuf = rsm_ + C::coef;
     const double2 *cf = g.tvcoef;
     // ---- the copy stream of this warp: planes b = 0..S-1 of its rows, item after item
-    auto item_base = [&](int it) {
-        return g.probs[it / (S * ntile)].gtv + (long)warp * rowstride + (long)(it % S) * M + (it / S) % ntile * 32 + lane;
+    int lit = R > 0 ? (int)blockIdx.x : items, lrow = 0, lb = 0, lslot = 0;
+    const double2 *lptr = nullptr;
+    auto open_item = [&]() {
+        if (lit >= items) return;
+        const int tau = (lit / S) % ntile * 32 + lane;
+        lptr = g.probs[lit / (S * ntile)].gtv + (long)warp * rowstride + (long)(lit % S) * M +
+               (tau < M ? tau : max(0, tau - 32));
     };
-    int lit = blockIdx.x, lrow = 0, lb = 0, lslot = 0;
-    const double2 *lptr = R > 0 ? item_base(lit) : nullptr;
+    open_item();
     auto copy_next = [&]() {
-        if (lptr) {
+        if (lit < items) {
             cp16g(ring + lslot * 32, lptr);
             if (S > 1 && lb < S - 1) {
                 lb++;
@@ -456,7 +461,7 @@ __global__ void __launch_bounds__(TvCfg<S>::NTH, 2) k_tv_ring(const GroupDev *__
                 if (++lrow == R) {
                     lrow = 0;
                     lit += gridDim.x;
-                    lptr = lit < items ? item_base(lit) : nullptr;
+                    open_item();
                 }
             }
         }
@@ -683,6 +688,70 @@ __global__ void k_tv_relayout(double2 *__restrict__ dst, const double2 *__restri
         const int rem = (int)(i % ((long)s2 * M)), e = rem / M, tau = rem % M;
         const long j = (t * M + tau) * s2 + e;  // libcntr index
         if (to_planes) dst[i] = src[j]; else dst[j] = src[i];
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// One time step t >= 0 between a herm_matrix in device memory and a host slice [ret(t, 0..t) | tv(t, .) |
+// les(0..t, t)] in libcntr's layout, one launch: the kernels read / write the host memory themselves
+// (pinned, mapped), whole lines at a time.  nrow = (t+1) s^2; planes: tv(t, .) is stored as element
+// planes e (ntau+1) + tau (a tile of 32 tau goes through shared memory), else in libcntr's layout; tv32:
+// FP32 copy of the tv row, or null.  Grid: 2 ceil(nrow / 1024) + slice_tv_blocks, 256 threads.
+// ---------------------------------------------------------------------------------------
+__host__ __device__ inline int slice_row_blocks(long nrow) { return (int)((nrow + 1023) / 1024); }
+__host__ __device__ inline int slice_tv_blocks(int M, int s2, int planes) {
+    return planes && s2 > 1 ? (M + 31) / 32 : (int)(((long)M * s2 + 1023) / 1024);
+}
+template <bool PACK>
+__global__ void __launch_bounds__(256) k_slice(double2 *host, double2 *ret, double2 *tv, double2 *les, float2 *tv32,
+                                               long nrow, int M, int s2, int planes) {
+    __shared__ double2 sm[32 * NESSI_MAXS * NESSI_MAXS];
+    const int nb = slice_row_blocks(nrow), blk = blockIdx.x, tid = threadIdx.x;
+    auto move = [&](double2 *dev, double2 *h, long n, long c0) {
+        double2 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const long x = c0 + tid + 256 * i;
+            if (x < n) v[i] = PACK ? dev[x] : h[x];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const long x = c0 + tid + 256 * i;
+            if (x < n) (PACK ? h : dev)[x] = v[i];
+        }
+    };
+    auto to32 = [](double2 v) { return make_float2((float)v.x, (float)v.y); };
+    if (blk < nb) {
+        move(ret, host, nrow, blk * 1024L);
+    } else if (blk < 2 * nb) {
+        move(les, host + nrow + (long)M * s2, nrow, (blk - nb) * 1024L);
+    } else if (!planes || s2 == 1) {
+        const long c0 = (blk - 2 * nb) * 1024L, n = (long)M * s2;
+        move(tv, host + nrow, n, c0);
+        if (!PACK && tv32)
+            for (long x = c0 + tid; x < n && x < c0 + 1024; x += 256) tv32[x] = to32(tv[x]);
+    } else {
+        const int tau0 = (blk - 2 * nb) * 32, cnt = min(32, M - tau0);
+        double2 *h = host + nrow + (long)tau0 * s2;
+        if (!PACK) {
+            for (int x = tid; x < cnt * s2; x += 256) sm[x] = h[x];
+            __syncthreads();
+        }
+        for (int x = tid; x < 32 * s2; x += 256) {
+            const int e = x / 32, l = x % 32;
+            if (l >= cnt) continue;
+            const long i = (long)e * M + tau0 + l;
+            if (PACK) {
+                sm[l * s2 + e] = tv[i];
+            } else {
+                tv[i] = sm[l * s2 + e];
+                if (tv32) tv32[i] = to32(sm[l * s2 + e]);
+            }
+        }
+        if (PACK) {
+            __syncthreads();
+            for (int x = tid; x < cnt * s2; x += 256) h[x] = sm[x];
+        }
     }
 }
 

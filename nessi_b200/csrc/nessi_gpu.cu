@@ -168,6 +168,13 @@ struct nessi_batch {
     GroupDev *d_groups = nullptr;  // the groups' device descriptors, refreshed by sync_groups
     double2 *scratch = nullptr;  // G^tv in libcntr layout during layout conversion (size1 > 1)
     long scratch_n = 0;
+    // pinned staging slots of one time-step slice each, for slices in pageable host memory (allocated
+    // at the first such call, one slice of the largest problem per slot)
+    static constexpr int NSTAGE = 4;
+    char *stage = nullptr;
+    size_t stage_bytes = 0;              // of one slot
+    cudaEvent_t stage_ev[NSTAGE] = {};   // the slot's last reader
+    int stage_next = 0;
     // kernel of the tv row: 1 (default) = k_tv (register loads, every size1), 0 = k_tv_stream
     // (history through shared memory by bulk copies, size1 <= 4; NESSI_TV_KERNEL=stream)
     int tv_kernel = 1;
@@ -854,6 +861,9 @@ int nessi_gpu_batch_destroy(nessi_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (void *q : b->allocs) cudaFree(q);
+    if (b->stage) cudaFreeHost(b->stage);
+    for (cudaEvent_t e : b->stage_ev)
+        if (e) cudaEventDestroy(e);
     for (auto &k : b->kp)
         for (cudaEvent_t e : k.ev) cudaEventDestroy(e);
     if (b->side) { cudaStreamSynchronize(b->side); cudaStreamDestroy(b->side); }
@@ -947,8 +957,56 @@ int nessi_gpu_get_G(nessi_batch *b, int p, void *ret, void *les, void *tv, void 
     return NESSI_OK;
 }
 
+// Device address of a host buffer that is pinned and mapped from its first to its last byte, else
+// null; *pageable tells whether the driver does not know the memory at all.
+static double2 *mapped_host(const void *host, size_t bytes, bool *pageable) {
+    cudaPointerAttributes a0, a1;
+    *pageable = false;
+    if (cudaPointerGetAttributes(&a0, host) != cudaSuccess ||
+        cudaPointerGetAttributes(&a1, (const char *)host + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    *pageable = a0.type == cudaMemoryTypeUnregistered && a1.type == cudaMemoryTypeUnregistered;
+    if (a0.type != cudaMemoryTypeHost || a1.type != cudaMemoryTypeHost || !a0.devicePointer ||
+        (char *)a1.devicePointer - (char *)a0.devicePointer != (long)bytes - 1 || ((size_t)a0.devicePointer & 15))
+        return nullptr;
+    return (double2 *)a0.devicePointer;
+}
+
+// A free staging slot of at least `bytes` (null: no pinned memory, the caller copies without one)
+static char *stage_slot(nessi_batch *b, size_t bytes, int *slot) {
+    if (!b->stage) {
+        size_t most = 0;
+        for (const Group &g : b->groups)
+            most = std::max(most, (size_t)(2L * (g.ntmax + 1) + g.ntau + 1) * g.s * g.s * sizeof(double2));
+        void *q = nullptr;
+        if (cudaHostAlloc(&q, most * nessi_batch::NSTAGE, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        for (auto &e : b->stage_ev)
+            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                cudaFreeHost(q);
+                return nullptr;
+            }
+        b->stage = (char *)q;
+        b->stage_bytes = most;
+    }
+    if (bytes > b->stage_bytes) return nullptr;
+    *slot = b->stage_next;
+    b->stage_next = (b->stage_next + 1) % nessi_batch::NSTAGE;
+    if (cudaEventSynchronize(b->stage_ev[*slot]) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return b->stage + *slot * b->stage_bytes;
+}
+
+// Time step tstp between a herm_matrix on the device and a host slice.  One launch moves the three
+// parts (k_slice): straight from / to pinned memory, else through a pinned slot.  A slice read from
+// pageable memory is copied into a slot first, so the call returns without waiting for the device.
+// Memory of another kind (managed, device, partly pinned) goes through cudaMemcpyAsync.
 static int slice_copy(nessi_batch *b, double2 *ret, double2 *tv, double2 *les, double2 *mat, int nt, int ntau, int s,
-                      int tstp, void *slice, bool to_device, bool tv_planes) {
+                      int tstp, void *slice, bool to_device, bool tv_planes, float2 *tv32 = nullptr) {
     const long s2 = (long)s * s, M = ntau + 1;
     if (tstp < -1 || tstp > nt) { set_err("time step %d out of range [-1, %d]", tstp, nt); return NESSI_ERR_ARG; }
     if (!slice) { set_err("null slice"); return NESSI_ERR_ARG; }
@@ -959,13 +1017,37 @@ static int slice_copy(nessi_batch *b, double2 *ret, double2 *tv, double2 *les, d
     };
     if (tstp == -1) {
         CKR(cp(mat, h, M * s2));
-    } else {
-        const long n1 = tstp + 1;
-        CKR(cp(ret + tri_h(tstp) * s2, h, n1 * s2));
-        if (tv_planes) CKR(tv_transfer(b, tv, h + n1 * s2, tstp, 1, (int)M, s, to_device));
-        else CKR(cp(tv + tstp * M * s2, h + n1 * s2, M * s2));
-        CKR(cp(les + tri_h(tstp) * s2, h + (n1 + M) * s2, n1 * s2));
+        CK(cudaStreamSynchronize(b->stream));
+        return NESSI_OK;
     }
+    const long nrow = (tstp + 1L) * s2, n = 2 * nrow + M * s2;
+    const size_t bytes = (size_t)n * sizeof(double2);
+    double2 *r = ret + tri_h(tstp) * s2, *v = tv + tstp * M * s2, *l = les + tri_h(tstp) * s2;
+    float2 *v32 = tv32 ? tv32 + tstp * M * s2 : nullptr;
+    bool pageable = false;
+    double2 *io = mapped_host(slice, bytes, &pageable);
+    int slot = -1;
+    char *st = !io && pageable ? stage_slot(b, bytes, &slot) : nullptr;
+    if (io || st) {
+        if (st && to_device) std::memcpy(st, slice, bytes);
+        if (st) CK(cudaHostGetDevicePointer((void **)&io, st, 0));
+        const unsigned blocks = (unsigned)(2 * slice_row_blocks(nrow) + slice_tv_blocks((int)M, (int)s2, tv_planes));
+        if (to_device) k_slice<false><<<blocks, 256, 0, b->stream>>>(io, r, v, l, v32, nrow, (int)M, (int)s2, tv_planes);
+        else k_slice<true><<<blocks, 256, 0, b->stream>>>(io, r, v, l, v32, nrow, (int)M, (int)s2, tv_planes);
+        CK(cudaGetLastError());
+        if (st && to_device) {
+            CK(cudaEventRecord(b->stage_ev[slot], b->stream));
+            return NESSI_OK;
+        }
+        CK(cudaStreamSynchronize(b->stream));
+        if (st) std::memcpy(slice, st, bytes);
+        return NESSI_OK;
+    }
+    CKR(cp(r, h, nrow));
+    if (tv_planes) CKR(tv_transfer(b, tv, h + nrow, tstp, 1, (int)M, s, to_device));
+    else CKR(cp(v, h + nrow, M * s2));
+    CKR(cp(l, h + nrow + M * s2, nrow));
+    if (to_device) CKR(refresh32(b, v32, v, M * s2));
     CK(cudaStreamSynchronize(b->stream));
     return NESSI_OK;
 }
@@ -980,13 +1062,8 @@ int nessi_gpu_set_timestep(nessi_batch *b, int p, int tstp, const void *slice) {
     CKR(check_prob(b, p));
     Prob &q = b->probs[p];
     if (tstp == -1) b->groups[q.group].gmat_valid = false;
-    CKR(slice_copy(b, q.gret, q.gtv, q.gles, q.gmat, q.d.nt, q.d.ntau, q.d.size1, tstp, (void *)slice, true, true));
-    if (tstp >= 0) {
-        const long row = (long)(q.d.ntau + 1) * q.d.size1 * q.d.size1;
-        CKR(refresh32(b, q.gtv32 ? q.gtv32 + tstp * row : nullptr, q.gtv + tstp * row, row));
-        CK(cudaStreamSynchronize(b->stream));
-    }
-    return NESSI_OK;
+    return slice_copy(b, q.gret, q.gtv, q.gles, q.gmat, q.d.nt, q.d.ntau, q.d.size1, tstp, (void *)slice, true, true,
+                      q.gtv32);
 }
 
 int nessi_gpu_set_H(nessi_batch *b, int p, const void *H) {
