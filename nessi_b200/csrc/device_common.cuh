@@ -37,6 +37,19 @@ __host__ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
 }
 __host__ __device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.y; }
 
+// ---- overlapped launches (programmatic stream serialization) --------------------------------
+// A kernel launched with launch_chained may start while its predecessor in the stream still runs.  It
+// waits (pdl_wait) before it reads or writes anything another kernel touches; since every kernel of a
+// chain does, "the predecessor has finished" implies that all earlier ones have.  pdl_trigger lets the
+// successor's CTAs take free SM resources once all CTAs of this kernel have started; long streaming
+// kernels leave it out, so that waiting CTAs do not sit beside them.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_entry() {
+    pdl_trigger();
+    pdl_wait();
+}
+
 // ---- integration tables (one order k per launch; indexed [k]) ----------------------
 struct IntegTables {
     double greg[NESSI_K1MAX][NESSI_K2MAX * NESSI_K2MAX];

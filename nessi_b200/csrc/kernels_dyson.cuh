@@ -3,8 +3,8 @@
 // layout in device memory (cntr_herm_matrix_impl.hpp:457-477).
 //
 // One time step n > k runs as
-//   k_prep_problem   s x s inverses of the step matrices (dyson_impl :179-213, :693-706, :983-1011)
-//   k_prep_group     history coefficients for tv, dense copies of Sigma^< and Sigma^tv
+//   k_prep           s x s inverses of the step matrices (dyson_impl :179-213, :693-706, :983-1011),
+//                    history coefficients for tv, dense copies of Sigma^< and Sigma^tv
 //   ret recursion    G^R(n, 0..n): k-block start + Volterra recursion in t'   (:80-222)
 //   k_tv             G^tv(n, 0..ntau): history stream + Matsubara integral + solve (:651-741)
 //   k_les_operands_t right-hand operands of the Sigma-shared products
@@ -63,19 +63,15 @@ struct PrepSel {
 __device__ __forceinline__ long tri(long t) { return t * (t + 1) / 2; }
 
 // ---------------------------------------------------------------------------------------
-// k_prep_problem: Minv_les[n] (= tv step matrix for n > k), Minv_ret[j] for j in [r0, r1]
+// prep_problem: Minv_les[n] (= tv step matrix for n > k), Minv_ret[j] for j in [r0, r1]
 //   tv/les:  mm = i/h bd0 + mu - H(n) - h w0 Sigma^R(n,n)        (dyson_impl :693-699, :983-1004)
 //   ret:     mm = i/h bd0 + mu - H(j)^dagger - h w0 Sigma^R(j,j) (dyson_impl :188-199)
 // ---------------------------------------------------------------------------------------
 // VIE2 ([1 + F] G = Q, cntr_vie2_impl.hpp:60-140, 645-725, 847-990): the step matrices are
 //   tv/les:  mm = 1 + h w0 F^R(j,j);   ret: mm = 1 + h w0 Fcc^R(j,j)
-template <int S, bool VIE = false>
-__global__ void k_prep_problem(const GroupDev *__restrict__ gt, GroupSel sel, PrepSel ps, int n) {
-    if ((int)blockIdx.x >= sel.nact[blockIdx.y]) return;
-    const GroupDev &g = gt[sel.gid[blockIdx.y]];
-    const ProbDev p = g.probs[blockIdx.x];
-    const int k = g.k, s2 = S * S;
-    const int les_lo = ps.les_lo[blockIdx.y], r0 = ps.ret_lo[blockIdx.y], r1 = n - k - 1;
+template <int S, bool VIE>
+__device__ __forceinline__ void prep_problem(const GroupDev &g, const ProbDev &p, int n, int les_lo, int r0) {
+    const int k = g.k, s2 = S * S, r1 = n - k - 1;
     const double h = g.h;
     const double2 ibd0 = cmk(0.0, bd_w(k, 0) / h);
     const double w0 = h * greg_omega(k, 0);
@@ -107,18 +103,17 @@ __global__ void k_prep_problem(const GroupDev *__restrict__ gt, GroupSel sel, Pr
 }
 
 // ---------------------------------------------------------------------------------------
-// k_prep_group: tv coefficients a_j = h w(n,j) Sigma^R(n,j) - [n-k-1<=j<n] (i/h) bd(n-j) 1
+// prep_group: tv coefficients a_j = h w(n,j) Sigma^R(n,j) - [n-k-1<=j<n] (i/h) bd(n-j) 1
 // (conv_impl :942-972 with the BDF terms of dyson_impl :681-692 folded in), and the dense
 // copies of Sigma^< (rows/columns d_lo..n) and Sigma^tv (rows d_lo..n).
 // ---------------------------------------------------------------------------------------
 // VIE2: a_j = -h w(n,j) F^R(n,j) (conv_tv with A = F, moved to the right-hand side).
-template <int S, bool VIE = false>
-__global__ void k_prep_group(const GroupDev *__restrict__ gt, GroupSel sel, PrepSel ps, int n) {
-    const GroupDev &g = gt[sel.gid[blockIdx.y]];
-    const int k = g.k, s2 = S * S, d_lo = ps.d_lo[blockIdx.y];
+template <int S, bool VIE>
+__device__ __forceinline__ void prep_group(const GroupDev &g, int n, int d_lo, int blk, int nblk) {
+    const int k = g.k, s2 = S * S;
     const double h = g.h;
-    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const long nth = (long)gridDim.x * blockDim.x;
+    const long tid = blk * (long)blockDim.x + threadIdx.x;
+    const long nth = (long)nblk * blockDim.x;
     // tv coefficients, j = 0..n-1
     for (long e = tid; e < (long)n * s2; e += nth) {
         int j = (int)(e / s2), ab = (int)(e % s2), a = ab / S, b = ab % S;
@@ -148,6 +143,17 @@ __global__ void k_prep_group(const GroupDev *__restrict__ gt, GroupSel sel, Prep
                     g.stv[((long)t * (g.ntau + 1) + m) * s2 + ab];
             }
     }
+}
+
+// k_prep: the step matrices and the dense operands of a step, one launch: blocks 0..np-1 the step
+// matrices (a problem each), the rest prep_group.  Grid (np + prep_group blocks, groups).
+template <int S, bool VIE>
+__global__ void __launch_bounds__(256) k_prep(const GroupDev *__restrict__ gt, GroupSel sel, PrepSel ps, int n, int np) {
+    pdl_entry();
+    const int y = blockIdx.y, x = blockIdx.x;
+    const GroupDev &g = gt[sel.gid[y]];
+    if (x >= np) prep_group<S, VIE>(g, n, ps.d_lo[y], x - np, (int)gridDim.x - np);
+    else if (x < sel.nact[y]) prep_problem<S, VIE>(g, g.probs[x], n, ps.les_lo[y], ps.ret_lo[y]);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -764,6 +770,7 @@ __global__ void __launch_bounds__(256) k_slice(double2 *host, double2 *ret, doub
 // (conv_sign = -1 for VIE2, whose Matsubara convolution enters the right-hand side with a minus sign.)
 template <int S>
 __global__ void k_mat_operator(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
+    pdl_entry();
     const GroupDev &g = gt[sel.gid[blockIdx.y]];
     const int k = g.k, s2 = S * S, ntau = g.ntau, M = ntau + 1;
     const long KS = (long)M * S;
@@ -817,6 +824,7 @@ template <int S> struct LoCfg {
 template <int S>
 __global__ void __launch_bounds__(256) k_les_operands_t(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
     constexpr int s2 = S * S, LOR = LoCfg<S>::LOR;
+    pdl_entry();
     const GroupDev &g = gt[sel.gid[blockIdx.z]];
     const ProbDev *probs = g.probs;
     const int nact = sel.nact[blockIdx.z];
@@ -891,6 +899,7 @@ __global__ void __launch_bounds__(128, 4) k_zgemm(const GroupDev *__restrict__ g
     LdRowK la;
     LdRowN lb;
     StRow st;
+    pdl_entry();
     const ProdDims d = prod_operands<OP>(gt[sel.gid[blockIdx.z]], n, sel.nact[blockIdx.z], la, lb, st);
     if ((int)blockIdx.y * 32 >= d.M || (int)blockIdx.x * 32 >= d.N) return;
     zgemm_pipe<32, 32>(la, lb, st, blockIdx.y * 32, blockIdx.x * 32, d.K, zsm);
@@ -901,6 +910,7 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_split(const GroupDev *__restri
     LdRowK la;
     LdRowN lb;
     StRow st;
+    pdl_entry();
     const ProdDims d = prod_operands<OP>(gt[sel.gid[blockIdx.z]], n, sel.nact[blockIdx.z], la, lb, st);
     if ((int)blockIdx.y * 32 >= d.M || (int)blockIdx.x * 8 >= d.N) return;
     zgemm_split(la, lb, st, blockIdx.y * 32, blockIdx.x * 8, d.K, red);
@@ -908,5 +918,6 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_split(const GroupDev *__restri
 // one group: the operands in the kernel's parameters (2002 x 512 x 2002 521 us, through the table 542)
 __global__ void __launch_bounds__(256, 2) k_zgemm_split1(LdRowK la, LdRowN lb, StRow st, int K) {
     __shared__ double2 red[8 * 32 * 8];
+    pdl_entry();
     zgemm_split(la, lb, st, blockIdx.y * 32, blockIdx.x * 8, K, red);
 }

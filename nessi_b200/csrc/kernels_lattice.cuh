@@ -22,6 +22,7 @@ __device__ __forceinline__ double poly_interp(int k, int a, int l) {
 // ---------------------------------------------------------------------------------------
 template <int S>
 __global__ void k_extrapolate(GroupDev g, const ProbDev *__restrict__ probs, int n) {
+    pdl_entry();
     const ProbDev p = probs[blockIdx.y];
     const int n1 = n + 1;
     if (n1 > p.nt) return;
@@ -94,6 +95,7 @@ template <int S>
 __global__ void __launch_bounds__(256) k_gloc(GroupDev g, const ProbDev *__restrict__ probs, int nprob, int tstp,
                                               double2 *part, long ldpart) {
     __shared__ double2 red[8][32];
+    pdl_entry();
     const int s2 = S * S, M = g.ntau + 1;
     const long nret = tstp >= 0 ? (long)(tstp + 1) * s2 : 0, ntv = (long)M * s2;
     const long total = tstp >= 0 ? 2 * nret + ntv : ntv;
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(256) k_gloc(GroupDev g, const ProbDev *__restr
 template <int S>
 __global__ void k_gloc_final(GroupDev g, int nprob, int tstp, const double2 *__restrict__ part, long ldpart,
                              int nchunk, LocDev loc) {
+    pdl_entry();
     const int s2 = S * S, M = g.ntau + 1;
     const long nret = tstp >= 0 ? (long)(tstp + 1) * s2 : 0, ntv = (long)M * s2;
     const long total = tstp >= 0 ? 2 * nret + ntv : ntv;
@@ -173,6 +176,7 @@ __device__ __forceinline__ void pol_ret_les(const double2 *gr, const double2 *gl
 
 template <int S>
 __global__ void k_sigma_2b(GroupDev g, LocDev loc, const double2 *__restrict__ udiag, int tstp, SigOut out) {
+    pdl_entry();
     const int s2 = S * S, ntau = g.ntau, M = ntau + 1;
     const double2 ii = cmk(0.0, 1.0);
     const double2 *U0 = udiag;  // U(-1)

@@ -67,9 +67,6 @@ template <int S> struct VbCfg {
     // packed column-major triangle: column l (s scalar columns) holds rows (l+1) s .. NR-1
     static __device__ __forceinline__ int off(int l) { return S * (l * NR - S * (l * (l + 1) / 2)); }
 };
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // T(i, l)[a][b]
 template <int S, bool RET>
 __device__ __forceinline__ const double2 *vol_t(const GroupDev &g, int n, int i, int l, int a, int b) {
@@ -462,6 +459,8 @@ template <int S, bool VIE>
 __global__ void __launch_bounds__(256) k_ret_start(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
     extern __shared__ double2 smem[];
     constexpr int s2 = S * S;
+    pdl_wait();     // before the trigger: k_vol_block reads the step matrices without waiting again
+    pdl_trigger();
     if ((int)blockIdx.x >= sel.nact[blockIdx.y]) return;
     const GroupDev &g = gt[sel.gid[blockIdx.y]];
     const ProbDev p = g.probs[blockIdx.x];
@@ -489,6 +488,8 @@ template <int S, bool VIE>
 __global__ void __launch_bounds__(256) k_les_start(const GroupDev *__restrict__ gt, GroupSel sel, int n) {
     extern __shared__ double2 smem[];
     constexpr int s2 = S * S;
+    pdl_wait();     // before the trigger: k_vol_block reads the step matrices without waiting again
+    pdl_trigger();
     if ((int)blockIdx.x >= sel.nact[blockIdx.y]) return;
     const GroupDev &g = gt[sel.gid[blockIdx.y]];
     const ProbDev p = g.probs[blockIdx.x];

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <map>
 #include <mutex>
 #include <cstdarg>
 #include <cstdio>
@@ -264,19 +265,29 @@ int find_group(nessi_batch *b, int user_id) {
 // ---- per-size kernel launch table ----------------------------------------------------
 // Dynamic shared memory of a kernel, with the SM's L1 / shared split set to all shared: kernels of
 // the two streams of a step can share an SM only when they ask for the same split.
+// The attributes only grow and are set once per kernel and size on a device.
 int share_sm(const void *kernel, size_t smem) {
+    static std::mutex m;
+    static std::map<std::pair<int, const void *>, size_t> done;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(m);
+    auto it = done.find({dev, kernel});
+    if (it != done.end() && it->second >= smem) return NESSI_OK;
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    done[{dev, kernel}] = smem;
     return NESSI_OK;
 }
 
 // Launch that may start before the previous kernel of the stream has finished: the kernel waits for
 // it (griddepcontrol.wait) before it touches anything that an earlier kernel of the chain wrote.
+// Not for the first kernel after a wait for another stream: that one is launched plainly.
 template <class... P, class... A>
-int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -293,7 +304,8 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
 bool zgemm_use_split(long M, long N, long K, int count = 1) {
     return K >= 256 || ((M + 31) / 32) * ((N + 31) / 32) * count < 148;
 }
-template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) {
+// chained: not the first kernel after a wait for another stream
+template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n, bool chained, cudaStream_t st) {
     ProdDims m{0, 0, 0};
     for (int i = 0; i < sel.ng; i++) {
         const Group &g = b->groups[sel.gid[i]];
@@ -302,20 +314,28 @@ template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n,
         m.N = std::max(m.N, d.N);
         m.K = std::max(m.K, d.K);
     }
-    if (zgemm_use_split(m.M, m.N, m.K, sel.ng)) {
+    // les*adv runs beside the tv stream: with enough tiles for an even spread the tiled form, which
+    // reads each operand tile once, leaves the stream more of the memory path (32 x 32 lattice step 9.95
+    // ms, k-split 10.5; 256 two-band k-points 15.9 and 16.4; with 490 to 604 tiles 1 to 2 % slower)
+    const long tiles = (long)((m.M + 31) / 32) * ((m.N + 31) / 32) * sel.ng;
+    const bool beside = OP == PROD_LESADV && b->precision == NESSI_PREC_FP64 && tiles >= 6 * 148;
+    if (!beside && zgemm_use_split(m.M, m.N, m.K, sel.ng)) {
         const dim3 grid((unsigned)((m.N + 7) / 8), (unsigned)((m.M + 31) / 32), (unsigned)sel.ng);
         if (sel.ng == 1) {
             LdRowK la;
             LdRowN lb;
             StRow sto;
             const ProdDims d = prod_operands<OP>(group_dev(b->groups[sel.gid[0]]), n, sel.nact[0], la, lb, sto);
+            if (chained) return launch_chained(k_zgemm_split1, grid, 256, 0, st, la, lb, sto, d.K);
             k_zgemm_split1<<<grid, 256, 0, st>>>(la, lb, sto, d.K);
         } else {
+            if (chained) return launch_chained(k_zgemm_split<OP>, grid, 256, 0, st, b->d_groups, sel, n);
             k_zgemm_split<OP><<<grid, 256, 0, st>>>(b->d_groups, sel, n);
         }
     } else {
         const dim3 grid((unsigned)((m.N + 31) / 32), (unsigned)((m.M + 31) / 32), (unsigned)sel.ng);
         const size_t sm = (size_t)zg::Pipe<32, 32, LdRowK, LdRowN>::total * sizeof(double2);
+        if (chained) return launch_chained(k_zgemm<OP>, grid, 128, sm, st, b->d_groups, sel, n);
         k_zgemm<OP><<<grid, 128, sm, st>>>(b->d_groups, sel, n);
     }
     CK(cudaGetLastError());
@@ -352,12 +372,12 @@ int volterra_class(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) 
         const size_t sm = ret_start_smem<S>(kmax);
         CKR(share_sm((const void *)k_ret_start<S, VIE>, sm));
         k_ret_start<S, VIE><<<dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st>>>(gt, sel, n);
+        CK(cudaGetLastError());
     } else {
         const size_t sm = les_start_smem<S>(kmax);
         CKR(share_sm((const void *)k_les_start<S, VIE>, sm));
-        k_les_start<S, VIE><<<dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st>>>(gt, sel, n);
+        CKR(launch_chained(k_les_start<S, VIE>, dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st, gt, sel, n));
     }
-    CK(cudaGetLastError());
     int wc = 1;
     while (wc < C::WMAX && cols > (long)wc * b->nsm) wc *= 2;
     const dim3 gd((unsigned)((maxact * S + wc - 1) / wc), (unsigned)sel.ng);
@@ -473,19 +493,18 @@ template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, i
             g.gmat_valid = true;
         }
     }
+    // step matrices, tv coefficients, dense Sigma
     b->prof_mark(NESSI_KERNEL_PREP);
-    k_prep_problem<S, VIE><<<dim3((unsigned)maxact, ng), 64, 0, st>>>(gt, sel, ps, n);
-    CK(cudaGetLastError());
-    k_prep_group<S, VIE><<<dim3((unsigned)std::min<long>((prep + 255) / 256, 1184), ng), 256, 0, st>>>(gt, sel, ps, n);
-    CK(cudaGetLastError());
+    const unsigned ngb = (unsigned)std::min<long>((prep + 255) / 256, 1184);
+    CKR(launch_chained(k_prep<S, VIE>, dim3((unsigned)maxact + ngb, ng), 256, 0, st, gt, sel, ps, n, maxact));
     b->prof_end(NESSI_KERNEL_PREP, 0.0);
     // Matsubara part of the tv row: Cmat = K_n Gmat_all (one GEMM per group)
     b->prof_mark(NESSI_KERNEL_MATOP);
-    k_mat_operator<S><<<dim3((unsigned)std::min<long>(((long)M * M * S * S + 255) / 256, 4736), ng), 256, 0, st>>>(gt, sel, n);
-    CK(cudaGetLastError());
+    CKR(launch_chained(k_mat_operator<S>, dim3((unsigned)std::min<long>(((long)M * M * S * S + 255) / 256, 4736), ng), 256, 0,
+                       st, gt, sel, n));
     b->prof_end(NESSI_KERNEL_MATOP, by_mat);
     b->prof_mark(NESSI_KERNEL_GEMM);
-    CKR(product_launch<PROD_MAT>(b, sel, n, st));
+    CKR(product_launch<PROD_MAT>(b, sel, n, true, st));
     b->prof_end(NESSI_KERNEL_GEMM, flop_mat);
     // side stream: retarded row, then les*adv = Ldense * badv (needs only G^R(n, .)); VIE2 moves the
     // convolution to the right-hand side: gles = -(tv*vt + les*adv)
@@ -495,7 +514,7 @@ template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, i
     CKR((volterra_class<S, VIE, true>(b, sel, n, b->side)));
     b->prof_end(NESSI_KERNEL_RET, flop_rec, b->side);
     b->prof_mark(NESSI_KERNEL_GEMM, b->side);
-    CKR(product_launch<PROD_LESADV>(b, sel, n, b->side));
+    CKR(product_launch<PROD_LESADV>(b, sel, n, true, b->side));
     b->prof_end(NESSI_KERNEL_GEMM, flop_les, b->side);
     CK(cudaEventRecord(b->ev_join, b->side));
     // main stream: tv row, then the tv*vt operand
@@ -520,20 +539,21 @@ template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, i
             const unsigned x = (unsigned)std::min(items, ng == 1 ? b->nsm : std::max(8, b->nsm / sel.ng));
             const size_t smr = (size_t)TvCfg<S>::total * sizeof(double2);
             CKR(share_sm((const void *)k_tv_ring<S, VIE>, smr));
+            // launched plainly: started early it takes its SMs before the recursion beside it does
+            // (32 x 32 lattice step 11.3 ms instead of 10.5, 256 two-band k-points 17.2 and 16.4)
             k_tv_ring<S, VIE><<<dim3(x, ng), TvCfg<S>::NTH, smr, st>>>(gt, sel, n);
         }
         CK(cudaGetLastError());
     }
     b->prof_end(NESSI_KERNEL_TV, by_tv);
     b->prof_mark(NESSI_KERNEL_LES_OPERANDS);
-    k_les_operands_t<S><<<dim3((unsigned)((M + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR), (unsigned)((maxact + LOT - 1) / LOT), ng),
-                          256, 0, st>>>(gt, sel, n);
-    CK(cudaGetLastError());
+    CKR(launch_chained(k_les_operands_t<S>, dim3((unsigned)((M + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR),
+                                                 (unsigned)((maxact + LOT - 1) / LOT), ng), 256, 0, st, gt, sel, n));
     b->prof_end(NESSI_KERNEL_LES_OPERANDS, by_vt);
     CK(cudaStreamWaitEvent(st, b->ev_join, 0));
     // tv*vt: gles += Sigma^tv * btv
     b->prof_mark(NESSI_KERNEL_GEMM);
-    CKR(product_launch<PROD_TVVT>(b, sel, n, st));
+    CKR(product_launch<PROD_TVVT>(b, sel, n, false, st));
     b->prof_end(NESSI_KERNEL_GEMM, flop_vt);
     // lesser column
     b->prof_mark(NESSI_KERNEL_LES);
@@ -618,9 +638,7 @@ int active_members(const nessi_batch *b, const Group &g, int tstp) {
 template <int S> int extrap_group(nessi_batch *b, Group &g, int n) {
     const long work = ((long)g.ntau + 1 + 2L * (n + 2)) * S * S;
     dim3 grid((unsigned)std::min<long>((work + 255) / 256, 64), (unsigned)g.members.size());
-    k_extrapolate<S><<<grid, 256, 0, b->stream>>>(group_dev(g), g.d_probs, n);
-    CK(cudaGetLastError());
-    return NESSI_OK;
+    return launch_chained(k_extrapolate<S>, grid, 256, 0, b->stream, group_dev(g), g.d_probs, n);
 }
 
 template <int S> int gloc_group(nessi_batch *b, Group &g, int tstp) {
@@ -629,13 +647,10 @@ template <int S> int gloc_group(nessi_batch *b, Group &g, int tstp) {
     const long M = g.ntau + 1, s2 = (long)S * S;
     const long total = tstp >= 0 ? (2L * (tstp + 1) + M) * s2 : M * s2;
     const int nchunk = (nact + GLOC_CHUNK - 1) / GLOC_CHUNK;
-    k_gloc<S><<<dim3((unsigned)((total + 31) / 32), (unsigned)nchunk), dim3(32, 8), 0, b->stream>>>(
-        group_dev(g), g.d_probs, nact, tstp, g.gloc_part, g.gloc_ld);
-    CK(cudaGetLastError());
-    k_gloc_final<S><<<(unsigned)std::min<long>((total + 255) / 256, 1184), 256, 0, b->stream>>>(
-        group_dev(g), nact, tstp, g.gloc_part, g.gloc_ld, nchunk, g.loc);
-    CK(cudaGetLastError());
-    return NESSI_OK;
+    CKR(launch_chained(k_gloc<S>, dim3((unsigned)((total + 31) / 32), (unsigned)nchunk), dim3(32, 8), 0, b->stream,
+                       group_dev(g), g.d_probs, nact, tstp, g.gloc_part, g.gloc_ld));
+    return launch_chained(k_gloc_final<S>, dim3((unsigned)std::min<long>((total + 255) / 256, 1184)), 256, 0, b->stream,
+                          group_dev(g), nact, tstp, g.gloc_part, g.gloc_ld, nchunk, g.loc);
 }
 
 void sigma_changed(Group &g, int tstp) {
@@ -649,9 +664,8 @@ template <int S> int sigma2b_group(nessi_batch *b, Group &g, int tstp) {
     const long M = g.ntau + 1, s2 = (long)S * S;
     const long work = tstp >= 0 ? ((long)tstp + 1 + M) * s2 : M * s2;
     SigOut o{g.sret, g.sles, g.stv, g.smat};
-    k_sigma_2b<S><<<(unsigned)std::min<long>((work + 255) / 256, 1184), 256, 0, b->stream>>>(group_dev(g), g.loc,
-                                                                                           g.U, tstp, o);
-    CK(cudaGetLastError());
+    CKR(launch_chained(k_sigma_2b<S>, dim3((unsigned)std::min<long>((work + 255) / 256, 1184)), 256, 0, b->stream,
+                       group_dev(g), g.loc, g.U, tstp, o));
     sigma_changed(g, tstp);
     return NESSI_OK;
 }
