@@ -7,8 +7,17 @@
 //   k_conv_tv    C^tv(n, tau)              convolution_timestep_tv       (:901-1073)
 //   k_conv_les   C^<(j, n)                 convolution_timestep_les_*    (:1075-1580)
 //   k_conv_mat   C^mat(tau)                convolution_matsubara         (:560-605)
-// Thread per output element (j or tau, then the s x s entry); work items of a problem are
-// spread over blockIdx.x, problems over blockIdx.y.
+// and k_conv_*_start for n < k, where the sums run to k with the hermitian continuations.  Work items
+// of a problem are spread over blockIdx.x, problems over blockIdx.y.
+//
+// Bound of the steps n >= k: memory, the operands' triangles and tv rows once (A^R, B^R, A^<, A^tv,
+// B^tv).  The lanes of a warp follow the index that is contiguous in memory and the sums are split
+// over the warps of a CTA: k_conv_ret and k_conv_tv have a lane per (output index, column b), every
+// warp takes each 8th term; k_conv_les has a CTA per JW consecutive rows j, a lane per term m, so that
+// the right-hand blocks are loaded once for the JW rows and a column access A^<(j.., m) is a whole
+// line.  Measured on a B200, 16 problems of size1 2, n 600, ntau 400 (ret / tv / les, us): a thread per
+// output element, each summing alone, took 333 / 453 / 987; this form 81 / 90 / 228 (3.0 TB/s of
+// operand bytes; one problem 137 us in all, before 1150).
 #pragma once
 #include "device_common.cuh"
 
@@ -110,14 +119,12 @@ __device__ double2 mat_int1(const double2 *A, const double2 *B, int m, int ntau,
 }
 
 // ---------------------------------------------------------------------------------------
-// k_conv_ret: C^R(n,j) = h sum_m W(j,m) A^R(n,m) B^R(m,j) (convolution_timestep_ret, :741-899).
-//   n >= k: m = j..n with W = gregory_weights(n-j, n-m) for m - j <= k, else 1 (m < n-k) or
-//           omega(n-m); for j > n-k also m = n-k..j-1 with B^R(m,j) = -Bcc^R(j,m)^dagger.
+// k_conv_ret_start: C^R(n,j) = h sum_m W(j,m) A^R(n,m) B^R(m,j) (convolution_timestep_ret, :741-899).
 //   n < k:  m = 0..k with polynomial weights poly_integration(j, n, m) and the continuations
 //           A^R(n,m) = -Acc^R(m,n)^dagger (m > n), B^R(m,j) = -Bcc^R(j,m)^dagger (m < j).
 // ---------------------------------------------------------------------------------------
 template <int S>
-__global__ void k_conv_ret(ConvBatch cb, int n) {
+__global__ void k_conv_ret_start(ConvBatch cb, int n) {
     constexpr int s2 = S * S;
     const ConvProb &P = cb.p[blockIdx.y];
     const int k = cb.k;
@@ -125,19 +132,7 @@ __global__ void k_conv_ret(ConvBatch cb, int n) {
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < (long)(n + 1) * s2; e += (long)gridDim.x * blockDim.x) {
         const int j = (int)(e / s2), ab = (int)(e % s2), a = ab / S, b = ab % S;
         double2 acc = cmk(0, 0);
-        if (n >= k) {
-            for (int m = n; m >= j; m--) {
-                double w;
-                if (m - j <= k) w = greg_w(k, n - j, n - m);
-                else w = m < n - k ? 1.0 : greg_omega(k, n - m);
-                acc = cfma(cmk(w, 0), emul<S>(P.A.ret + (ctri(n) + m) * s2, P.B.ret + (ctri(m) + j) * s2, a, b), acc);
-            }
-            for (int m = (n - k > 0 ? n - k : 0); m < j; m++) {
-                const double w = greg_w(k, n - j, n - m);
-                acc = cfma(cmk(-w, 0), emul_ad<S>(P.A.ret + (ctri(n) + m) * s2, P.Bcc.ret + (ctri(j) + m) * s2, a, b),
-                           acc);
-            }
-        } else {
+        {
             for (int m = 0; m <= k; m++) {
                 double w = poly_int(k, j, n, m);
                 double2 t = cmk(0, 0);
@@ -156,12 +151,12 @@ __global__ void k_conv_ret(ConvBatch cb, int n) {
 }
 
 // ---------------------------------------------------------------------------------------
-// k_conv_tv: C^tv(n,tau) = dtau matsubara_integral_2(A^tv(n,.), B^mat)(tau)
+// k_conv_tv_start: C^tv(n,tau) = dtau matsubara_integral_2(A^tv(n,.), B^mat)(tau)
 //                        + h sum_{j=0}^{max(n,k)} w(n,j) A'(n,j) B^tv(j,tau)   (:901-1073)
 // with A'(n,j) = A^R(n,j) (j <= n) or -Acc^R(j,n)^dagger.
 // ---------------------------------------------------------------------------------------
 template <int S>
-__global__ void k_conv_tv(ConvBatch cb, int n) {
+__global__ void k_conv_tv_start(ConvBatch cb, int n) {
     constexpr int s2 = S * S;
     const ConvProb &P = cb.p[blockIdx.y];
     const int k = cb.k, ntau = cb.ntau, M = ntau + 1, n1 = n > k ? n : k;
@@ -182,7 +177,7 @@ __global__ void k_conv_tv(ConvBatch cb, int n) {
 }
 
 // ---------------------------------------------------------------------------------------
-// k_conv_les: C^<(j,n), j = 0..n (convolution_timestep_les, :1525-1580) as the sum of
+// k_conv_les_start: C^<(j,n), j = 0..n (convolution_timestep_les, :1525-1580) as the sum of
 //   tv*vt   sum_m w(ntau,m) A^tv(j,m) (-i dtau)(-sig_A) Bcc^tv(n,ntau-m)^dagger      (:1075-1242)
 //   les*adv sum_m L(j,m) badv(m), L = A^< or -Acc^<(m,j)^dagger (m < j),
 //           badv(m) = h w(n,m) Bcc^R(n,m)^dagger (m <= n) or -h w(n,m) B^R(m,n)       (:1244-1394)
@@ -190,7 +185,7 @@ __global__ void k_conv_tv(ConvBatch cb, int n) {
 //           bl(m) = h B^<(m,n) (m <= n) or -h Bcc^<(n,m)^dagger                        (:1396-1523)
 // ---------------------------------------------------------------------------------------
 template <int S>
-__global__ void k_conv_les(ConvBatch cb, int n) {
+__global__ void k_conv_les_start(ConvBatch cb, int n) {
     constexpr int s2 = S * S;
     const ConvProb &P = cb.p[blockIdx.y];
     const int k = cb.k, ntau = cb.ntau, M = ntau + 1, n1 = n > k ? n : k;
@@ -233,6 +228,238 @@ __global__ void k_conv_les(ConvBatch cb, int n) {
                 acc = cfma(cmk(-w, 0), t, acc);
             }
         P.C.les[(ctri(n) + j) * s2 + ab] = acc;
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// k_conv_ret, n >= k: C^R(n,j) = h sum_m W(j,m) A^R(n,m) B^R(m,j), m = j..n with W =
+// gregory_weights(n-j, n-m) for m - j <= k, else 1 (m < n-k) or omega(n-m); for j > n-k also
+// m = n-k..j-1 with B^R(m,j) = -Bcc^R(j,m)^dagger.  Lane = (j, b), 8 warps split m.
+// ---------------------------------------------------------------------------------------
+template <int S>
+__global__ void __launch_bounds__(256) k_conv_ret(ConvBatch cb, int n) {
+    constexpr int s2 = S * S;
+    __shared__ double2 red[8 * 32 * S];
+    const ConvProb &P = cb.p[blockIdx.y];
+    const int k = cb.k, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + lane, j = x / S, b = x % S, j0 = (int)(blockIdx.x * 32) / S;
+    const bool live = j <= n;
+    double2 acc[S];
+#pragma unroll
+    for (int a = 0; a < S; a++) acc[a] = cmk(0, 0);
+    const double2 *A = P.A.ret + ctri(n) * s2;
+    const int mlo = min(j0, n - k);
+#pragma unroll 4
+    for (int m = mlo + warp; m <= n; m += 8) {
+        if (!live || (m < j && m < n - k)) continue;
+        double2 y[S];
+        double w;
+        if (m >= j) {
+            const double2 *B = P.B.ret + (ctri(m) + j) * s2 + b;
+#pragma unroll
+            for (int c = 0; c < S; c++) y[c] = B[c * S];
+            w = m - j <= k ? greg_w(k, n - j, n - m) : (m < n - k ? 1.0 : greg_omega(k, n - m));
+        } else {
+            const double2 *B = P.Bcc.ret + (ctri(j) + m) * s2 + b * S;
+#pragma unroll
+            for (int c = 0; c < S; c++) y[c] = cconj(B[c]);
+            w = -greg_w(k, n - j, n - m);
+        }
+#pragma unroll
+        for (int c = 0; c < S; c++) y[c] = cscale(y[c], w);
+#pragma unroll
+        for (int a = 0; a < S; a++)
+#pragma unroll
+            for (int c = 0; c < S; c++) acc[a] = cfma(A[(long)m * s2 + a * S + c], y[c], acc[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < S; a++) red[(a * 8 + warp) * 32 + lane] = acc[a];
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * S; e += 256) {
+        const int a = e / 32, l = e % 32, xx = blockIdx.x * 32 + l;
+        double2 v = red[a * 256 + l];
+#pragma unroll
+        for (int w = 1; w < 8; w++) v = cadd(v, red[a * 256 + w * 32 + l]);
+        if (xx / S <= n) P.C.ret[(ctri(n) + xx / S) * s2 + a * S + xx % S] = cscale(v, cb.h);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// k_conv_tv, n >= k: C^tv(n,tau) = dtau matsubara_integral_2(A^tv(n,.), B^mat)(tau)
+//                               + h sum_{j=0}^{n} w(n,j) A^R(n,j) B^tv(j,tau)   (:901-1073)
+// Lane = (tau, b), 8 warps split j and the Matsubara sum (matsubara_integral_2 as in mat_int2).
+// ---------------------------------------------------------------------------------------
+// mat += w A B, column b of the block product (B points at column b)
+template <int S>
+__device__ __forceinline__ void cv_mat(double2 *mat, double w, const double2 *A, const double2 *B) {
+#pragma unroll
+    for (int c = 0; c < S; c++) {
+        const double2 y = cscale(B[c * S], w);
+#pragma unroll
+        for (int a = 0; a < S; a++) mat[a] = cfma(A[a * S + c], y, mat[a]);
+    }
+}
+template <int S>
+__global__ void __launch_bounds__(256) k_conv_tv(ConvBatch cb, int n) {
+    constexpr int s2 = S * S;
+    __shared__ double2 red[8 * 32 * S];
+    const ConvProb &P = cb.p[blockIdx.y];
+    const int k = cb.k, ntau = cb.ntau, M = ntau + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + lane, m = min(x / S, ntau), b = x % S, r = ntau - m;
+    const double h = cb.h, dtau = cb.beta / ntau, sg = (double)cb.sig_b;
+    double2 acc[S], mat[S];
+#pragma unroll
+    for (int a = 0; a < S; a++) acc[a] = mat[a] = cmk(0, 0);
+    const double2 *A = P.A.ret + ctri(n) * s2, *B = P.B.tv + (long)m * s2 + b;
+#pragma unroll 4
+    for (int j = warp; j <= n; j += 8) {
+        const double w = h * greg_w(k, n, j);
+        double2 y[S];
+#pragma unroll
+        for (int c = 0; c < S; c++) y[c] = cscale(B[(long)j * M * s2 + c * S], w);
+#pragma unroll
+        for (int a = 0; a < S; a++)
+#pragma unroll
+            for (int c = 0; c < S; c++) acc[a] = cfma(A[(long)j * s2 + a * S + c], y[c], acc[a]);
+    }
+    const double2 *At = P.A.tv + (long)n * M * s2, *Bm = P.B.mat + b;
+    for (int l = warp; l <= ntau; l += 8) {
+        if (r >= k && l <= r) cv_mat<S>(mat, greg_w(k, r, l), At + (long)(m + l) * s2, Bm + (long)l * s2);
+        if (m >= k && l <= m) cv_mat<S>(mat, sg * greg_w(k, m, l), At + (long)(m - l) * s2, Bm + (long)(ntau - l) * s2);
+    }
+    if ((r > 0 && r < k) || (m > 0 && m < k))
+        for (int e = warp; e < (k + 1) * (k + 1); e += 8) {
+            const int l = e / (k + 1), jj = e % (k + 1);
+            if (r > 0 && r < k) cv_mat<S>(mat, rcorr_w(k, r, l, jj), At + (long)(ntau - l) * s2, Bm + (long)jj * s2);
+            if (m > 0 && m < k) cv_mat<S>(mat, sg * rcorr_w(k, m, l, jj), At + (long)jj * s2, Bm + (long)(ntau - l) * s2);
+        }
+#pragma unroll
+    for (int a = 0; a < S; a++)
+        red[(a * 8 + warp) * 32 + lane] = cmk(fma(dtau, mat[a].x, acc[a].x), fma(dtau, mat[a].y, acc[a].y));
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * S; e += 256) {
+        const int a = e / 32, l = e % 32, xx = blockIdx.x * 32 + l;
+        double2 v = red[a * 256 + l];
+#pragma unroll
+        for (int w = 1; w < 8; w++) v = cadd(v, red[a * 256 + w * 32 + l]);
+        if (xx / S <= ntau) P.C.tv[((long)n * M + xx / S) * s2 + a * S + xx % S] = v;
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// k_conv_les, n >= k: C^<(j,n), j = 0..n, as the sum of
+//   tv*vt   sum_m w(ntau,m) A^tv(j,m) (-i dtau)(-sig_A) Bcc^tv(n,ntau-m)^dagger      (:1075-1242)
+//   les*adv sum_m L(j,m) badv(m), L = A^< or -Acc^<(m,j)^dagger (m < j),
+//           badv(m) = h w(n,m) Bcc^R(n,m)^dagger                                      (:1244-1394)
+//   ret*les sum_{m<=j} w(j,m) A^R(j,m) h B^<(m,n) [- sum_{m=j+1}^{k} w(j,m) Acc^R(m,j)^dagger h B^<(m,n),
+//           j < k]                                                                    (:1396-1523)
+// A CTA of 4 warps takes JW rows j; lanes split m; CB columns b of the s x s blocks at a time.
+// ---------------------------------------------------------------------------------------
+template <int S> struct CvCfg {
+    static constexpr int JW = S == 1 ? 8 : (S == 2 ? 4 : (S == 3 ? 2 : 1));
+    static constexpr int CB = S <= 4 ? S : 2;
+};
+// acc += w L' R, L' = L or (tr) L^dagger, an s x s block; R s x CB
+template <int S, int CB>
+__device__ __forceinline__ void cv_fold(double2 (*acc)[CB], const double2 *L, bool tr, double w, const double2 (*R)[CB]) {
+#pragma unroll
+    for (int a = 0; a < S; a++)
+#pragma unroll
+        for (int c = 0; c < S; c++) {
+            double2 l = L[tr ? c * S + a : a * S + c];
+            l = cmk(l.x * w, l.y * (tr ? -w : w));
+#pragma unroll
+            for (int e = 0; e < CB; e++) acc[a][e] = cfma(l, R[c][e], acc[a][e]);
+        }
+}
+template <int S>
+__global__ void __launch_bounds__(128) k_conv_les(ConvBatch cb, int n) {
+    constexpr int s2 = S * S, JW = CvCfg<S>::JW, CB = CvCfg<S>::CB, NE = JW * S * CB;
+    __shared__ double2 red[NE * 4];
+    const ConvProb &P = cb.p[blockIdx.y];
+    const int k = cb.k, ntau = cb.ntau, M = ntau + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double h = cb.h, dtau = cb.beta / ntau, fvt = dtau * (double)cb.sig_a;  // (-i dtau)(-sig_A) = i fvt
+    const int j0 = blockIdx.x * JW;
+    for (int c0 = 0; c0 < S; c0 += CB) {
+        double2 acc[JW][S][CB];
+#pragma unroll
+        for (int q = 0; q < JW; q++)
+#pragma unroll
+            for (int a = 0; a < S; a++)
+#pragma unroll
+                for (int e = 0; e < CB; e++) acc[q][a][e] = cmk(0, 0);
+        double2 R[S][CB];
+        // tv*vt
+        for (int m = tid; m <= ntau; m += 128) {
+            const double w = fvt * greg_w(k, ntau, m);
+            const double2 *B = P.Bcc.tv + ((long)n * M + ntau - m) * s2;
+#pragma unroll
+            for (int c = 0; c < S; c++)
+#pragma unroll
+                for (int e = 0; e < CB; e++) {  // i w B^dagger
+                    const double2 v = c0 + e < S ? B[(c0 + e) * S + c] : cmk(0, 0);
+                    R[c][e] = cmk(w * v.y, w * v.x);
+                }
+#pragma unroll
+            for (int q = 0; q < JW; q++)
+                cv_fold<S, CB>(acc[q], P.A.tv + ((long)min(j0 + q, n) * M + m) * s2, false, 1.0, R);
+        }
+        // les*adv
+        for (int m = tid; m <= n; m += 128) {
+            const double w = h * greg_w(k, n, m);
+            const double2 *B = P.Bcc.ret + (ctri(n) + m) * s2;
+#pragma unroll
+            for (int c = 0; c < S; c++)
+#pragma unroll
+                for (int e = 0; e < CB; e++) R[c][e] = c0 + e < S ? cscale(cconj(B[(c0 + e) * S + c]), w) : cmk(0, 0);
+#pragma unroll
+            for (int q = 0; q < JW; q++) {
+                const int j = min(j0 + q, n);
+                const bool up = m >= j;
+                const double2 *L = up ? P.A.les + (ctri(m) + j) * s2 : P.Acc.les + (ctri(j) + m) * s2;
+                cv_fold<S, CB>(acc[q], L, !up, up ? 1.0 : -1.0, R);
+            }
+        }
+        // ret*les (rows j < k: to k, with the continuation of A)
+        const int jmax = min(j0 + JW - 1, n), mhi = max(jmax, j0 < k ? k : 0);
+        for (int m = tid; m <= mhi; m += 128) {
+            const double2 *B = P.B.les + (ctri(n) + m) * s2;
+#pragma unroll
+            for (int c = 0; c < S; c++)
+#pragma unroll
+                for (int e = 0; e < CB; e++) R[c][e] = c0 + e < S ? cscale(B[c * S + c0 + e], h) : cmk(0, 0);
+#pragma unroll
+            for (int q = 0; q < JW; q++) {
+                const int j = min(j0 + q, n);
+                if (m > j && (j >= k || m > k)) continue;
+                const bool low = m <= j;
+                const double w = low ? greg_w(k, j, m) : -greg_w(k, j, m);
+                const double2 *L = low ? P.A.ret + (ctri(j) + m) * s2 : P.Acc.ret + (ctri(m) + j) * s2;
+                cv_fold<S, CB>(acc[q], L, !low, w, R);
+            }
+        }
+        // sum over the lanes, then over the warps
+#pragma unroll
+        for (int q = 0; q < JW; q++)
+#pragma unroll
+            for (int a = 0; a < S; a++)
+#pragma unroll
+                for (int e = 0; e < CB; e++) {
+                    double2 v = acc[q][a][e];
+#pragma unroll
+                    for (int off = 16; off > 0; off >>= 1) {
+                        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+                        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+                    }
+                    if (lane == 0) red[((q * S + a) * CB + e) * 4 + warp] = v;
+                }
+        __syncthreads();
+        for (int x = tid; x < NE; x += 128) {
+            const int q = x / (S * CB), a = (x / CB) % S, e = x % CB;
+            const double2 v = cadd(cadd(red[x * 4], red[x * 4 + 1]), cadd(red[x * 4 + 2], red[x * 4 + 3]));
+            if (j0 + q <= n && c0 + e < S) P.C.les[(ctri(n) + j0 + q) * s2 + a * S + c0 + e] = v;
+        }
+        __syncthreads();
     }
 }
 

@@ -1762,11 +1762,20 @@ template <int S> int conv_launch(const ConvBatch &cb, int n, cudaStream_t st) {
         CK(cudaGetLastError());
         return NESSI_OK;
     }
-    k_conv_ret<S><<<dim3(blocks((n + 1) * s2), cb.count), 128, 0, st>>>(cb, n);
-    CK(cudaGetLastError());
-    k_conv_tv<S><<<dim3(blocks(M * s2), cb.count), 128, 0, st>>>(cb, n);
-    CK(cudaGetLastError());
-    k_conv_les<S><<<dim3(blocks((n + 1) * s2), cb.count), 128, 0, st>>>(cb, n);
+    if (n < cb.k) {
+        k_conv_ret_start<S><<<dim3(blocks((n + 1) * s2), cb.count), 128, 0, st>>>(cb, n);
+        CK(cudaGetLastError());
+        k_conv_tv_start<S><<<dim3(blocks(M * s2), cb.count), 128, 0, st>>>(cb, n);
+        CK(cudaGetLastError());
+        k_conv_les_start<S><<<dim3(blocks((n + 1) * s2), cb.count), 128, 0, st>>>(cb, n);
+    } else {
+        const unsigned y = (unsigned)cb.count;
+        k_conv_ret<S><<<dim3((unsigned)(((n + 1) * S + 31) / 32), y), 256, 0, st>>>(cb, n);
+        CK(cudaGetLastError());
+        k_conv_tv<S><<<dim3((unsigned)((M * S + 31) / 32), y), 256, 0, st>>>(cb, n);
+        CK(cudaGetLastError());
+        k_conv_les<S><<<dim3((unsigned)(n / CvCfg<S>::JW + 1), y), 128, 0, st>>>(cb, n);
+    }
     CK(cudaGetLastError());
     return NESSI_OK;
 }
