@@ -83,82 +83,135 @@ __device__ __forceinline__ double rcorr_w(int k, int m, int j, int l) {
     return c_tab.rcorr[k][((m - 1) * NESSI_K1MAX + j) * NESSI_K1MAX + l];
 }
 
-// ---- execution groups for the small dense block solves --------------------------------------
-// CtaExec: all threads of the block; WarpExec: the 32 lanes of one warp.
-struct CtaExec {
-    __device__ __forceinline__ int t() const { return threadIdx.x; }
-    __device__ __forceinline__ int n() const { return blockDim.x; }
-    __device__ __forceinline__ void sync() const { __syncthreads(); }
-};
-struct WarpExec {
-    int lane;
-    __device__ __forceinline__ int t() const { return lane; }
-    __device__ __forceinline__ int n() const { return 32; }
-    __device__ __forceinline__ void sync() const { __syncwarp(); }
-};
-
-// ---- dense solve A X = B (n x n, nrhs columns), partial pivoting, by an execution group ------
+// ---- dense solve A X = B (n x n, nrhs columns), partial pivoting, by the whole CTA -------------
 // A (n x n, row-major, lda = n) and B (n x nrhs, row-major) live in shared memory and
-// are overwritten; on return B holds X.  Every member of the group must call it.
+// are overwritten; on return B holds X.  Every thread of the CTA must call it.
 // Returns nonzero in *status (shared) if a zero pivot was met.
-template <class X>
-__device__ inline void grp_solve(const X &x, double2 *A, double2 *B, int n, int nrhs, int *s_piv, int *status) {
-    const int tid = x.t(), nth = x.n();
+// Bound: the chain of n columns; per column the pivot search (the first warp), one division per
+// row, and the update of the rest, then as many steps of a column-wise back substitution.
+__device__ inline void grp_solve(double2 *A, double2 *B, int n, int nrhs, int *s_piv, int *status) {
+    const int tid = threadIdx.x, nth = blockDim.x;
     for (int c = 0; c < n; c++) {
-        if (tid == 0) {
+        if (tid < 32) {
             int p = c;
-            double best = cabs2(A[c * n + c]);
-            for (int i = c + 1; i < n; i++) {
-                double a = cabs2(A[i * n + c]);
+            double best = -1.0;
+            for (int i = c + tid; i < n; i += 32) {
+                const double a = cabs2(A[i * n + c]);
                 if (a > best) { best = a; p = i; }
             }
-            *s_piv = p;
-            if (best == 0.0) *status = 1;
-        }
-        x.sync();
-        int p = *s_piv;
-        if (p != c) {
-            for (int j = tid; j < n + nrhs; j += nth) {
-                if (j < n) {
-                    double2 t = A[c * n + j]; A[c * n + j] = A[p * n + j]; A[p * n + j] = t;
-                } else {
-                    int jj = j - n;
-                    double2 t = B[c * nrhs + jj]; B[c * nrhs + jj] = B[p * nrhs + jj]; B[p * nrhs + jj] = t;
-                }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                const double ob = __shfl_xor_sync(0xffffffffu, best, off);
+                const int op = __shfl_xor_sync(0xffffffffu, p, off);
+                if (ob > best || (ob == best && op < p)) { best = ob; p = op; }
+            }
+            if (tid == 0) {
+                *s_piv = p;
+                if (best == 0.0) *status = 1;
             }
         }
-        x.sync();
+        __syncthreads();
+        const int p = *s_piv;
+        if (p != c)
+            for (int j = tid; j < n + nrhs; j += nth) {
+                double2 *u = j < n ? A + c * n + j : B + c * nrhs + j - n, *v = j < n ? A + p * n + j : B + p * nrhs + j - n;
+                const double2 t = *u;
+                *u = *v;
+                *v = t;
+            }
+        __syncthreads();
         double2 piv = A[c * n + c];
         if (piv.x == 0.0 && piv.y == 0.0) piv = cmk(1.0, 0.0);  // status already flagged
+        for (int i = c + 1 + tid; i < n; i += nth) A[i * n + c] = cdiv(A[i * n + c], piv);
+        __syncthreads();
         // eliminate rows below c
         const int w = n - c - 1 + nrhs;  // columns c+1..n-1 and rhs
         for (int idx = tid; idx < (n - c - 1) * w; idx += nth) {
-            int i = c + 1 + idx / w, j = idx % w;
-            double2 f = cdiv(A[i * n + c], piv);
-            if (j < n - c - 1) {
-                int jj = c + 1 + j;
-                A[i * n + jj] = csub(A[i * n + jj], cmul(f, A[c * n + jj]));
-            } else {
-                int jj = j - (n - c - 1);
-                B[i * nrhs + jj] = csub(B[i * nrhs + jj], cmul(f, B[c * nrhs + jj]));
-            }
+            const int i = c + 1 + idx / w, j = idx % w;
+            const double2 f = A[i * n + c];
+            double2 *u = j < n - c - 1 ? A + i * n + c + 1 + j : B + i * nrhs + j - (n - c - 1);
+            const double2 *v = j < n - c - 1 ? A + c * n + c + 1 + j : B + c * nrhs + j - (n - c - 1);
+            *u = csub(*u, cmul(f, *v));
         }
-        x.sync();
-        // column c below the pivot is no longer needed (implicit zeros)
+        __syncthreads();
     }
-    // back substitution, one rhs column per thread
+    // back substitution, column by column
     for (int i = n - 1; i >= 0; i--) {
-        for (int j = tid; j < nrhs; j += nth) {
-            double2 acc = B[i * nrhs + j];
-            for (int l = i + 1; l < n; l++) acc = csub(acc, cmul(A[i * n + l], B[l * nrhs + j]));
-            B[i * nrhs + j] = cdiv(acc, A[i * n + i].x == 0.0 && A[i * n + i].y == 0.0 ? cmk(1, 0) : A[i * n + i]);
+        double2 d = A[i * n + i];
+        if (d.x == 0.0 && d.y == 0.0) d = cmk(1.0, 0.0);
+        for (int j = tid; j < nrhs; j += nth) B[i * nrhs + j] = cdiv(B[i * nrhs + j], d);
+        __syncthreads();
+        for (int idx = tid; idx < i * nrhs; idx += nth) {
+            const int r = idx / nrhs, j = idx % nrhs;
+            B[idx] = csub(B[idx], cmul(A[r * n + i], B[i * nrhs + j]));
         }
-        x.sync();
+        __syncthreads();
     }
 }
 
+// The same for n <= 32 by one warp, a row per lane: no rows are exchanged (a lane remembers the column
+// its row is the pivot of), the pivot comes from one 32-bit maximum over the leading words of the
+// candidates' larger component, and every lane has the reciprocal of its candidate ready by then.
+// Bound: the chain of n columns, about 500 cycles each, and 200 per row of the back substitution.
+__device__ inline void warp_solve(double2 *A, double2 *B, int n, int nrhs, int *status) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    double2 *Ar = A + lane * n, *Br = B + lane * nrhs, rp = cmk(1.0, 0.0);
+    int ord = lane < n ? -1 : n;  // the column this row is the pivot of
+    for (int c = 0; c < n; c++) {
+        const bool cand = ord < 0;
+        const double2 v = cand ? Ar[c] : cmk(0, 0);
+        const double m = cabs2(v), im = 1.0 / m;
+        const unsigned key = cand ? 1u + (unsigned)__double2hiint(fmax(fabs(v.x), fabs(v.y))) : 0u;
+        const unsigned best = __reduce_max_sync(all, key);
+        const int p = __ffs(__ballot_sync(all, key == best)) - 1;
+        double2 r = cmk(v.x * im, -v.y * im);
+        if (lane == p) {
+            if (!(m > 1e-290 && m < 1e290)) {  // the square left the range of a double
+                if (v.x == 0.0 && v.y == 0.0) *status = 1;
+                r = v.x == 0.0 && v.y == 0.0 ? cmk(1.0, 0.0) : cdiv(cmk(1.0, 0.0), v);
+            }
+            ord = c;
+            rp = r;
+        }
+        r = cmk(__shfl_sync(all, r.x, p), __shfl_sync(all, r.y, p));
+        if (ord < 0) {
+            const double2 f = cmul(v, r);
+            const double2 *Ap = A + p * n, *Bp = B + p * nrhs;
+            for (int j = c + 1; j < n; j++) Ar[j] = csub(Ar[j], cmul(f, Ap[j]));
+            for (int j = 0; j < nrhs; j++) Br[j] = csub(Br[j], cmul(f, Bp[j]));
+        }
+        __syncwarp();
+    }
+    for (int i = n - 1; i >= 0; i--) {
+        const int p = __ffs(__ballot_sync(all, ord == i)) - 1;
+        if (lane == p)
+            for (int j = 0; j < nrhs; j++) Br[j] = cmul(Br[j], rp);
+        __syncwarp();
+        if (ord < i) {
+            const double2 f = Ar[i], *Bp = B + p * nrhs;
+            for (int j = 0; j < nrhs; j++) Br[j] = csub(Br[j], cmul(f, Bp[j]));
+        }
+        __syncwarp();
+    }
+    for (int j = 0; j < nrhs; j++) {  // rows back into the order of the unknowns
+        const double2 x = lane < n ? Br[j] : cmk(0, 0);
+        __syncwarp();
+        if (lane < n) B[ord * nrhs + j] = x;
+        __syncwarp();
+    }
+}
+
+// Small systems by the CTA's first warp, the others by the whole CTA.  Start rows of a step in us, warp / CTA:
+// size1 1 (5 unknowns, one problem) 9 / 13, size1 2 (10 unknowns, 32 problems) 16 / 22, size1 4 (20 unknowns
+// and 4 right-hand sides, 32 problems) 32 / 38.  Above, a row per lane leaves too much to one warp.
 __device__ inline void cta_solve(double2 *A, double2 *B, int n, int nrhs, int *s_piv, int *status) {
-    grp_solve(CtaExec{}, A, B, n, nrhs, s_piv, status);
+    if (n <= 32 && n * (n + nrhs) <= 700) {
+        if (threadIdx.x < 32) warp_solve(A, B, n, nrhs, status);
+        __syncthreads();
+    } else {
+        grp_solve(A, B, n, nrhs, s_piv, status);
+    }
 }
 
 // Invert an s x s complex matrix held by one thread (Gauss-Jordan, partial pivoting).

@@ -6,7 +6,8 @@
 //   k_prep           s x s inverses of the step matrices (dyson_impl :179-213, :693-706, :983-1011),
 //                    history coefficients for tv, dense copies of Sigma^< and Sigma^tv
 //   ret recursion    G^R(n, 0..n): k-block start + Volterra recursion in t'   (:80-222)
-//   k_tv             G^tv(n, 0..ntau): history stream + Matsubara integral + solve (:651-741)
+//   k_tv_ring        G^tv(n, 0..ntau): (k_tv_mixed with the FP32 copy of the history)
+//                    history stream + Matsubara integral + solve (:651-741)
 //   k_les_operands_t right-hand operands of the Sigma-shared products
 //   k_zgemm products     tv*vt + les*adv convolutions for all problems at once (conv_impl :1075-1394)
 //   les recursion    G^<(0..n, n): k-block start + Volterra recursion in t (:893-1056)
@@ -160,234 +161,132 @@ __global__ void __launch_bounds__(256) k_prep(const GroupDev *__restrict__ gt, G
 // Start blocks: the k x k block systems of dyson_timestep_ret (:112-157) and
 // dyson_timestep_les (:926-982), solved by the whole CTA in shared memory.
 // ---------------------------------------------------------------------------------------
-// ret: unknowns X_q = G(n, n-q-1); equations sum_q X_q mm(p,q) = qq(p)  (left solve)
-template <int S, class X = CtaExec>
-__device__ void ret_start_block(const GroupDev &g, const ProbDev &p, int n, double2 *smem, const X &x = X()) {
-    const int k = g.k, s2 = S * S, KS = k * S;
-    const double h = g.h;
-    double2 *mm = smem;                 // k*k blocks (block (p,q) at (p*k+q)*s2)
-    double2 *qq = mm + k * k * s2;      // k blocks
-    double2 *A = qq + k * s2;           // (KS x KS)
-    double2 *R = A + KS * KS;           // (KS x S)
-    int *ipiv = (int *)(R + KS * S);
-    int *status = ipiv + 1;
-    double2 *grow = p.gret + tri(n) * s2;  // G(n, .)
-    for (int e = x.t(); e < k * k * s2; e += x.n()) mm[e] = cmk(0, 0);
-    for (int e = x.t(); e < k * s2; e += x.n()) qq[e] = cmk(0, 0);
-    if (x.t() == 0) *status = 0;
-    x.sync();
-    // thread per (row-block pr, element ab): fills block row pr of mm and qq(pr)
-    for (int e = x.t(); e < k * s2; e += x.n()) {
-        int pr = e / s2, ab = e % s2, a = ab / S, b = ab % S;
-        int j = pr + 1;
-        double2 q = cmk(0, 0);
-        // derivative: l == 0 -> qq -= (i/h) P(j,0) G(n,n); G(n,n) = -i 1
-        {
-            double2 cw = cmk(0.0, poly_diff(k, j, 0) / h);
-            double2 gnn = a == b ? cmk(0.0, -1.0) : cmk(0, 0);
-            q = csub(q, cmul(cw, gnn));
-        }
-        for (int l = 1; l <= k; l++) {
-            if (a == b) mm[(pr * k + l - 1) * s2 + ab] = cadd(mm[(pr * k + l - 1) * s2 + ab], cmk(0.0, poly_diff(k, j, l) / h));
-        }
-        // H: mm(pr,pr) += mu - H(n-j)
-        {
-            double2 hv = p.H[(long)(n - j + 1) * s2 + ab];
-            double2 v = cneg(hv);
-            if (a == b) v = cadd(v, cmk(p.mu, 0.0));
-            mm[(pr * k + pr) * s2 + ab] = cadd(mm[(pr * k + pr) * s2 + ab], v);
-        }
-        // integral: l = 0..k, w = h w(j,l), stemp = Sigma(n-l, n-j) or -Sigma(n-j,n-l)^dagger
-        for (int l = 0; l <= k; l++) {
-            double w = h * greg_w(k, j, l);
-            double2 st;
-            if (l <= j) st = g.sret[(tri(n - l) + (n - j)) * s2 + ab];
-            else { st = cconj(g.sret[(tri(n - j) + (n - l)) * s2 + b * S + a]); w = -w; }
-            if (l == 0) {
-                // qq += w * G(n,n) * stemp, G(n,n) = -i 1  ->  -i w stemp
-                q = cadd(q, cmul(cmk(0.0, -w), st));
-            } else {
-                int idx = (pr * k + l - 1) * s2 + ab;
-                mm[idx] = csub(mm[idx], cscale(st, w));
-            }
-        }
-        qq[pr * s2 + ab] = q;
-    }
-    x.sync();
-    // conjugate-transpose to a right solve: A[(pr,a),(q,b)] = conj(mm(pr,q)[b][a]),
-    // R[(pr,a),c] = conj(qq(pr)[c][a])
-    for (int e = x.t(); e < KS * KS; e += x.n()) {
-        int r = e / KS, c = e % KS, pr = r / S, a = r % S, q = c / S, b = c % S;
-        A[e] = cconj(mm[(pr * k + q) * s2 + b * S + a]);
-    }
-    for (int e = x.t(); e < KS * S; e += x.n()) {
-        int r = e / S, c = e % S, pr = r / S, a = r % S;
-        R[e] = cconj(qq[pr * s2 + c * S + a]);
-    }
-    x.sync();
-    grp_solve(x, A, R, KS, S, ipiv, status);
-    // X_q[a][c] = conj(Y[(q,c), a]) -> G(n, n-q-1)
-    for (int e = x.t(); e < k * s2; e += x.n()) {
-        int q = e / s2, ac = e % s2, a = ac / S, c = ac % S;
-        grow[(long)(n - q - 1) * s2 + ac] = cconj(R[(q * S + c) * S + a]);
-    }
-    x.sync();
-}
-
-// VIE2 ret (vie2_timestep_ret, cntr_vie2_impl.hpp:60-140, called with F and Fcc swapped):
-// unknowns X_q = G(n, n-q-1), q = 0..k-1, with G(n,n) = Q(n,n) set;
-//   sum_q X_q mm(p,q) = qq(p),  mm(p,q) = 1 delta_pq + h w(j,l) F'(n-l, n-j) [l = q+1]
-//   qq(p) = Q(n, n-j) - h w(j,0) G(n,n) F'(n, n-j),  j = p+1,
-// F'(t,t') = Fcc^R(t,t') for t >= t' and F^R(t',t)^dagger otherwise (sign folded into w).
-template <int S, class X = CtaExec>
-__device__ void ret_start_block_vie(const GroupDev &g, const ProbDev &p, int n, double2 *smem, const X &x = X()) {
-    const int k = g.k, s2 = S * S, KS = k * S;
-    const double h = g.h;
-    double2 *mm = smem;
-    double2 *qq = mm + k * k * s2;
-    double2 *A = qq + k * s2;
-    double2 *R = A + KS * KS;
-    int *ipiv = (int *)(R + KS * S);
-    int *status = ipiv + 1;
-    double2 *grow = p.gret + tri(n) * s2;
-    for (int e = x.t(); e < k * k * s2; e += x.n()) mm[e] = cmk(0, 0);
-    if (x.t() == 0) *status = 0;
-    x.sync();
-    for (int e = x.t(); e < k * s2; e += x.n()) {
-        const int pr = e / s2, ab = e % s2, a = ab / S, b = ab % S, j = pr + 1;
-        double2 q = p.qret[(tri(n) + n - j) * s2 + ab];
-        if (a == b) mm[(pr * k + pr) * s2 + ab] = cadd(mm[(pr * k + pr) * s2 + ab], cmk(1.0, 0.0));
-        for (int l = 0; l <= k; l++) {
-            double w = -h * greg_w(k, j, l);
-            if (l == 0) {
-                // qq += w G(n,n) F'(n, n-j)
-                const double2 *fr = g.rret + (tri(n) + n - j) * s2;
-                double2 t = cmk(0, 0);
-                for (int c = 0; c < S; c++) t = cfma(grow[(long)n * s2 + a * S + c], fr[c * S + b], t);
-                q = cfma(cmk(w, 0.0), t, q);
-            } else {
-                double2 st;
-                if (l <= j) st = g.rret[(tri(n - l) + n - j) * s2 + ab];
-                else { st = cconj(g.sret[(tri(n - j) + n - l) * s2 + b * S + a]); w = -w; }
-                const int idx = (pr * k + l - 1) * s2 + ab;
-                mm[idx] = csub(mm[idx], cscale(st, w));
-            }
-        }
-        qq[pr * s2 + ab] = q;
-    }
-    x.sync();
-    for (int e = x.t(); e < KS * KS; e += x.n()) {
-        int r = e / KS, c = e % KS, pr = r / S, a = r % S, q = c / S, b = c % S;
-        A[e] = cconj(mm[(pr * k + q) * s2 + b * S + a]);
-    }
-    for (int e = x.t(); e < KS * S; e += x.n()) {
-        int r = e / S, c = e % S, pr = r / S, a = r % S;
-        R[e] = cconj(qq[pr * s2 + c * S + a]);
-    }
-    x.sync();
-    grp_solve(x, A, R, KS, S, ipiv, status);
-    for (int e = x.t(); e < k * s2; e += x.n()) {
-        int q = e / s2, ac = e % s2, a = ac / S, c = ac % S;
-        grow[(long)(n - q - 1) * s2 + ac] = cconj(R[(q * S + c) * S + a]);
-    }
-    x.sync();
-}
-
-// VIE2 les (vie2_timestep_les, cntr_vie2_impl.hpp:847-990): unknowns x_j = G^<(j,n), j = 0..k;
-//   sum_m mm(j,m) x_m = gl(j) + Q^<(j,n),  mm(j,m) = 1 delta_jm + h w(j,m) F'(j,m),
-// F'(j,m) = F^R(j,m) for j >= m and -Fcc^R(m,j)^dagger otherwise (right solve).
-template <int S, class X = CtaExec>
-__device__ void les_start_block_vie(const GroupDev &g, const ProbDev &p, int n, const double2 *gl, long ldc,
-                                    double2 *xcol, double2 *smem, const X &x = X()) {
-    const int k = g.k, K1 = k + 1, s2 = S * S, KS = K1 * S;
-    const double h = g.h;
-    double2 *A = smem;
-    double2 *R = A + KS * KS;
-    int *ipiv = (int *)(R + KS * S);
-    int *status = ipiv + 1;
-    if (x.t() == 0) *status = 0;
-    for (int e = x.t(); e < K1 * s2; e += x.n()) {
-        const int j = e / s2, ad = e % s2, a = ad / S, d = ad % S;
-        double2 q = gl[((long)j * S + a) * ldc + d];
-        q = cadd(q, j <= n ? p.qles[(tri(n) + j) * s2 + ad] : cneg(cconj(p.qles[(tri(j) + n) * s2 + d * S + a])));
-        R[(j * S + a) * S + d] = q;
-        if (d == 0) {
-            for (int m = 0; m <= k; m++) {
-                const double w = h * greg_w(k, j, m);
-                for (int b = 0; b < S; b++) {
-                    double2 st = j >= m ? g.sret[(tri(j) + m) * s2 + a * S + b]
-                                        : cneg(cconj(g.rret[(tri(m) + j) * s2 + b * S + a]));
-                    double2 v = cscale(st, w);
-                    if (m == j && a == b) v = cadd(v, cmk(1.0, 0.0));
-                    A[(j * S + a) * KS + m * S + b] = v;
-                }
-            }
-        }
-    }
-    x.sync();
-    grp_solve(x, A, R, KS, S, ipiv, status);
-    for (int e = x.t(); e < K1 * s2; e += x.n()) {
-        const int j = e / s2, ad = e % s2, a = ad / S, d = ad % S;
-        xcol[(long)j * s2 + ad] = R[(j * S + a) * S + d];
-    }
-    x.sync();
-}
-
-// les: unknowns x_j = G^<(j,n), j = 1..k; sum_q mm(p,q) x_{q+1} = qq(p)  (right solve)
-template <int S, class X = CtaExec>
-__device__ void les_start_block(const GroupDev &g, const ProbDev &p, int n, const double2 *gl, long ldc,
-                                double2 *xcol, double2 *smem, const X &x = X()) {
+// A thread per matrix element: its terms are loaded independently, so the assembly costs a few memory
+// latencies, not one per term.
+// ret: unknowns X_q = G(n, n-q-1); equations sum_q X_q mm(p,q) = qq(p)  (left solve), solved as the
+// right solve of the block-wise adjoints: A[(p,a),(q,b)] = conj(mm(p,q)[b][a]), R[(p,a),c] = conj(qq(p)[c][a]).
+// Dyson, j = p+1, l = q+1, stemp(l) = Sigma(n-l, n-j) (l <= j) or -Sigma(n-j, n-l)^dagger:
+//   mm(p,q) = (i/h) P(j,l) 1 + delta_lj (mu - H(n-j)) - h w(j,l) stemp(l)
+//   qq(p) = -(i/h) P(j,0) G(n,n) + h w(j,0) G(n,n) stemp(0),  G(n,n) = -i 1
+// VIE2 (vie2_timestep_ret, cntr_vie2_impl.hpp:60-140, called with F and Fcc swapped), G(n,n) = Q(n,n) set,
+// F'(t,t') = Fcc^R(t,t') for t >= t' and -F^R(t',t)^dagger otherwise:
+//   mm(p,q) = 1 delta_pq + h w(j,l) F'(n-l, n-j),  qq(p) = Q(n, n-j) - h w(j,0) G(n,n) F'(n, n-j)
+template <int S, bool VIE>
+__device__ void ret_start_block(const GroupDev &g, const ProbDev &p, int n, double2 *smem) {
     const int k = g.k, s2 = S * S, KS = k * S;
     const double h = g.h;
     double2 *A = smem;           // (KS x KS)
     double2 *R = A + KS * KS;    // (KS x S)
     int *ipiv = (int *)(R + KS * S);
     int *status = ipiv + 1;
-    if (x.t() == 0) *status = 0;
-    for (int e = x.t(); e < KS * KS; e += x.n()) A[e] = cmk(0, 0);
-    x.sync();
-    // thread per (pr, a, d): qq(pr)[a][d] and the row (pr,a) of A
-    for (int e = x.t(); e < k * s2; e += x.n()) {
-        int pr = e / s2, ad = e % s2, a = ad / S, d = ad % S;
-        int j = pr + 1;
-        double2 q = gl[((long)j * S + a) * ldc + d];  // gles(j)
-        double2 cw0 = cmk(0.0, poly_diff(k, j, 0) / h);
-        q = csub(q, cmul(cw0, xcol[ad]));  // x_0 = xcol[0..s2)
-        // h w(j,0) Sigma^R(j,0) x_0
-        {
-            double w = h * greg_w(k, j, 0);
-            double2 acc = cmk(0, 0);
-            for (int b = 0; b < S; b++) acc = cfma(g.sret[(tri(j) + 0) * s2 + a * S + b], xcol[b * S + d], acc);
-            q = cadd(q, cscale(acc, w));
+    double2 *grow = p.gret + tri(n) * s2;  // G(n, .)
+    if (threadIdx.x == 0) *status = 0;
+    for (int e = threadIdx.x; e < KS * (KS + S); e += blockDim.x) {
+        const int r = e / (KS + S), c = e % (KS + S), j = r / S + 1, b = r % S;
+        if (c < KS) {  // element mm(j-1, l-1)[a][b]
+            const int l = c / S + 1, a = c % S;
+            double w = h * greg_w(k, j, l);
+            double2 st;
+            if (l <= j) {
+                st = g.rret[(tri(n - l) + n - j) * s2 + a * S + b];
+            } else {
+                st = cconj(g.sret[(tri(n - j) + n - l) * s2 + b * S + a]);
+                w = -w;
+            }
+            double2 v = cmk(0, 0);
+            if (VIE) {
+                if (l == j && a == b) v = cmk(1.0, 0.0);
+                v = cadd(v, cscale(st, w));
+            } else {
+                if (a == b) v = cmk(0.0, poly_diff(k, j, l) / h);
+                if (l == j) {
+                    double2 u = cneg(p.H[(long)(n - j + 1) * s2 + a * S + b]);
+                    if (a == b) u = cadd(u, cmk(p.mu, 0.0));
+                    v = cadd(v, u);
+                }
+                v = csub(v, cscale(st, w));
+            }
+            A[r * KS + c] = cconj(v);
+        } else {  // element qq(j-1)[a][b]
+            const int a = c - KS;
+            const double w = h * greg_w(k, j, 0);
+            const double2 *fr = g.rret + (tri(n) + n - j) * s2;
+            double2 q;
+            if (VIE) {
+                double2 t = cmk(0, 0);
+                for (int x = 0; x < S; x++) t = cfma(grow[(long)n * s2 + a * S + x], fr[x * S + b], t);
+                q = cfma(cmk(-w, 0.0), t, p.qret[(tri(n) + n - j) * s2 + a * S + b]);
+            } else {
+                q = a == b ? cneg(cmul(cmk(0.0, poly_diff(k, j, 0) / h), cmk(0.0, -1.0))) : cmk(0, 0);
+                q = cadd(q, cmul(cmk(0.0, -w), fr[a * S + b]));
+            }
+            R[r * S + a] = cconj(q);
         }
-        R[(pr * S + a) * S + d] = q;
-        if (d == 0) {
-            for (int m = 1; m <= k; m++) {
-                double2 cwm = cmk(0.0, poly_diff(k, j, m) / h);
-                double w = h * greg_w(k, j, m);
-                for (int b = 0; b < S; b++) {
-                    double2 st;
-                    if (j >= m) st = g.sret[(tri(j) + m) * s2 + a * S + b];
-                    else st = cneg(cconj(g.sret[(tri(m) + j) * s2 + b * S + a]));
-                    double2 v = cscale(st, -w);
-                    if (a == b) v = cadd(v, cwm);
-                    if (m == j) {
-                        double2 hv = p.H[(long)(j + 1) * s2 + a * S + b];
-                        v = csub(v, hv);
-                        if (a == b) v = cadd(v, cmk(p.mu, 0.0));
-                    }
-                    A[(pr * S + a) * KS + (m - 1) * S + b] = v;
+    }
+    __syncthreads();
+    cta_solve(A, R, KS, S, ipiv, status);
+    // X_q[a][c] = conj(Y[(q,c), a]) -> G(n, n-q-1)
+    for (int e = threadIdx.x; e < k * s2; e += blockDim.x) {
+        const int q = e / s2, ac = e % s2, a = ac / S, c = ac % S;
+        grow[(long)(n - q - 1) * s2 + ac] = cconj(R[(q * S + c) * S + a]);
+    }
+    __syncthreads();
+}
+
+// les (right solve).  Dyson: unknowns x_j = G^<(j,n), j = 1..k, x_0 = xcol[0] known:
+//   sum_m mm(j,m) x_m = gl(j) - (i/h) P(j,0) x_0 + h w(j,0) Sigma^R(j,0) x_0
+//   mm(j,m) = (i/h) P(j,m) 1 + delta_jm (mu - H(j)) - h w(j,m) st(j,m)
+// VIE2 (vie2_timestep_les, cntr_vie2_impl.hpp:847-990): unknowns j = 0..k:
+//   sum_m mm(j,m) x_m = gl(j) + Q^<(j,n),  mm(j,m) = 1 delta_jm + h w(j,m) st(j,m)
+// st(j,m) = Sigma^R(j,m) (F^R) for j >= m and -Sigma^R(m,j)^dagger (-Fcc^R) otherwise.
+template <int S, bool VIE>
+__device__ void les_start_block(const GroupDev &g, const ProbDev &p, int n, const double2 *gl, long ldc, double2 *xcol,
+                                double2 *smem) {
+    constexpr int j0 = VIE ? 0 : 1;
+    const int k = g.k, s2 = S * S, KS = (k + 1 - j0) * S;
+    const double h = g.h;
+    double2 *A = smem;           // (KS x KS)
+    double2 *R = A + KS * KS;    // (KS x S)
+    int *ipiv = (int *)(R + KS * S);
+    int *status = ipiv + 1;
+    if (threadIdx.x == 0) *status = 0;
+    for (int e = threadIdx.x; e < KS * (KS + S); e += blockDim.x) {
+        const int r = e / (KS + S), c = e % (KS + S), j = r / S + j0, a = r % S;
+        if (c < KS) {
+            const int m = c / S + j0, b = c % S;
+            const double w = h * greg_w(k, j, m);
+            const double2 st = j >= m ? g.sret[(tri(j) + m) * s2 + a * S + b]
+                                      : cneg(cconj(g.rret[(tri(m) + j) * s2 + b * S + a]));
+            double2 v = cscale(st, VIE ? w : -w);
+            if (VIE) {
+                if (m == j && a == b) v = cadd(v, cmk(1.0, 0.0));
+            } else {
+                if (a == b) v = cadd(v, cmk(0.0, poly_diff(k, j, m) / h));
+                if (m == j) {
+                    v = csub(v, p.H[(long)(j + 1) * s2 + a * S + b]);
+                    if (a == b) v = cadd(v, cmk(p.mu, 0.0));
                 }
             }
+            A[r * KS + c] = v;
+        } else {
+            const int d = c - KS;
+            double2 q = gl[((long)j * S + a) * ldc + d];
+            if (VIE) {
+                q = cadd(q, j <= n ? p.qles[(tri(n) + j) * s2 + a * S + d] : cneg(cconj(p.qles[(tri(j) + n) * s2 + d * S + a])));
+            } else {
+                const double w = h * greg_w(k, j, 0);
+                double2 t = cmk(0, 0);
+                for (int b = 0; b < S; b++) t = cfma(g.sret[tri(j) * s2 + a * S + b], xcol[b * S + d], t);
+                q = csub(q, cmul(cmk(0.0, poly_diff(k, j, 0) / h), xcol[a * S + d]));
+                q = cadd(q, cscale(t, w));
+            }
+            R[r * S + d] = q;
         }
     }
-    x.sync();
-    grp_solve(x, A, R, KS, S, ipiv, status);
-    for (int e = x.t(); e < k * s2; e += x.n()) {
-        int q = e / s2, ad = e % s2, a = ad / S, d = ad % S;
-        xcol[(long)(q + 1) * s2 + ad] = R[(q * S + a) * S + d];
-    }
-    x.sync();
+    __syncthreads();
+    cta_solve(A, R, KS, S, ipiv, status);
+    for (int e = threadIdx.x; e < KS * S; e += blockDim.x) xcol[j0 * s2 + e] = R[e];
+    __syncthreads();
 }
 
 // ---------------------------------------------------------------------------------------

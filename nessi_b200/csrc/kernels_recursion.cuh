@@ -470,9 +470,7 @@ __global__ void __launch_bounds__(256) k_ret_start(const GroupDev *__restrict__ 
     for (int e = threadIdx.x; e < s2; e += blockDim.x)
         grow[(long)n * s2 + e] = VIE ? p.qret[(tri(n) + n) * s2 + e] : (e / S == e % S ? cmk(0.0, -1.0) : cmk(0, 0));
     __syncthreads();
-    if (VIE) ret_start_block_vie<S>(g, p, n, smem);
-    else ret_start_block<S>(g, p, n, smem);
-    __syncthreads();
+    ret_start_block<S, VIE>(g, p, n, smem);
     for (int e = threadIdx.x; e < (k + 1) * s2; e += blockDim.x) {
         const int l = e / s2, b = (e % s2) / S, d = e % S;  // Y_l[b][d] = G(n, n-l)[d][b]
         const double2 y = grow[(long)(n - l) * s2 + d * S + b];
@@ -497,17 +495,14 @@ __global__ void __launch_bounds__(256) k_les_start(const GroupDev *__restrict__ 
     const long ldc = g.ldc;
     const double2 *gl = g.gles + (long)p.col * S;
     double2 *xcol = p.gles + tri(n) * s2;
-    if (VIE) {
-        les_start_block_vie<S>(g, p, n, gl, ldc, xcol, smem);
-    } else {
+    if (!VIE) {
         for (int ad = threadIdx.x; ad < s2; ad += blockDim.x) {
             const int a = ad / S, d = ad % S;
             xcol[ad] = cneg(cconj(p.gtv[((long)n * s2 + d * S + a) * (g.ntau + 1) + 0]));
         }
         __syncthreads();
-        les_start_block<S>(g, p, n, gl, ldc, xcol, smem);
     }
-    __syncthreads();
+    les_start_block<S, VIE>(g, p, n, gl, ldc, xcol, smem);
     for (int e = threadIdx.x; e < (k + 1) * s2; e += blockDim.x) {
         const int l = e / s2, b = (e % s2) / S, d = e % S;
         g.vy[((long)l * S + b) * ldc + p.col * S + d] = cscale(xcol[e], greg_omega(k, l));

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256) k_dyson_start(GroupDev g, const ProbDev *
             xw[ad] = cneg(cconj(GTV(n, d * S + a, 0)));
         }
         __syncthreads();
-        les_start_block<S>(g, p, n, gl, S, xw, scr + (k + 1) * s2);
+        les_start_block<S, false>(g, p, n, gl, S, xw, scr + (k + 1) * s2);
         for (int e = tid; e < (n + 1) * s2; e += nth) xcol[e] = xw[e];
         __syncthreads();
     }
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) k_vie2_start(GroupDev g, const ProbDev *_
             gl[e] = cneg(v);
         }
         __syncthreads();
-        les_start_block_vie<S>(g, p, n, gl, S, xw, scr);
+        les_start_block<S, true>(g, p, n, gl, S, xw, scr);
         double2 *xcol = p.gles + tri(n) * s2;  // G^<(0..n, n)
         for (int e = tid; e < (n + 1) * s2; e += nth) xcol[e] = xw[e];
         __syncthreads();
