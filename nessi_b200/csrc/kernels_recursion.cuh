@@ -26,21 +26,24 @@
 //
 // k_vol_block, one launch per block: the CTA stages the block's triangle a_{i-l} T(i, l) (128
 // scalar rows, 130 KB) and the step inverses in shared memory with asynchronous copies; then a warp
-// (s >= 3: four warps, a slot of 32 rows each) solves one or two columns (p, d), 128 rows
+// (s >= 3: four warps, a slot of 32 rows each) solves a column (s = 2: two) (p, d), 128 rows
 // right-looking from registers: a lane holds scalar rows lane + 32 t of a column, and after a time
 // row is solved every lane folds it into its own rows.
 // Bound: the chain of 128 / s dependent rows; per row the solve with D_l, the broadcast and the update
 // of the next row (a dependent FP64 FMA takes 9 cycles, a shared-memory round trip 33), with the
-// triangle's column of the next row loaded one row ahead.  Two columns per warp share those loads.
+// triangle's column of the next row loaded one row ahead.  Columns per warp: one for size1 1 (blocks of
+// ret and les, 1024 problems, n 1000: 340 us; two that share the loads 475, their sums are longer than
+// the chain).  Size1 2: two at eight columns per CTA, else one (256 problems, n 1000: 687 us, 512
+// problems 1048; built for one only: 775 and 1004).
 // 128 scalar rows: the widest triangle that fits in shared memory beside the tv stream's ring, so
 // that a step of n rows is n s / 128 launch pairs.  The kernels of a recursion are launched with
 // programmatic stream serialization: what does not depend on the solution (triangle, near block,
 // step inverses) is staged while the previous kernel still runs.
 //
 // Measured on a B200, alone, ret + les of a step in us (blocks / trailing products / start rows):
-// size1 1, 1024 problems, n 1000: 853 (477 / 391 / 46); size1 2, 256 problems, n 1000: 1419 (688 /
-// 781 / 47); size1 4, 32 problems, n 1200: 2607 (1244 / 1456 / 81); size1 8, 18 problems, n 600: 3177
-// (1275 / 1626 / 226); size1 1, one problem, n 400: 141.  Synchronous staging, without the overlap of
+// size1 1, 1024 problems, n 1000: 699 (340 / 389 / 33); size1 2, 256 problems, n 1000: 1402 (687 /
+// 785 / 32); size1 4, 32 problems, n 1200: 2593 (1247 / 1450 / 64); size1 8, 18 problems, n 600: 3125
+// (1275 / 1617 / 173); size1 1, one problem, n 400: 119.  Synchronous staging, without the overlap of
 // launches, one warp per column for s >= 3: 957, 1842, 3774, 4175 and 238.
 #pragma once
 #include "kernels_dyson.cuh"
@@ -53,8 +56,8 @@ template <int S> struct VbCfg {
     static constexpr int NRP = NR | 1;               // odd stride of a column buffer
     static constexpr int TRI = S * S * (NBT * (NBT - 1) / 2);
     static constexpr int NEAR = NESSI_K1MAX * S;     // rows next to the block above, and their sources
-    // s <= 2: a warp solves one or two columns, all four slots; s >= 3: four warps per column, a slot each
-    static constexpr int NTH = S <= 4 ? 256 : 512, NW = NTH / 32, WMAX = S <= 2 ? 8 : NTH / 128, NC = S <= 2 ? 2 : 1;
+    // s <= 2: a warp solves NC columns, all four slots; s >= 3: four warps per column, a slot each
+    static constexpr int NTH = S <= 4 ? 256 : 512, NW = NTH / 32, WMAX = S <= 2 ? 8 : NTH / 128, NC = S == 2 ? 2 : 1;
     // shared memory in double2: 32 of padding (unpredicated loads of solved rows), triangle, near
     // block, then per column the near values, the column and (s >= 3) the row being solved, then the
     // step inverses of the problems touched
@@ -80,13 +83,13 @@ __device__ __forceinline__ double2 sub_ib(double2 acc, double b, double2 x) {
     return cmk(fma(b, x.y, acc.x), fma(-b, x.x, acc.y));
 }
 
-// s <= 2: NC columns of a block, solved by a warp.  acc[c][t] = right-hand side of scalar row
+// s <= 2: a column (s = 2: NC columns) of a block, solved by a warp.  acc[c][t] = right-hand side of scalar row
 // lane + 32 t of column c on entry; xs (shared, stride NRP) receives the solved rows.  D: step
 // inverses (s = 1: registers, rows lane + 32 t; s = 2: shared).  bdp[32 + delta] = bd / h for
 // 1 <= delta <= k+1, else 0.  The accumulators of solved rows are not used again.
-template <bool VIE, int NC>
-__device__ __forceinline__ void vol_chain1(double2 (*acc)[4], const double2 *coef, double2 (*D)[4], const double *bdp,
-                                           double gh, int K1, int nb, double2 *xs, int lane) {
+template <bool VIE>
+__device__ __forceinline__ void vol_chain1(double2 *acc, const double2 *coef, const double2 *D, const double *bdp, double gh,
+                                           int K1, int nb, double2 *xs, int lane) {
     using C = VbCfg<1>;
     const double2 *cl = coef - 1 + lane;  // column l: row lane + 32 t at cl[32 t]
     double2 cv[4];
@@ -103,18 +106,15 @@ __device__ __forceinline__ void vol_chain1(double2 (*acc)[4], const double2 *coe
             cl += C::NR - 2 - (32 * ph + ll);
 #pragma unroll
             for (int t = ph; t < 4; t++) nv[t] = 32 * t + lane > 32 * ph + ll + 1 ? cl[32 * t] : cmk(0, 0);
+            const double2 x = shfl2(cmul(D[ph], acc[ph]), ll), xg = cscale(x, gh);
+            if (lane == ll) xs[32 * ph + ll] = x;
+            double2 u = acc[ph];
+            if (!VIE) u = sub_ib(u, b0, x);
+            acc[ph] = cfma(cv[ph], xg, u);
 #pragma unroll
-            for (int c = 0; c < NC; c++) {
-                const double2 x = shfl2(cmul(D[c][ph], acc[c][ph]), ll), xg = cscale(x, gh);
-                if (lane == ll) xs[c * C::NRP + 32 * ph + ll] = x;
-                double2 u = acc[c][ph];
-                if (!VIE) u = sub_ib(u, b0, x);
-                acc[c][ph] = cfma(cv[ph], xg, u);
-#pragma unroll
-                for (int t = ph + 1; t < 4; t++) {
-                    if (!VIE && t == ph + 1 && ll + K1 >= 32) acc[c][t] = sub_ib(acc[c][t], b1, x);
-                    acc[c][t] = cfma(cv[t], xg, acc[c][t]);
-                }
+            for (int t = ph + 1; t < 4; t++) {
+                if (!VIE && t == ph + 1 && ll + K1 >= 32) acc[t] = sub_ib(acc[t], b1, x);
+                acc[t] = cfma(cv[t], xg, acc[t]);
             }
 #pragma unroll
             for (int t = ph; t < 4; t++) cv[t] = nv[t];
@@ -359,8 +359,7 @@ __global__ void __launch_bounds__(VbCfg<S>::NTH, VbCfg<S>::NTH == 256 ? 2 : 1) k
                     acc[cc][t] = cc < nc && warp * nc + cc < ncol && lane + 32 * t < NRb ? rhs(warp * nc + cc, lane + 32 * t) : cmk(0, 0);
             __syncwarp();
             if constexpr (S == 1) {
-                if (nc == 2) vol_chain1<VIE, 2>(acc, coef, Dr, bdp, gh, K1, nb, xs, lane);
-                else vol_chain1<VIE, 1>(acc, coef, Dr, bdp, gh, K1, nb, xs, lane);
+                vol_chain1<VIE>(acc[0], coef, Dr[0], bdp, gh, K1, nb, xs, lane);
             } else {  // two columns of a warp are one problem's
                 const double2 *D = dm + ((c0 + warp * nc) / S - p0) * NR * S;
                 if (nc == 2) vol_chain2<VIE, 2>(acc, coef, D, bdp, gh, K1, nb, xs, lane);
