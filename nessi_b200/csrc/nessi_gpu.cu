@@ -152,6 +152,13 @@ struct KProf {
     double bytes = 0;  // algorithmic bytes of the recorded launches
 };
 
+// A pair of streams on which a size1 class of groups steps (main and side, see step_class), forked from
+// and joined to the batch stream.
+struct StepLane {
+    cudaStream_t st = nullptr, side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
+};
+
 struct nessi_batch {
     int device = 0;
     bool prof = false;
@@ -159,7 +166,8 @@ struct nessi_batch {
     int precision = NESSI_PREC_FP64;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;       // runs the retarded component concurrently with tv
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_lanes = nullptr;
+    std::vector<StepLane> lanes;       // for the second, third, ... size1 of the batch
     bool own_stream = true;
     cudaGraphExec_t graph = nullptr;                     // recorded time steps (nessi_gpu_graph_record)
     std::vector<Prob> probs;
@@ -176,7 +184,7 @@ struct nessi_batch {
     size_t stage_bytes = 0;              // of one slot
     cudaEvent_t stage_ev[NSTAGE] = {};   // the slot's last reader
     int stage_next = 0;
-    // kernel of the tv row: 1 (default) = k_tv (register loads, every size1), 0 = k_tv_stream
+    // kernel of the tv row: 1 (default) = k_tv_ring / k_tv_mixed (every size1), 0 = k_tv_stream
     // (history through shared memory by bulk copies, size1 <= 4; NESSI_TV_KERNEL=stream)
     int tv_kernel = 1;
     int nsm = 0;                        // SMs of the device
@@ -345,9 +353,7 @@ template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n,
 // Volterra kernels reported by nessi_gpu_get_volterra_choice: the blocked recursion
 #define NESSI_VOLTERRA_BLOCKED 102
 
-template <int S> size_t ret_start_smem(int k) {
-    return (size_t)(k * k * S * S + k * S * S + (k * S) * (k * S) + k * S * S) * 16 + 16;
-}
+template <int S> size_t ret_start_smem(int k) { return (size_t)(k * S * k * S + k * S * S) * 16 + 16; }
 template <int S> size_t les_start_smem(int k) {
     const int K1 = k + 1;  // the VIE2 start block has k+1 unknowns
     return (size_t)((K1 * S) * (K1 * S) + K1 * S * S) * 16 + 16;
@@ -452,8 +458,8 @@ int tv_stream_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, 
 
 // Time step n of the selected groups, all of size1 = S and one kind: every kernel is one launch for
 // all of them.
-template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, int n) {
-    cudaStream_t st = b->stream;
+template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, int n, const StepLane &ln) {
+    cudaStream_t st = ln.st;
     const GroupDev *gt = b->d_groups;
     const unsigned ng = (unsigned)sel.ng;
     PrepSel ps;
@@ -494,31 +500,31 @@ template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, i
         }
     }
     // step matrices, tv coefficients, dense Sigma
-    b->prof_mark(NESSI_KERNEL_PREP);
+    b->prof_mark(NESSI_KERNEL_PREP, st);
     const unsigned ngb = (unsigned)std::min<long>((prep + 255) / 256, 1184);
     CKR(launch_chained(k_prep<S, VIE>, dim3((unsigned)maxact + ngb, ng), 256, 0, st, gt, sel, ps, n, maxact));
-    b->prof_end(NESSI_KERNEL_PREP, 0.0);
+    b->prof_end(NESSI_KERNEL_PREP, 0.0, st);
     // Matsubara part of the tv row: Cmat = K_n Gmat_all (one GEMM per group)
-    b->prof_mark(NESSI_KERNEL_MATOP);
+    b->prof_mark(NESSI_KERNEL_MATOP, st);
     CKR(launch_chained(k_mat_operator<S>, dim3((unsigned)std::min<long>(((long)M * M * S * S + 255) / 256, 4736), ng), 256, 0,
                        st, gt, sel, n));
-    b->prof_end(NESSI_KERNEL_MATOP, by_mat);
-    b->prof_mark(NESSI_KERNEL_GEMM);
+    b->prof_end(NESSI_KERNEL_MATOP, by_mat, st);
+    b->prof_mark(NESSI_KERNEL_GEMM, st);
     CKR(product_launch<PROD_MAT>(b, sel, n, true, st));
-    b->prof_end(NESSI_KERNEL_GEMM, flop_mat);
+    b->prof_end(NESSI_KERNEL_GEMM, flop_mat, st);
     // side stream: retarded row, then les*adv = Ldense * badv (needs only G^R(n, .)); VIE2 moves the
     // convolution to the right-hand side: gles = -(tv*vt + les*adv)
-    CK(cudaEventRecord(b->ev_fork, st));
-    CK(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-    b->prof_mark(NESSI_KERNEL_RET, b->side);
-    CKR((volterra_class<S, VIE, true>(b, sel, n, b->side)));
-    b->prof_end(NESSI_KERNEL_RET, flop_rec, b->side);
-    b->prof_mark(NESSI_KERNEL_GEMM, b->side);
-    CKR(product_launch<PROD_LESADV>(b, sel, n, true, b->side));
-    b->prof_end(NESSI_KERNEL_GEMM, flop_les, b->side);
-    CK(cudaEventRecord(b->ev_join, b->side));
+    CK(cudaEventRecord(ln.fork, st));
+    CK(cudaStreamWaitEvent(ln.side, ln.fork, 0));
+    b->prof_mark(NESSI_KERNEL_RET, ln.side);
+    CKR((volterra_class<S, VIE, true>(b, sel, n, ln.side)));
+    b->prof_end(NESSI_KERNEL_RET, flop_rec, ln.side);
+    b->prof_mark(NESSI_KERNEL_GEMM, ln.side);
+    CKR(product_launch<PROD_LESADV>(b, sel, n, true, ln.side));
+    b->prof_end(NESSI_KERNEL_GEMM, flop_les, ln.side);
+    CK(cudaEventRecord(ln.join, ln.side));
     // main stream: tv row, then the tv*vt operand
-    b->prof_mark(NESSI_KERNEL_TV);
+    b->prof_mark(NESSI_KERNEL_TV, st);
     bool streamed = false;
     if constexpr (S <= 4) {
         if (b->tv_kernel == 0) {
@@ -545,20 +551,20 @@ template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, i
         }
         CK(cudaGetLastError());
     }
-    b->prof_end(NESSI_KERNEL_TV, by_tv);
-    b->prof_mark(NESSI_KERNEL_LES_OPERANDS);
+    b->prof_end(NESSI_KERNEL_TV, by_tv, st);
+    b->prof_mark(NESSI_KERNEL_LES_OPERANDS, st);
     CKR(launch_chained(k_les_operands_t<S>, dim3((unsigned)((M + LoCfg<S>::LOR - 1) / LoCfg<S>::LOR),
                                                  (unsigned)((maxact + LOT - 1) / LOT), ng), 256, 0, st, gt, sel, n));
-    b->prof_end(NESSI_KERNEL_LES_OPERANDS, by_vt);
-    CK(cudaStreamWaitEvent(st, b->ev_join, 0));
+    b->prof_end(NESSI_KERNEL_LES_OPERANDS, by_vt, st);
+    CK(cudaStreamWaitEvent(st, ln.join, 0));
     // tv*vt: gles += Sigma^tv * btv
-    b->prof_mark(NESSI_KERNEL_GEMM);
+    b->prof_mark(NESSI_KERNEL_GEMM, st);
     CKR(product_launch<PROD_TVVT>(b, sel, n, false, st));
-    b->prof_end(NESSI_KERNEL_GEMM, flop_vt);
+    b->prof_end(NESSI_KERNEL_GEMM, flop_vt, st);
     // lesser column
-    b->prof_mark(NESSI_KERNEL_LES);
+    b->prof_mark(NESSI_KERNEL_LES, st);
     CKR((volterra_class<S, VIE, false>(b, sel, n, st)));
-    b->prof_end(NESSI_KERNEL_LES, flop_rec);
+    b->prof_end(NESSI_KERNEL_LES, flop_rec, st);
     return NESSI_OK;
 }
 
@@ -693,20 +699,20 @@ int mat_dispatch(nessi_batch *b, Group &g, int method, int force_herm) {
 }
 int vie2_mat_dispatch(nessi_batch *b, Group &g, int method) { NESSI_SIZE_SWITCH(vie2_mat_group, b, g, method) }
 
-template <int S> int step_class_any(nessi_batch *b, bool vie, const GroupSel &sel, int n) {
-    return vie ? step_class<S, true>(b, sel, n) : step_class<S, false>(b, sel, n);
+template <int S> int step_class_any(nessi_batch *b, bool vie, const GroupSel &sel, int n, const StepLane &ln) {
+    return vie ? step_class<S, true>(b, sel, n, ln) : step_class<S, false>(b, sel, n, ln);
 }
 
-int step_dispatch(nessi_batch *b, int s, bool vie, const GroupSel &sel, int n) {
+int step_dispatch(nessi_batch *b, int s, bool vie, const GroupSel &sel, int n, const StepLane &ln) {
     switch (s) {
-        case 1: return step_class_any<1>(b, vie, sel, n);
-        case 2: return step_class_any<2>(b, vie, sel, n);
-        case 3: return step_class_any<3>(b, vie, sel, n);
-        case 4: return step_class_any<4>(b, vie, sel, n);
-        case 5: return step_class_any<5>(b, vie, sel, n);
-        case 6: return step_class_any<6>(b, vie, sel, n);
-        case 7: return step_class_any<7>(b, vie, sel, n);
-        case 8: return step_class_any<8>(b, vie, sel, n);
+        case 1: return step_class_any<1>(b, vie, sel, n, ln);
+        case 2: return step_class_any<2>(b, vie, sel, n, ln);
+        case 3: return step_class_any<3>(b, vie, sel, n, ln);
+        case 4: return step_class_any<4>(b, vie, sel, n, ln);
+        case 5: return step_class_any<5>(b, vie, sel, n, ln);
+        case 6: return step_class_any<6>(b, vie, sel, n, ln);
+        case 7: return step_class_any<7>(b, vie, sel, n, ln);
+        case 8: return step_class_any<8>(b, vie, sel, n, ln);
     }
     set_err("size1 = %d not supported (1..8)", s);
     return NESSI_ERR_ARG;
@@ -796,6 +802,24 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
         g.members.push_back(i);
         b->probs[i].group = gi;
     }
+    {
+        bool seen[NESSI_MAXS + 1] = {};
+        int classes = 0;
+        for (const Group &g : b->groups)
+            if (!seen[g.s]) {
+                seen[g.s] = true;
+                classes++;
+            }
+        b->lanes.resize((size_t)classes - 1);
+        bool ok = cudaEventCreateWithFlags(&b->ev_lanes, cudaEventDisableTiming) == cudaSuccess;
+        for (StepLane &ln : b->lanes)
+            ok = ok && cudaStreamCreateWithFlags(&ln.st, cudaStreamNonBlocking) == cudaSuccess &&
+                 cudaStreamCreateWithFlags(&ln.side, cudaStreamNonBlocking) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&ln.fork, cudaEventDisableTiming) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&ln.join, cudaEventDisableTiming) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&ln.done, cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) { set_err("stream/event creation failed"); return fail(NESSI_ERR_CUDA); }
+    }
     // device storage
     for (int i = 0; i < count; i++) {
         Prob &p = b->probs[i];
@@ -873,6 +897,13 @@ int nessi_gpu_batch_destroy(nessi_batch *b) {
     if (!b) return NESSI_OK;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
+    for (StepLane &ln : b->lanes) {
+        for (cudaStream_t t : {ln.st, ln.side})
+            if (t) { cudaStreamSynchronize(t); cudaStreamDestroy(t); }
+        for (cudaEvent_t e : {ln.fork, ln.join, ln.done})
+            if (e) cudaEventDestroy(e);
+    }
+    if (b->ev_lanes) cudaEventDestroy(b->ev_lanes);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (void *q : b->allocs) cudaFree(q);
     if (b->stage) cudaFreeHost(b->stage);
@@ -1149,7 +1180,27 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
             for (int i = 0; i < nact[gi]; i++)
                 if (!b->probs[g.members[i]].qret) { set_err("%s: Q of problem %d not set", name, g.members[i]); return NESSI_ERR_ARG; }
     }
-    for (int s = 1; s <= NESSI_MAXS; s++) {
+    // ... and groups of different size1 beside each other, each on a pair of streams of its own: a
+    // class of few problems leaves most of the SMs idle (96 uneven problems of five sizes, n 600: 13.5 ms
+    // one after the other, 12.0)
+    bool active[NESSI_MAXS + 1] = {};
+    int nclass = 0;
+    for (size_t gi = 0; gi < b->groups.size(); gi++)
+        if (nact[gi] > 0 && !active[b->groups[gi].s]) {
+            active[b->groups[gi].s] = true;
+            nclass++;
+        }
+    if (nclass > 1) CK(cudaEventRecord(b->ev_lanes, b->stream));
+    int used = 0;
+    for (int s = NESSI_MAXS; s >= 1; s--) {
+        if (!active[s]) continue;
+        StepLane ln;
+        if (used == 0) {
+            ln.st = b->stream; ln.side = b->side; ln.fork = b->ev_fork; ln.join = b->ev_join;
+        } else {
+            ln = b->lanes[used - 1];
+            CK(cudaStreamWaitEvent(ln.st, b->ev_lanes, 0));
+        }
         GroupSel sel;
         sel.ng = 0;
         for (size_t gi = 0; gi < b->groups.size(); gi++) {
@@ -1158,11 +1209,14 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
                 sel.nact[sel.ng++] = nact[gi];
             }
             if (sel.ng == NESSI_GSEL || (gi + 1 == b->groups.size() && sel.ng > 0)) {
-                CKR(step_dispatch(b, s, vie, sel, n));
+                CKR(step_dispatch(b, s, vie, sel, n, ln));
                 sel.ng = 0;
             }
         }
+        if (used > 0) CK(cudaEventRecord(ln.done, ln.st));
+        used++;
     }
+    for (int i = 1; i < used; i++) CK(cudaStreamWaitEvent(b->stream, b->lanes[i - 1].done, 0));
     return NESSI_OK;
 }
 
