@@ -316,7 +316,7 @@ def mixed_companion(b, W, nt, k, fp64_value, args, world, stream):
                     bm.lattice_2b_timestep(n, W.ncorr)
                 else:
                     bm.dyson_timestep(n)
-        prop()  # eager: the Volterra autotuner decides here
+        prop()  # eager warm-up
         bm.synchronize()
         bm.set_profiling(True)
         prop()
@@ -655,21 +655,22 @@ def main():
 
     groups = sorted(W.sigma.keys()) if isinstance(W.sigma, dict) else [0]
     volterra = {str(gid): b.volterra_choice(gid) for gid in groups}
-    # own kernels launched per timed step, from the launch structure of one Dyson step n of a group:
-    # k_prep_problem, k_prep_group, k_mat_operator, the Matsubara product, les*adv, k_tv,
-    # k_les_operands_t, tv*vt; ret and les: the start rows, a diagonal kernel per block of 128 // size1
-    # time rows and a trailing product between blocks.  A lattice step adds k_extrapolate, per corrector
-    # k_gloc + k_gloc_final + k_sigma_2b, and the final k-average.
+    # own kernels launched per timed step, from the launch structure of one Dyson step n of the groups
+    # of one size1: k_prep, k_mat_operator, the Matsubara product, les*adv, the tv row,
+    # k_les_operands_t, tv*vt; ret and les: the start rows and the product that carries them into the
+    # later rows, then a diagonal kernel per block of 4 (32 // size1) time rows with a trailing product
+    # after all but the last.  A lattice step adds k_extrapolate, per corrector k_gloc + k_gloc_final +
+    # k_sigma_2b, and the final k-average.
     def dyson_launches(n, s):
-        return 8 + 2 * (2 * ((n - k + 128 // s - 1) // (128 // s)))
+        rows = 4 * (32 // s)
+        return 7 + 2 * (1 + 2 * ((n - k + rows - 1) // rows))
     if W.lattice:
         gpu_launches = sum(1 + W.ncorr * (3 + dyson_launches(n, 1)) + 2 for n in range(k + 1, nt + 1)) * args.steps
     else:
         top = {}
         for d in W.descs:
-            g = d.get("sigma_group", 0)
-            top[g] = max(top.get(g, (0, 0)), (d["nt"], d["size1"]))
-        gpu_launches = sum(dyson_launches(n, s) for m, s in top.values() for n in range(k + 1, m + 1)) * args.steps
+            top[d["size1"]] = max(top.get(d["size1"], 0), d["nt"])
+        gpu_launches = sum(dyson_launches(n, s) for s, m in top.items() for n in range(k + 1, m + 1)) * args.steps
     mixed_err = None
     if args.mixed_error and args.precision == "mixed":
         mixed_err = compare_with_fp64(b, W, run_step, nt, k)

@@ -5,10 +5,10 @@
 //   G^tv(n, tau) = Minv_les[n] Q(tau)
 // a_j = tvcoef (k_prep_group), Cmat = K_n Gmat_all (the Matsubara integral as one group GEMM).
 //
-// The history stream is the HBM-bound part of a time step.  The register-load form (k_tv: a
-// thread per (tau, column), 4 rows in flight per thread) needs 64 warps per SM to keep enough bytes
-// in flight.  Here one persistent CTA per SM keeps up to five stages of ~32 KB in flight through
-// the bulk-copy engine, and 8 consumer warps reduce them.
+// The history stream is the HBM-bound part of a time step.  The default form (k_tv_ring) gives every
+// warp a ring of its own, filled by cp.async.  Here one persistent CTA per SM keeps up to five stages
+// of ~32 KB in flight through the bulk-copy engine, and 8 consumer warps reduce them; slower, kept as
+// an independent form of the same sums.
 //
 // Work items are (problem, tau chunk of width tw); CTA b takes items b, b + G, b + 2G, ... and the
 // stages of all its items form one sequence through a ring of STAGES buffers.  A stage holds the
