@@ -72,7 +72,9 @@ int nessi_gpu_set_G(nessi_batch *b, int p, const void *ret, const void *les, con
 int nessi_gpu_get_G(nessi_batch *b, int p, void *ret, void *les, void *tv, void *mat);
 /* One time step of G as a herm_matrix_timestep slice [ret(n,0..n) | tv(n,0..ntau) |
  * les(0..n,n)] (cntr_herm_matrix_timestep_decl.hpp:67-75; herm_matrix::get_timestep,
- * cntr_herm_matrix_impl.hpp:2156).  tstp = -1 gives mat. */
+ * cntr_herm_matrix_impl.hpp:2156).  tstp = -1 gives mat.  The slice may be reused when the call returns
+ * (a set from pageable memory has been copied by then, but its upload may still be queued); slices
+ * cannot be set or read while the batch's stream is captured. */
 int nessi_gpu_get_timestep(nessi_batch *b, int p, int tstp, void *slice);
 int nessi_gpu_set_timestep(nessi_batch *b, int p, int tstp, const void *slice);
 /* H(t) of problem p as cntr::function<double> data, (nt+2) s^2 complex. */

@@ -1071,20 +1071,20 @@ static int slice_copy(nessi_batch *b, double2 *ret, double2 *tv, double2 *les, d
     float2 *v32 = tv32 ? tv32 + tstp * M * s2 : nullptr;
     bool pageable = false;
     double2 *io = mapped_host(slice, bytes, &pageable);
+    if (!io && pageable && to_device) {
+        // the launch would be recorded, and its replays would read whatever the slot holds then: a
+        // slice stays refused while the stream is captured, here as in the paths that wait
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(b->stream, &cs));
+        if (cs != cudaStreamCaptureStatusNone) {
+            set_err("a time-step slice cannot be set while the stream is captured");
+            return NESSI_ERR_CUDA;
+        }
+    }
     int slot = -1;
     char *st = !io && pageable ? stage_slot(b, bytes, &slot) : nullptr;
     if (io || st) {
-        if (st && to_device) {
-            // the launch would be recorded, and its replays would read whatever the slot holds then: a
-            // slice stays refused while the stream is captured, here as in the paths that wait
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            CK(cudaStreamIsCapturing(b->stream, &cs));
-            if (cs != cudaStreamCaptureStatusNone) {
-                set_err("a time-step slice cannot be set while the stream is captured");
-                return NESSI_ERR_CUDA;
-            }
-            std::memcpy(st, slice, bytes);
-        }
+        if (st && to_device) std::memcpy(st, slice, bytes);
         if (st) CK(cudaHostGetDevicePointer((void **)&io, st, 0));
         const unsigned blocks = (unsigned)(2 * slice_row_blocks(nrow) + slice_tv_blocks((int)M, (int)s2, tv_planes));
         if (to_device) k_slice<false><<<blocks, 256, 0, b->stream>>>(io, r, v, l, v32, nrow, (int)M, (int)s2, tv_planes);
