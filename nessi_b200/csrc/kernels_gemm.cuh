@@ -16,13 +16,7 @@
 
 namespace zg {
 constexpr int BK = 8;        // complex k per stage (one m16n8k8 k-step)
-constexpr int LDS = BK + 4;  // shared row stride in complex: 12 = 4 (mod 8) -> conflict-free fragment loads
 constexpr int NTH = 128;     // threads of a tile group
-// shared memory (complex elements) of one tile group
-template <int BM, int BN> struct Smem {
-    static constexpr int stage = (BM + BN) * LDS;
-    static constexpr int total = 2 * stage;
-};
 }  // namespace zg
 
 // D (16x8, fp64) += A (16x8) B (8x8); fragment layout of mma.m16n8k8 .f64: with g = lane/4,
