@@ -40,7 +40,10 @@ __host__ __device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x +
 // ---- overlapped launches (programmatic stream serialization) --------------------------------
 // A kernel launched with launch_chained may start while its predecessor in the stream still runs.  It
 // waits (pdl_wait) before it reads or writes anything another kernel touches; since every kernel of a
-// chain does, "the predecessor has finished" implies that all earlier ones have.  pdl_trigger lets the
+// chain does, "the predecessor has finished" implies that all earlier ones have.  What the kernels of a
+// chain write is read by ordinary or cp.async loads only: the read-only path (__ldg, or a const
+// __restrict__ pointer) is for data that no kernel writes while the reader is resident, and pdl_wait does
+// not order it.  pdl_trigger lets the
 // successor's CTAs take free SM resources once all CTAs of this kernel have started; long streaming
 // kernels leave it out, so that waiting CTAs do not sit beside them.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -222,7 +222,11 @@ __device__ __forceinline__ void zgemm_split(const LA &la, const LB &lb, const PU
             for (int c = 0; c < 2; c++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) acc[i][j][c][e] = 0.0;
-    auto ld = [](const double2 *p) { return p ? __ldg(p) : cmk(0, 0); };
+    // Ordinary loads (ld.global.ca): a chained kernel is resident while its predecessor writes these
+    // operands, and the read-only path (ld.global.nc) may only be used for data nobody writes while the
+    // kernel lives.  __ldca and not *p: the pointers come out of a table, so that *p is a generic load
+    // (step of one problem, n 200: 117.6 us, with __ldca 113.7, with read-only loads 114.1).
+    auto ld = [](const double2 *p) { return p ? __ldca(p) : cmk(0, 0); };
 #pragma unroll 2
     for (int k0 = warp * 8; k0 < K; k0 += 64) {
         double2 a[2][4], b[NT][2];

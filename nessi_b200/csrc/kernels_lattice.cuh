@@ -122,10 +122,10 @@ __global__ void __launch_bounds__(256) k_gloc(GroupDev g, const ProbDev *__restr
     }
 }
 
-// pass 2: G_loc element e = (1/P) sum_c part[c][e], chunks in order, stored in libcntr layout
+// pass 2: G_loc element e = (1/P) sum_c part[c][e], chunks in order, stored in libcntr layout.  part is
+// not restrict: k_gloc still writes it when this kernel, launched beside it, is already resident.
 template <int S>
-__global__ void k_gloc_final(GroupDev g, int nprob, int tstp, const double2 *__restrict__ part, long ldpart,
-                             int nchunk, LocDev loc) {
+__global__ void k_gloc_final(GroupDev g, int nprob, int tstp, const double2 *part, long ldpart, int nchunk, LocDev loc) {
     pdl_entry();
     const int s2 = S * S, M = g.ntau + 1;
     const long nret = tstp >= 0 ? (long)(tstp + 1) * s2 : 0, ntv = (long)M * s2;
