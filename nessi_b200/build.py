@@ -1,8 +1,9 @@
 """Build recipe for libnessi_gpu.so (in-tree, sm_100a) and libnessi_io.so (host only).
 
 ``python -m nessi_b200.build`` compiles nessi_b200/csrc/*.cu with nvcc for
-``-gencode arch=compute_100a,code=sm_100a`` into nessi_b200/libnessi_gpu.so, and the text
-checkpoint format (csrc/hm_text_io.cpp) with g++ into nessi_b200/libnessi_io.so.
+``-gencode arch=compute_100a,code=sm_100a`` into nessi_b200/nessi_gpu.o and links it into
+nessi_b200/libnessi_gpu.so, and the text checkpoint format (csrc/hm_text_io.cpp) with g++ into
+nessi_b200/libnessi_io.so.
 No GPU is needed to build.
 """
 import os
@@ -13,10 +14,11 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnessi_gpu.so")
+OBJ = os.path.join(HERE, "nessi_gpu.o")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
-         "-Xcompiler", "-fPIC", "-shared", "-ccbin", "/usr/bin/g++"]
-SOURCES = ["nessi_gpu.cu"]
+         "-Xcompiler", "-fPIC", "-ccbin", "/usr/bin/g++"]
+SOURCE = "nessi_gpu.cu"
 IO_LIB = os.path.join(HERE, "libnessi_io.so")
 IO_SOURCES = [os.path.join(CSRC, "hm_text_io.cpp"), os.path.join(os.path.dirname(HERE), "include", "nessi_io.h")]
 CXX = "/usr/bin/g++"  # the host compiler nvcc uses for the CUDA library
@@ -31,11 +33,28 @@ def _inputs():
     return out
 
 
-def up_to_date():
-    if not os.path.exists(LIB):
+def up_to_date(path=LIB):
+    if not os.path.exists(path):
         return False
-    t = os.path.getmtime(LIB)
+    t = os.path.getmtime(path)
     return all(os.path.getmtime(f) <= t for f in _inputs())
+
+
+def build_object(force=False, verbose=False):
+    """nessi_gpu.o, the compiled library before it is linked with the CUDA runtime."""
+    if not force and up_to_date(OBJ):
+        return OBJ
+    tmp = OBJ + ".tmp"
+    cmd = [NVCC] + FLAGS + ["-c", "-o", tmp, os.path.join(CSRC, SOURCE)]
+    if verbose:
+        print(" ".join(cmd))
+    start = time.time()
+    subprocess.check_call(cmd, cwd=CSRC)
+    os.replace(tmp, OBJ)
+    # stamp the object with the time the compile read its sources, so that a source edited
+    # while nvcc ran is newer than the object and the next build compiles it
+    os.utime(OBJ, (start, start))
+    return OBJ
 
 
 def build_io(force=False, verbose=False):
@@ -56,16 +75,15 @@ def build(force=False, verbose=False):
     build_io(force=force, verbose=verbose)
     if not force and up_to_date():
         return LIB
+    build_object(force=force, verbose=verbose)
     tmp = LIB + ".tmp"
-    cmd = [NVCC] + FLAGS + ["-o", tmp] + [os.path.join(CSRC, s) for s in SOURCES]
+    cmd = [NVCC] + FLAGS + ["-shared", "-o", tmp, OBJ]
     if verbose:
         print(" ".join(cmd))
-    start = time.time()
     subprocess.check_call(cmd, cwd=CSRC)
     os.replace(tmp, LIB)  # a process that has the old library loaded keeps its copy
-    # stamp the library with the time the compile read its sources, so that a source edited
-    # while nvcc ran is newer than the library and the next build compiles it
-    os.utime(LIB, (start, start))
+    stamp = os.path.getmtime(OBJ)  # as the object: newer sources are compiled next time
+    os.utime(LIB, (stamp, stamp))
     return LIB
 
 

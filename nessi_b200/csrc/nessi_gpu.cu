@@ -1,5 +1,6 @@
 // libnessi_gpu.so: batches of Kadanoff-Baym problems advanced on one B200.
 // Host side of the C ABI declared in include/nessi_gpu.h.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -1002,21 +1003,46 @@ int nessi_gpu_get_G(nessi_batch *b, int p, void *ret, void *les, void *tv, void 
     return NESSI_OK;
 }
 
-// Device address of a host buffer that is pinned and mapped from its first to its last byte, else
-// null; *pageable tells whether the driver does not know the memory at all.
-static double2 *mapped_host(const void *host, size_t bytes, bool *pageable) {
-    cudaPointerAttributes a0, a1;
+// What the driver says of a host address (all zero: it does not know the memory)
+struct HostMem {
+    unsigned long long type = 0, managed = 0, device = 0, start = 0, size = 0, access = 0;
+};
+static bool host_mem(const void *p, HostMem *m) {
+    using Fn = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Fn fn = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) != cudaSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (Fn)f;
+    }();
+    *m = HostMem();
+    CUpointer_attribute at[6] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                 CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void *out[6] = {&m->type, &m->managed, &m->device, &m->start, &m->size, &m->access};
+    return fn && fn(6, at, out, (CUdeviceptr)(uintptr_t)p) == CUDA_SUCCESS;
+}
+
+// Device address of a host buffer that lies as a whole in one pinned, mapped range which the device may
+// read (and, where it is written, write), else null.  The first and the last byte alone do not show
+// that: two registrations may have a gap between them.  *pageable tells whether the driver knows
+// neither the first byte nor the last, so that the buffer can go through a staging slot.
+static double2 *mapped_host(const void *host, size_t bytes, bool written, bool *pageable) {
+    HostMem a, z;
     *pageable = false;
-    if (cudaPointerGetAttributes(&a0, host) != cudaSuccess ||
-        cudaPointerGetAttributes(&a1, (const char *)host + bytes - 1) != cudaSuccess) {
-        cudaGetLastError();
+    if (!host_mem(host, &a)) return nullptr;
+    if (a.type == 0) {
+        *pageable = host_mem((const char *)host + bytes - 1, &z) && z.type == 0;
         return nullptr;
     }
-    *pageable = a0.type == cudaMemoryTypeUnregistered && a1.type == cudaMemoryTypeUnregistered;
-    if (a0.type != cudaMemoryTypeHost || a1.type != cudaMemoryTypeHost || !a0.devicePointer ||
-        (char *)a1.devicePointer - (char *)a0.devicePointer != (long)bytes - 1 || ((size_t)a0.devicePointer & 15))
+    const unsigned long long need = written ? CU_MEM_ACCESS_FLAGS_PROT_READWRITE : CU_MEM_ACCESS_FLAGS_PROT_READ;
+    if (a.type != CU_MEMORYTYPE_HOST || a.managed || !a.device || (a.device & 15) || (a.access & need) != need ||
+        a.device < a.start || a.device - a.start > a.size || bytes > a.size - (a.device - a.start))
         return nullptr;
-    return (double2 *)a0.devicePointer;
+    return (double2 *)a.device;
 }
 
 // A free staging slot of at least `bytes` (null: no pinned memory, the caller copies without one)
@@ -1070,7 +1096,7 @@ static int slice_copy(nessi_batch *b, double2 *ret, double2 *tv, double2 *les, d
     double2 *r = ret + tri_h(tstp) * s2, *v = tv + tstp * M * s2, *l = les + tri_h(tstp) * s2;
     float2 *v32 = tv32 ? tv32 + tstp * M * s2 : nullptr;
     bool pageable = false;
-    double2 *io = mapped_host(slice, bytes, &pageable);
+    double2 *io = mapped_host(slice, bytes, !to_device, &pageable);
     if (!io && pageable && to_device) {
         // the launch would be recorded, and its replays would read whatever the slot holds then: a
         // slice stays refused while the stream is captured, here as in the paths that wait

@@ -1,0 +1,81 @@
+"""Host code of the library where a call fails or a buffer is not what it seems, on a CUDA runtime without
+a device (fake_runtime.py): which calls are made, in which order, and what a failed call leaves behind."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import fake_runtime
+
+PAGE = 4096
+_open = []
+
+
+@pytest.fixture
+def fake():
+    gpu, f = fake_runtime.load()
+    f.reset()
+    f.unpin_all()
+    yield gpu, f
+    f.reset()
+    f.unpin_all()
+    while _open:
+        _open.pop().close()
+    gpu.finalize()
+
+
+def _batch(gpu, shapes, nt=40, ntau=16, k=5):
+    """A batch with one group per (size1, problems)."""
+    b = gpu.Batch([dict(nt=nt, ntau=ntau, size1=s, sig=-1, solve_order=k, sigma_group=g, beta=2.0, h=0.1)
+                   for g, (s, cnt) in enumerate(shapes) for _ in range(cnt)])
+    _open.append(b)
+    return b
+
+
+def _pages(n):
+    """A page-aligned host buffer of n pages: (owner, address)."""
+    a = np.zeros((n + 1) * PAGE, np.uint8)
+    return a, (a.ctypes.data + PAGE - 1) // PAGE * PAGE
+
+
+def _launched(f, kernel):
+    return [x for x in f.calls("launch") if kernel in x]
+
+
+# ---- slices in host memory of different kinds -------------------------------------------------------
+NT, NTAU = 400, 100  # a slice of step 400: 14.4 kB, four pages
+
+
+@pytest.mark.parametrize("pins,write,direct", [
+    ([(0, 4)], True, True),                     # one range over all of it
+    ([(0, 4)], False, True),
+    ([(0, 1), (3, 1)], True, False),            # first and last byte pinned, a gap between
+    ([(0, 1), (3, 1)], False, False),
+    ([(0, 2), (2, 2)], True, False),            # two ranges side by side are two mappings
+    ([(0, 3)], True, False),                    # the end is pageable
+    ([(1, 3)], True, False),                    # the start is
+    ([(0, 4, "read")], False, True),            # a range the device may only read
+    ([(0, 4, "read")], True, False),
+])
+def test_only_memory_in_one_range_is_used_in_place(fake, pins, write, direct):
+    gpu, f = fake
+    b = _batch(gpu, [(1, 1)], NT, NTAU)
+    owner, base = _pages(4)
+    for p in pins:
+        f.pin(base + p[0] * PAGE, p[1] * PAGE, read_only=len(p) > 2)
+    L = gpu.load_library()
+    f.reset()
+    call = L.nessi_gpu_get_timestep if write else L.nessi_gpu_set_timestep
+    assert call(b._h, 0, NT, ctypes.c_void_p(base)) == 0
+    assert len(_launched(f, "k_slice")) == (1 if direct else 0)
+    assert len(f.calls("cudaMemcpyAsync")) == (0 if direct else 3)
+    assert not f.calls("cudaHostAlloc")
+
+
+def test_pageable_slices_go_through_a_slot(fake):
+    gpu, f = fake
+    b = _batch(gpu, [(1, 1)], NT, NTAU)
+    owner, base = _pages(4)
+    f.reset()
+    assert gpu.load_library().nessi_gpu_set_timestep(b._h, 0, NT, ctypes.c_void_p(base)) == 0
+    assert len(_launched(f, "k_slice")) == 1 and not f.calls("cudaStreamSynchronize")
