@@ -1196,6 +1196,36 @@ static int find_group_checked(nessi_batch *b, int group, Group **out) {
     return NESSI_OK;
 }
 
+// Streams of the i-th size1 class of a step: the batch's own, then the lanes
+static StepLane step_lane(const nessi_batch *b, int i) {
+    if (i > 0) return b->lanes[i - 1];
+    StepLane ln;
+    ln.st = b->stream; ln.side = b->side; ln.fork = b->ev_fork; ln.join = b->ev_join;
+    return ln;
+}
+
+// The batch stream waits for the first `used` lanes.  A step joins its side stream itself, unless it
+// failed: then that is done here, so that nothing it launched runs beside the caller's next call.  The
+// step's error stands; one of the joins after it is not reported.
+static int join_lanes(nessi_batch *b, int used, bool failed) {
+    cudaError_t err = cudaSuccess;
+    auto keep = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
+    for (int i = 0; i < used; i++) {
+        const StepLane ln = step_lane(b, i);
+        if (failed) {
+            keep(cudaEventRecord(ln.join, ln.side));
+            keep(cudaStreamWaitEvent(ln.st, ln.join, 0));
+        }
+        if (i > 0) {
+            keep(cudaEventRecord(ln.done, ln.st));
+            keep(cudaStreamWaitEvent(b->stream, ln.done, 0));
+        }
+    }
+    if (failed) cudaGetLastError();
+    else CK(err);
+    return NESSI_OK;
+}
+
 static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
     NvtxRange nvtx_(vie ? "nessi::vie2_timestep" : "nessi::dyson_timestep");
     CKR(check_batch(b));
@@ -1227,33 +1257,29 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
             nclass++;
         }
     if (nclass > 1) CK(cudaEventRecord(b->ev_lanes, b->stream));
-    int used = 0;
-    for (int s = NESSI_MAXS; s >= 1; s--) {
+    int used = 0, rc = NESSI_OK;
+    for (int s = NESSI_MAXS; s >= 1 && rc == NESSI_OK; s--) {
         if (!active[s]) continue;
-        StepLane ln;
-        if (used == 0) {
-            ln.st = b->stream; ln.side = b->side; ln.fork = b->ev_fork; ln.join = b->ev_join;
-        } else {
-            ln = b->lanes[used - 1];
-            CK(cudaStreamWaitEvent(ln.st, b->ev_lanes, 0));
+        const StepLane ln = step_lane(b, used++);
+        if (used > 1 && cudaStreamWaitEvent(ln.st, b->ev_lanes, 0) != cudaSuccess) {
+            set_err("%s: forking a stream failed", name);
+            rc = NESSI_ERR_CUDA;
         }
         GroupSel sel;
         sel.ng = 0;
-        for (size_t gi = 0; gi < b->groups.size(); gi++) {
+        for (size_t gi = 0; gi < b->groups.size() && rc == NESSI_OK; gi++) {
             if (b->groups[gi].s == s && nact[gi] > 0) {
                 sel.gid[sel.ng] = (int)gi;
                 sel.nact[sel.ng++] = nact[gi];
             }
             if (sel.ng == NESSI_GSEL || (gi + 1 == b->groups.size() && sel.ng > 0)) {
-                CKR(step_dispatch(b, s, vie, sel, n, ln));
+                rc = step_dispatch(b, s, vie, sel, n, ln);
                 sel.ng = 0;
             }
         }
-        if (used > 0) CK(cudaEventRecord(ln.done, ln.st));
-        used++;
     }
-    for (int i = 1; i < used; i++) CK(cudaStreamWaitEvent(b->stream, b->lanes[i - 1].done, 0));
-    return NESSI_OK;
+    const int joined = join_lanes(b, used, rc != NESSI_OK);
+    return rc != NESSI_OK ? rc : joined;
 }
 
 int nessi_gpu_dyson_timestep(nessi_batch *b, int n) { return timestep_kind(b, n, false, "dyson_timestep"); }

@@ -21,16 +21,19 @@ static std::map<void *, int> g_ids;  // streams and events by their order of cre
 struct HostRange { char *p; size_t n; int access; };
 static std::vector<HostRange> g_host;  // pinned ranges
 static int g_next = 1;
+static cudaError_t g_last = cudaSuccess;
 static std::string g_pushed;
 static std::vector<cudaStream_t> g_push_stream;
 
 static int id_of(const void *p) { return p ? g_ids[(void *)p] : 0; }
+// a call that fails by plan has "failed" in front of its name in the log
 static cudaError_t call(const char *name, const std::string &what = "") {
-    g_log.push_back(std::string(name) + (what.empty() ? "" : " " + what));
     const long n = ++g_calls[name];
     auto it = g_plan.find(name);
-    if (it != g_plan.end() && it->second.count(n)) return (cudaError_t)it->second[n];
-    return cudaSuccess;
+    const int error = it != g_plan.end() && it->second.count(n) ? it->second[n] : 0;
+    g_log.push_back((error ? "failed " : "") + std::string(name) + (what.empty() ? "" : " " + what));
+    if (error) g_last = (cudaError_t)error;
+    return (cudaError_t)error;
 }
 static std::string num(long long x) { return std::to_string(x); }
 template <class T> static cudaError_t create(const char *name, T *out) {
@@ -49,7 +52,7 @@ static const HostRange *range_of(const void *p) {
 
 extern "C" {
 // ---- for the tests
-void fake_reset(void) { g_log.clear(); g_plan.clear(); g_calls.clear(); }
+void fake_reset(void) { g_log.clear(); g_plan.clear(); g_calls.clear(); g_last = cudaSuccess; }
 void fake_fail(const char *name, long nth, int error) { g_calls[name] = 0; g_plan[name][nth] = error; }
 long fake_log_size(void) { return (long)g_log.size(); }
 const char *fake_log_line(long i) { return g_log[i].c_str(); }
@@ -94,7 +97,11 @@ cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) { *v = a == cudaDevAttrMultiProcessorCount ? 148 : 232448; return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize(void) { return call("cudaDeviceSynchronize"); }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void) {
+    const cudaError_t e = g_last;
+    g_last = cudaSuccess;
+    return e;
+}
 const char *cudaGetErrorName(cudaError_t) { return "fake error"; }
 const char *cudaGetErrorString(cudaError_t) { return "planned by the test"; }
 

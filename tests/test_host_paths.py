@@ -79,3 +79,49 @@ def test_pageable_slices_go_through_a_slot(fake):
     f.reset()
     assert gpu.load_library().nessi_gpu_set_timestep(b._h, 0, NT, ctypes.c_void_p(base)) == 0
     assert len(_launched(f, "k_slice")) == 1 and not f.calls("cudaStreamSynchronize")
+
+
+# ---- order of a step's launches -----------------------------------------------------------------------
+def _order(log):
+    """(launches, what each stream's next operation is ordered after), from a log: launches by number,
+    streams and events as sets of the launches they wait for."""
+    seen, events, launches = {}, {}, []
+    for line in log:
+        w = line.split()
+        if w[0] == "launch":
+            launches.append(line)
+            seen.setdefault(w[1], set()).add(len(launches) - 1)
+        elif w[0] == "cudaEventRecord":
+            events[w[1]] = set(seen.get(w[2], ()))
+        elif w[0] == "cudaStreamWaitEvent":
+            seen.setdefault(w[1], set()).update(events.get(w[2], ()))
+    return launches, seen
+
+
+def _batch_stream(f, b, gpu):
+    """The number of the batch stream: it is the one that synchronize waits for."""
+    f.reset()
+    b.synchronize()
+    return f.calls("cudaStreamSynchronize")[0].split()[1]
+
+
+@pytest.mark.parametrize("shapes", [[(1, 3)], [(1, 2), (3, 2), (8, 1)]])
+def test_every_launch_of_a_step_is_joined_whatever_fails(fake, shapes):
+    gpu, f = fake
+    b = _batch(gpu, shapes)
+    main = _batch_stream(f, b, gpu)
+    b.dyson_timestep(20)
+    for call in ("launch", "cudaEventRecord", "cudaStreamWaitEvent"):
+        f.reset()
+        b.dyson_timestep(20)
+        count = len(f.calls(call))
+        launches, seen = _order(f.log())
+        assert len(launches) > 10 * len(shapes) and seen[main] == set(range(len(launches)))
+        for nth in range(1, count + 1):
+            f.reset()
+            f.fail(call, nth, 1)
+            with pytest.raises(gpu.NessiGpuError):
+                b.dyson_timestep(20)
+            launches, seen = _order(f.log())
+            if call == "launch" or nth <= count - 2 * (len(shapes) - 1):  # a last join that fails can only be reported
+                assert seen.get(main, set()) == set(range(len(launches))), (call, nth)
