@@ -115,6 +115,7 @@ struct Prob {
     double2 *H = nullptr, *minv_ret = nullptr, *minv_les = nullptr;
     float2 *gtv32 = nullptr;
     double2 *qret = nullptr, *qles = nullptr, *qtv = nullptr, *qmat = nullptr;  // VIE2 source term
+    bool has_q = false;              // all of them allocated and in the device descriptor
 };
 
 struct Group {
@@ -224,6 +225,9 @@ struct nessi_batch {
         *p = (double2 *)q;
         return NESSI_OK;
     }
+    // For sets of arrays that are allocated at their first use: what an earlier, failed call got stays, so
+    // that a repeated call completes the set
+    int alloc_once(double2 **p, long long n_cplx) { return *p ? NESSI_OK : alloc(p, n_cplx); }
 };
 
 namespace {
@@ -1244,7 +1248,7 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
         nact[gi] = active_members(b, g, n);
         if (vie)
             for (int i = 0; i < nact[gi]; i++)
-                if (!b->probs[g.members[i]].qret) { set_err("%s: Q of problem %d not set", name, g.members[i]); return NESSI_ERR_ARG; }
+                if (!b->probs[g.members[i]].has_q) { set_err("%s: Q of problem %d not set", name, g.members[i]); return NESSI_ERR_ARG; }
     }
     // ... and groups of different size1 beside each other, each on a pair of streams of its own: a
     // class of few problems leaves most of the SMs idle (96 uneven problems of five sizes, n 600: 13.5 ms
@@ -1358,7 +1362,7 @@ static int start_kind(nessi_batch *b, bool vie, const char *name) {
         any = true;
         for (int i : g.members) {
             if (b->probs[i].d.nt < g.k) { set_err("%s: nt must be >= SolveOrder", name); return NESSI_ERR_ARG; }
-            if (vie && !b->probs[i].qret) { set_err("%s: Q of problem %d not set", name, i); return NESSI_ERR_ARG; }
+            if (vie && !b->probs[i].has_q) { set_err("%s: Q of problem %d not set", name, i); return NESSI_ERR_ARG; }
         }
     }
     if (!any) { set_err("%s: the batch has no %s group", name, vie ? "VIE2 (nessi_gpu_set_F)" : "Dyson"); return NESSI_ERR_ARG; }
@@ -1414,13 +1418,15 @@ static int sync_probdev(nessi_batch *b, int p) {
 
 static int ensure_q(nessi_batch *b, int p) {
     Prob &q = b->probs[p];
-    if (q.qret) return NESSI_OK;
+    if (q.has_q) return NESSI_OK;
     const long s2 = (long)q.d.size1 * q.d.size1, nt = q.d.nt, M = q.d.ntau + 1;
-    CKR(b->alloc(&q.qret, tri_h(nt + 1) * s2));
-    CKR(b->alloc(&q.qles, tri_h(nt + 1) * s2));
-    CKR(b->alloc(&q.qtv, (nt + 1) * M * s2));
-    CKR(b->alloc(&q.qmat, M * s2));
-    return sync_probdev(b, p);
+    CKR(b->alloc_once(&q.qret, tri_h(nt + 1) * s2));
+    CKR(b->alloc_once(&q.qles, tri_h(nt + 1) * s2));
+    CKR(b->alloc_once(&q.qtv, (nt + 1) * M * s2));
+    CKR(b->alloc_once(&q.qmat, M * s2));
+    CKR(sync_probdev(b, p));
+    q.has_q = true;
+    return NESSI_OK;
 }
 
 int nessi_gpu_set_Q(nessi_batch *b, int p, const void *ret, const void *les, const void *tv, const void *mat) {
@@ -1443,13 +1449,16 @@ int nessi_gpu_set_Q_timestep(nessi_batch *b, int p, int tstp, const void *slice)
     return slice_copy(b, q.qret, q.qtv, q.qles, q.qmat, q.d.nt, q.d.ntau, q.d.size1, tstp, (void *)slice, true, true);
 }
 
+// Makes a group a VIE2 group: with all its arrays and the device table in place, or not at all
 static int ensure_fcc(nessi_batch *b, Group &g) {
-    g.vie = true;
-    if (g.fccret) return NESSI_OK;
+    if (g.vie) return NESSI_OK;
     const long s2 = (long)g.s * g.s, N = g.ntmax + 1;
-    CKR(b->alloc(&g.fccret, tri_h(N) * s2));
-    CKR(b->alloc(&g.fccles, tri_h(N) * s2));
-    return sync_groups(b);
+    CKR(b->alloc_once(&g.fccret, tri_h(N) * s2));
+    CKR(b->alloc_once(&g.fccles, tri_h(N) * s2));
+    g.vie = true;
+    const int r = sync_groups(b);
+    if (r != NESSI_OK) g.vie = false;
+    return r;
 }
 
 int nessi_gpu_set_F(nessi_batch *b, int group, const void *ret, const void *les, const void *tv, const void *mat,
@@ -1478,8 +1487,11 @@ int nessi_gpu_set_Fcc_mat(nessi_batch *b, int group, const void *cc_mat) {
     CKR(ensure_fcc(b, *g));
     const long M = g->ntau + 1, s2 = (long)g->s * g->s;
     if (!g->fccmat) {
-        CKR(b->alloc(&g->fccmat, M * s2));
-        CKR(sync_groups(b));
+        double2 *m = nullptr;
+        CKR(b->alloc(&m, M * s2));
+        g->fccmat = m;
+        const int r = sync_groups(b);
+        if (r != NESSI_OK) { g->fccmat = nullptr; return r; }
     }
     CKR(copy_cplx(b, g->fccmat, cc_mat, M * s2, cudaMemcpyHostToDevice));
     CK(cudaStreamSynchronize(b->stream));
@@ -1507,16 +1519,15 @@ int nessi_gpu_set_F_timestep(nessi_batch *b, int group, int tstp, const void *sl
 
 
 static int ensure_loc(nessi_batch *b, Group &g) {
-    if (g.loc.ret) return NESSI_OK;
+    if (g.gloc_part) return NESSI_OK;  // the last one of the set
     const long s2 = (long)g.s * g.s, N = g.ntmax + 1, M = g.ntau + 1;
-    CKR(b->alloc(&g.loc.ret, tri_h(N) * s2));
-    CKR(b->alloc(&g.loc.les, tri_h(N) * s2));
-    CKR(b->alloc(&g.loc.tv, N * M * s2));
-    CKR(b->alloc(&g.loc.mat, M * s2));
+    CKR(b->alloc_once(&g.loc.ret, tri_h(N) * s2));
+    CKR(b->alloc_once(&g.loc.les, tri_h(N) * s2));
+    CKR(b->alloc_once(&g.loc.tv, N * M * s2));
+    CKR(b->alloc_once(&g.loc.mat, M * s2));
     g.gloc_ld = (2 * N + M) * s2;  // longest slice
     const long nchunk = ((long)g.members.size() + GLOC_CHUNK - 1) / GLOC_CHUNK;
-    CKR(b->alloc(&g.gloc_part, nchunk * g.gloc_ld));
-    return NESSI_OK;
+    return b->alloc_once(&g.gloc_part, nchunk * g.gloc_ld);
 }
 
 int nessi_gpu_set_U(nessi_batch *b, int group, const void *U) {

@@ -125,3 +125,70 @@ def test_every_launch_of_a_step_is_joined_whatever_fails(fake, shapes):
             launches, seen = _order(f.log())
             if call == "launch" or nth <= count - 2 * (len(shapes) - 1):  # a last join that fails can only be reported
                 assert seen.get(main, set()) == set(range(len(launches))), (call, nth)
+
+
+# ---- arrays that are allocated at their first use --------------------------------------------------------
+def _hm(gpu, nt=40, ntau=16, s=2):
+    from nessi_b200 import herm_matrix
+    return herm_matrix(nt, ntau, s, -1)
+
+
+def _table_uploads(f):
+    """The copies of sync_groups: the ones that are waited for right after."""
+    log = f.log()
+    return [a for a, z in zip(log, log[1:]) if a.startswith("cudaMemcpyAsync") and z.startswith("cudaStreamSynchronize")]
+
+
+@pytest.mark.parametrize("call,nth", [("cudaMalloc", 1), ("cudaMalloc", 2), ("cudaMemcpyAsync", 1), ("cudaStreamSynchronize", 1)])
+def test_a_group_becomes_vie2_as_a_whole(fake, call, nth):
+    gpu, f = fake
+    f.reset()
+    b = _batch(gpu, [(2, 2)])
+    table = _table_uploads(f)[-1]  # the last one of the creation
+    F = _hm(gpu)
+    b.dyson_timestep(20)
+    f.reset()
+    f.fail(call, nth)
+    with pytest.raises(gpu.NessiGpuError):
+        b.set_F(0, F, F)
+    f.reset()
+    with pytest.raises(gpu.NessiGpuError) as e:  # not yet: no launch on half of its arrays
+        b.vie2_timestep(20)
+    assert "has no VIE2" in str(e.value) and not f.calls("launch")
+    b.set_F(0, F, F)
+    assert table in _table_uploads(f) and len(f.calls("cudaMalloc")) <= 3  # the rest of F, and Fcc^mat
+    for p in (0, 1):
+        b.set_Q(p, F)
+    b.vie2_timestep(20)
+
+
+@pytest.mark.parametrize("nth", [1, 2, 3, 4])
+def test_a_source_term_is_set_as_a_whole(fake, nth):
+    gpu, f = fake
+    b = _batch(gpu, [(2, 1)])
+    F = _hm(gpu)
+    b.set_F(0, F, F)
+    f.reset()
+    f.fail("cudaMalloc", nth)
+    with pytest.raises(gpu.NessiGpuError):
+        b.set_Q(0, F)
+    f.reset()
+    with pytest.raises(gpu.NessiGpuError) as e:
+        b.vie2_timestep(20)
+    assert "not set" in str(e.value) and not f.calls("launch")
+    b.set_Q(0, F)
+    assert len(f.calls("cudaMalloc")) == 5 - nth  # what the failed call had got is kept
+    b.vie2_timestep(20)
+
+
+@pytest.mark.parametrize("nth", [1, 2, 3, 4, 5])
+def test_the_average_is_allocated_as_a_whole(fake, nth):
+    gpu, f = fake
+    b = _batch(gpu, [(2, 3)])
+    f.reset()
+    f.fail("cudaMalloc", nth)
+    with pytest.raises(gpu.NessiGpuError):
+        b.gloc_timestep(0, 20)
+    f.reset()
+    b.gloc_timestep(0, 20)
+    assert len(f.calls("cudaMalloc")) == 6 - nth and _launched(f, "k_gloc_final")
