@@ -170,6 +170,7 @@ struct nessi_batch {
     cudaStream_t side = nullptr;       // runs the retarded component concurrently with tv
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_lanes = nullptr;
     std::vector<StepLane> lanes;       // for the second, third, ... size1 of the batch
+    bool waited = false;               // the last operation of `stream` may be a wait for another stream
     bool own_stream = true;
     cudaGraphExec_t graph = nullptr;                     // recorded time steps (nessi_gpu_graph_record)
     std::vector<Prob> probs;
@@ -208,6 +209,13 @@ struct nessi_batch {
         prof_mark(id, st);
         kp[id].launches++;
         kp[id].bytes += bytes;
+    }
+
+    // whether the next launch on the batch stream may be chained
+    bool chains() {
+        const bool c = !waited;
+        waited = false;
+        return c;
     }
 
     int alloc(double2 **p, long long n_cplx) {
@@ -293,11 +301,12 @@ int share_sm(const void *kernel, size_t smem) {
     return NESSI_OK;
 }
 
-// Launch that may start before the previous kernel of the stream has finished: the kernel waits for
-// it (griddepcontrol.wait) before it touches anything that an earlier kernel of the chain wrote.
-// Not for the first kernel after a wait for another stream: that one is launched plainly.
+// Chained launch (programmatic stream serialization): the kernel may start before the previous kernel of
+// the stream has finished, and waits for it (griddepcontrol.wait) before it touches anything that an
+// earlier kernel of the chain wrote.  The first kernel after a wait for another stream is launched
+// plainly: it has nothing to overlap with, and a recorded graph gets full edges from both streams there.
 template <class... P, class... A>
-int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+int launch(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -307,9 +316,13 @@ int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained ? 1 : 0;
     CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
     return NESSI_OK;
+}
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    return launch(true, kernel, grid, block, smem, st, args...);
 }
 
 // Products on the repo's DMMA GEMM (kernels_gemm.cuh).  Long K, or too few 32 x 32 tiles for the
@@ -462,8 +475,8 @@ int tv_stream_launch(nessi_batch *b, const GroupDev &gd, const Group &g, int n, 
 }
 
 // Time step n of the selected groups, all of size1 = S and one kind: every kernel is one launch for
-// all of them.
-template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, int n, const StepLane &ln) {
+// all of them.  chained: its first kernel follows another one, not a wait for another stream.
+template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, int n, const StepLane &ln, bool chained) {
     cudaStream_t st = ln.st;
     const GroupDev *gt = b->d_groups;
     const unsigned ng = (unsigned)sel.ng;
@@ -507,7 +520,7 @@ template <int S, bool VIE> int step_class(nessi_batch *b, const GroupSel &sel, i
     // step matrices, tv coefficients, dense Sigma
     b->prof_mark(NESSI_KERNEL_PREP, st);
     const unsigned ngb = (unsigned)std::min<long>((prep + 255) / 256, 1184);
-    CKR(launch_chained(k_prep<S, VIE>, dim3((unsigned)maxact + ngb, ng), 256, 0, st, gt, sel, ps, n, maxact));
+    CKR(launch(chained, k_prep<S, VIE>, dim3((unsigned)maxact + ngb, ng), 256, 0, st, gt, sel, ps, n, maxact));
     b->prof_end(NESSI_KERNEL_PREP, 0.0, st);
     // Matsubara part of the tv row: Cmat = K_n Gmat_all (one GEMM per group)
     b->prof_mark(NESSI_KERNEL_MATOP, st);
@@ -649,7 +662,7 @@ int active_members(const nessi_batch *b, const Group &g, int tstp) {
 template <int S> int extrap_group(nessi_batch *b, Group &g, int n) {
     const long work = ((long)g.ntau + 1 + 2L * (n + 2)) * S * S;
     dim3 grid((unsigned)std::min<long>((work + 255) / 256, 64), (unsigned)g.members.size());
-    return launch_chained(k_extrapolate<S>, grid, 256, 0, b->stream, group_dev(g), g.d_probs, n);
+    return launch(b->chains(), k_extrapolate<S>, grid, 256, 0, b->stream, group_dev(g), g.d_probs, n);
 }
 
 template <int S> int gloc_group(nessi_batch *b, Group &g, int tstp) {
@@ -658,7 +671,7 @@ template <int S> int gloc_group(nessi_batch *b, Group &g, int tstp) {
     const long M = g.ntau + 1, s2 = (long)S * S;
     const long total = tstp >= 0 ? (2L * (tstp + 1) + M) * s2 : M * s2;
     const int nchunk = (nact + GLOC_CHUNK - 1) / GLOC_CHUNK;
-    CKR(launch_chained(k_gloc<S>, dim3((unsigned)((total + 31) / 32), (unsigned)nchunk), dim3(32, 8), 0, b->stream,
+    CKR(launch(b->chains(), k_gloc<S>, dim3((unsigned)((total + 31) / 32), (unsigned)nchunk), dim3(32, 8), 0, b->stream,
                        group_dev(g), g.d_probs, nact, tstp, g.gloc_part, g.gloc_ld));
     return launch_chained(k_gloc_final<S>, dim3((unsigned)std::min<long>((total + 255) / 256, 1184)), 256, 0, b->stream,
                           group_dev(g), nact, tstp, g.gloc_part, g.gloc_ld, nchunk, g.loc);
@@ -675,7 +688,7 @@ template <int S> int sigma2b_group(nessi_batch *b, Group &g, int tstp) {
     const long M = g.ntau + 1, s2 = (long)S * S;
     const long work = tstp >= 0 ? ((long)tstp + 1 + M) * s2 : M * s2;
     SigOut o{g.sret, g.sles, g.stv, g.smat};
-    CKR(launch_chained(k_sigma_2b<S>, dim3((unsigned)std::min<long>((work + 255) / 256, 1184)), 256, 0, b->stream,
+    CKR(launch(b->chains(), k_sigma_2b<S>, dim3((unsigned)std::min<long>((work + 255) / 256, 1184)), 256, 0, b->stream,
                        group_dev(g), g.loc, g.U, tstp, o));
     sigma_changed(g, tstp);
     return NESSI_OK;
@@ -704,20 +717,20 @@ int mat_dispatch(nessi_batch *b, Group &g, int method, int force_herm) {
 }
 int vie2_mat_dispatch(nessi_batch *b, Group &g, int method) { NESSI_SIZE_SWITCH(vie2_mat_group, b, g, method) }
 
-template <int S> int step_class_any(nessi_batch *b, bool vie, const GroupSel &sel, int n, const StepLane &ln) {
-    return vie ? step_class<S, true>(b, sel, n, ln) : step_class<S, false>(b, sel, n, ln);
+template <int S> int step_class_any(nessi_batch *b, bool vie, const GroupSel &sel, int n, const StepLane &ln, bool chained) {
+    return vie ? step_class<S, true>(b, sel, n, ln, chained) : step_class<S, false>(b, sel, n, ln, chained);
 }
 
-int step_dispatch(nessi_batch *b, int s, bool vie, const GroupSel &sel, int n, const StepLane &ln) {
+int step_dispatch(nessi_batch *b, int s, bool vie, const GroupSel &sel, int n, const StepLane &ln, bool chained) {
     switch (s) {
-        case 1: return step_class_any<1>(b, vie, sel, n, ln);
-        case 2: return step_class_any<2>(b, vie, sel, n, ln);
-        case 3: return step_class_any<3>(b, vie, sel, n, ln);
-        case 4: return step_class_any<4>(b, vie, sel, n, ln);
-        case 5: return step_class_any<5>(b, vie, sel, n, ln);
-        case 6: return step_class_any<6>(b, vie, sel, n, ln);
-        case 7: return step_class_any<7>(b, vie, sel, n, ln);
-        case 8: return step_class_any<8>(b, vie, sel, n, ln);
+        case 1: return step_class_any<1>(b, vie, sel, n, ln, chained);
+        case 2: return step_class_any<2>(b, vie, sel, n, ln, chained);
+        case 3: return step_class_any<3>(b, vie, sel, n, ln, chained);
+        case 4: return step_class_any<4>(b, vie, sel, n, ln, chained);
+        case 5: return step_class_any<5>(b, vie, sel, n, ln, chained);
+        case 6: return step_class_any<6>(b, vie, sel, n, ln, chained);
+        case 7: return step_class_any<7>(b, vie, sel, n, ln, chained);
+        case 8: return step_class_any<8>(b, vie, sel, n, ln, chained);
     }
     set_err("size1 = %d not supported (1..8)", s);
     return NESSI_ERR_ARG;
@@ -1219,10 +1232,12 @@ static int join_lanes(nessi_batch *b, int used, bool failed) {
         if (failed) {
             keep(cudaEventRecord(ln.join, ln.side));
             keep(cudaStreamWaitEvent(ln.st, ln.join, 0));
+            b->waited = true;
         }
         if (i > 0) {
             keep(cudaEventRecord(ln.done, ln.st));
             keep(cudaStreamWaitEvent(b->stream, ln.done, 0));
+            b->waited = true;
         }
     }
     if (failed) cudaGetLastError();
@@ -1269,6 +1284,7 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
             set_err("%s: forking a stream failed", name);
             rc = NESSI_ERR_CUDA;
         }
+        bool chained = used == 1 && b->chains();
         GroupSel sel;
         sel.ng = 0;
         for (size_t gi = 0; gi < b->groups.size() && rc == NESSI_OK; gi++) {
@@ -1277,7 +1293,8 @@ static int timestep_kind(nessi_batch *b, int n, bool vie, const char *name) {
                 sel.nact[sel.ng++] = nact[gi];
             }
             if (sel.ng == NESSI_GSEL || (gi + 1 == b->groups.size() && sel.ng > 0)) {
-                rc = step_dispatch(b, s, vie, sel, n, ln);
+                rc = step_dispatch(b, s, vie, sel, n, ln, chained);
+                chained = true;
                 sel.ng = 0;
             }
         }

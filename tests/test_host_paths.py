@@ -192,3 +192,39 @@ def test_the_average_is_allocated_as_a_whole(fake, nth):
     f.reset()
     b.gloc_timestep(0, 20)
     assert len(f.calls("cudaMalloc")) == 6 - nth and _launched(f, "k_gloc_final")
+
+
+# ---- chained launches ---------------------------------------------------------------------------------------
+def _chained_after_a_wait(log):
+    """The chained launches whose stream was last told to wait for another stream."""
+    last, bad = {}, []
+    for line in log:
+        w = line.split()
+        if w[0] == "cudaStreamWaitEvent":
+            last[w[1]] = line
+        elif w[0] == "launch":
+            if w[2] == "chained" and last.get(w[1], "").startswith("cudaStreamWaitEvent"):
+                bad.append(line)
+            last[w[1]] = line
+    return bad
+
+
+@pytest.mark.parametrize("shapes", [[(1, 3)], [(2, 70)], [(1, 2), (3, 2), (8, 1)], [(1, 1)] * 70 + [(2, 1)]])
+def test_the_first_launch_after_a_wait_is_plain(fake, shapes):
+    gpu, f = fake
+    b = _batch(gpu, shapes)
+    U = np.ones((42, shapes[0][0]), np.complex128)
+    b.set_U(0, U)
+    f.reset()
+    for n in (20, 21):
+        b.dyson_timestep(n)
+    for n in (22, 23):
+        b.lattice_2b_timestep(n, 2)
+    b.dyson_timestep(24)
+    b.sigma_2b_timestep(0, 24)
+    log = f.log()
+    assert not _chained_after_a_wait(log)
+    # and most launches are chained: the rule costs no more than the waits of a step
+    kinds = [x.split()[2] for x in log if x.startswith("launch")]
+    waits = sum(x.startswith("cudaStreamWaitEvent") for x in log)
+    assert kinds.count("chained") > 0.5 * len(kinds) and waits < len(kinds)
