@@ -108,6 +108,65 @@ int check_twiddle_smem(const void *kernel, int ntau, const char *name) {
     return NESSI_OK;
 }
 
+// Pinned blocks for the slices of batches, kept for the process: cudaHostAlloc and cudaFreeHost take 1.8
+// and 0.5 ms, more than the steps of a small batch.  A batch takes a block at its first slice in
+// pageable memory and gives it back, idle, when it is closed; at most STAGE_KEEP bytes wait here, and
+// nessi_gpu_finalize frees them.
+struct StageBlock {
+    char *p = nullptr;
+    size_t bytes = 0;
+};
+constexpr size_t STAGE_KEEP = 32u << 20;
+constexpr int STAGE_KEPT = 16;
+std::mutex g_stage_mutex;
+StageBlock g_stage[STAGE_KEPT];  // free blocks (p = null: no block)
+
+StageBlock take_stage(size_t bytes) {
+    StageBlock out;
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mutex);
+        StageBlock *best = nullptr;
+        for (StageBlock &f : g_stage)
+            if (f.p && f.bytes >= bytes && (!best || f.bytes < best->bytes)) best = &f;
+        if (best) {
+            std::swap(out, *best);
+            return out;
+        }
+    }
+    void *q = nullptr;
+    const size_t n = (bytes + 0xffff) / 0x10000 * 0x10000;
+    if (cudaHostAlloc(&q, n, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return out;
+    }
+    out.p = (char *)q;
+    out.bytes = n;
+    return out;
+}
+void give_stage(const StageBlock &blk) {
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mutex);
+        size_t kept = blk.bytes;
+        StageBlock *slot = nullptr;
+        for (StageBlock &f : g_stage) {
+            kept += f.bytes;
+            if (!f.p) slot = &f;
+        }
+        if (slot && kept <= STAGE_KEEP) {
+            *slot = blk;
+            return;
+        }
+    }
+    cudaFreeHost(blk.p);
+}
+void free_stages() {
+    std::lock_guard<std::mutex> lock(g_stage_mutex);
+    for (StageBlock &f : g_stage) {
+        if (f.p) cudaFreeHost(f.p);
+        f = StageBlock();
+    }
+}
+
 struct Prob {
     nessi_problem_desc d;
     int group = -1;
@@ -180,10 +239,10 @@ struct nessi_batch {
     GroupDev *d_groups = nullptr;  // the groups' device descriptors, refreshed by sync_groups
     double2 *scratch = nullptr;  // G^tv in libcntr layout during layout conversion (size1 > 1)
     long scratch_n = 0;
-    // pinned staging slots of one time-step slice each, for slices in pageable host memory (allocated
-    // at the first such call, one slice of the largest problem per slot)
+    // pinned staging slots of one time-step slice each, for slices in pageable host memory (a block is
+    // taken at the first such call, one slice of the largest problem per slot)
     static constexpr int NSTAGE = 4;
-    char *stage = nullptr;
+    StageBlock stage;
     size_t stage_bytes = 0;              // of one slot
     cudaEvent_t stage_ev[NSTAGE] = {};   // the slot's last reader
     int stage_next = 0;
@@ -255,6 +314,8 @@ GroupDev group_dev(const Group &g) {
     d.conv_sign = g.vie ? -1.0 : 1.0;
     return d;
 }
+
+constexpr size_t ERR_BYTES = 256;  // the batch's error word, in front of its descriptor table
 
 // The device table of the groups' descriptors, after any of their pointers changed
 int sync_groups(nessi_batch *b) {
@@ -779,15 +840,6 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
         set_err("SM count query failed");
         return fail(NESSI_ERR_CUDA);
     }
-    {
-        void *q = nullptr;
-        if (cudaMalloc(&q, sizeof(int)) != cudaSuccess || cudaMemset(q, 0, sizeof(int)) != cudaSuccess) {
-            set_err("cudaMalloc of the error word failed");
-            return fail(NESSI_ERR_OOM);
-        }
-        b->allocs.push_back(q);
-        b->d_err = (int *)q;
-    }
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
         set_err("stream creation failed");
         return fail(NESSI_ERR_CUDA);
@@ -829,7 +881,7 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
                 classes++;
             }
         b->lanes.resize((size_t)classes - 1);
-        bool ok = cudaEventCreateWithFlags(&b->ev_lanes, cudaEventDisableTiming) == cudaSuccess;
+        bool ok = classes == 1 || cudaEventCreateWithFlags(&b->ev_lanes, cudaEventDisableTiming) == cudaSuccess;
         for (StepLane &ln : b->lanes)
             ok = ok && cudaStreamCreateWithFlags(&ln.st, cudaStreamNonBlocking) == cudaSuccess &&
                  cudaStreamCreateWithFlags(&ln.side, cudaStreamNonBlocking) == cudaSuccess &&
@@ -899,11 +951,19 @@ int nessi_gpu_batch_create(nessi_batch **out, const nessi_problem_desc *desc, in
             return fail(NESSI_ERR_CUDA);
         }
     }
-    {
+    {   // one allocation for the error word and the descriptor table
         void *q = nullptr;
-        if (cudaMalloc(&q, b->groups.size() * sizeof(GroupDev)) != cudaSuccess) { set_err("cudaMalloc failed"); return fail(NESSI_ERR_OOM); }
+        if (cudaMalloc(&q, ERR_BYTES + b->groups.size() * sizeof(GroupDev)) != cudaSuccess) {
+            set_err("cudaMalloc of the group descriptors failed");
+            return fail(NESSI_ERR_OOM);
+        }
         b->allocs.push_back(q);
-        b->d_groups = (GroupDev *)q;
+        b->d_err = (int *)q;
+        b->d_groups = (GroupDev *)((char *)q + ERR_BYTES);
+        if (cudaMemsetAsync(q, 0, ERR_BYTES, b->stream) != cudaSuccess) {
+            set_err("clearing the error word failed");
+            return fail(NESSI_ERR_CUDA);
+        }
         const int r = sync_groups(b);
         if (r) return fail(r);
     }
@@ -924,9 +984,14 @@ int nessi_gpu_batch_destroy(nessi_batch *b) {
     if (b->ev_lanes) cudaEventDestroy(b->ev_lanes);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (void *q : b->allocs) cudaFree(q);
-    if (b->stage) cudaFreeHost(b->stage);
+    bool idle = true;  // a block that an upload may still read is not handed on
     for (cudaEvent_t e : b->stage_ev)
-        if (e) cudaEventDestroy(e);
+        if (e) {
+            idle = cudaEventSynchronize(e) == cudaSuccess && idle;
+            cudaEventDestroy(e);
+        }
+    if (b->stage.p && idle) give_stage(b->stage);
+    else if (b->stage.p) cudaFreeHost(b->stage.p);
     for (auto &k : b->kp)
         for (cudaEvent_t e : k.ev) cudaEventDestroy(e);
     if (b->side) { cudaStreamSynchronize(b->side); cudaStreamDestroy(b->side); }
@@ -948,6 +1013,7 @@ int nessi_gpu_finalize(void) {
         CK(cudaDeviceSynchronize());
     }
     g_tables_ready.clear();  // the next init or batch uploads the integration tables again
+    free_stages();
     return NESSI_OK;
 }
 
@@ -1064,29 +1130,25 @@ static double2 *mapped_host(const void *host, size_t bytes, bool written, bool *
 
 // A free staging slot of at least `bytes` (null: no pinned memory, the caller copies without one)
 static char *stage_slot(nessi_batch *b, size_t bytes, int *slot) {
-    if (!b->stage) {
+    if (!b->stage.p) {
         size_t most = 0;
         for (const Group &g : b->groups)
             most = std::max(most, (size_t)(2L * (g.ntmax + 1) + g.ntau + 1) * g.s * g.s * sizeof(double2));
-        void *q = nullptr;
-        if (cudaHostAlloc(&q, most * nessi_batch::NSTAGE, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
         for (auto &e : b->stage_ev)
             if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
                 cudaGetLastError();
-                cudaFreeHost(q);
+                e = nullptr;
                 return nullptr;
             }
-        b->stage = (char *)q;
+        b->stage = take_stage(most * nessi_batch::NSTAGE);
+        if (!b->stage.p) return nullptr;
         b->stage_bytes = most;
     }
     if (bytes > b->stage_bytes) return nullptr;
     *slot = b->stage_next;
     b->stage_next = (b->stage_next + 1) % nessi_batch::NSTAGE;
     if (cudaEventSynchronize(b->stage_ev[*slot]) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    return b->stage + *slot * b->stage_bytes;
+    return b->stage.p + *slot * b->stage_bytes;
 }
 
 // Time step tstp between a herm_matrix on the device and a host slice.  One launch moves the three

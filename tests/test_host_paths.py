@@ -228,3 +228,84 @@ def test_the_first_launch_after_a_wait_is_plain(fake, shapes):
     kinds = [x.split()[2] for x in log if x.startswith("launch")]
     waits = sum(x.startswith("cudaStreamWaitEvent") for x in log)
     assert kinds.count("chained") > 0.5 * len(kinds) and waits < len(kinds)
+
+
+# ---- staging blocks of the process ---------------------------------------------------------------------------
+def _slices(gpu, b, nt=40, ntau=16, s=2, count=6):
+    data = np.zeros((2 * (nt + 1) + ntau + 1, s, s), np.complex128)
+    for _ in range(count):
+        b.set_timestep(0, nt, data)
+        b.get_timestep(0, nt, data)
+
+
+def test_batches_in_a_row_share_a_staging_block(fake):
+    gpu, f = fake
+    f.reset()
+    for _ in range(5):
+        b = _batch(gpu, [(2, 1)])
+        _slices(gpu, b)
+        b.close()
+    assert len(f.calls("cudaHostAlloc")) == 1 and not f.calls("cudaFreeHost")
+    log = f.log()  # before it is handed on, a batch waits for the uploads that read it
+    last = max(i for i, x in enumerate(log) if x.startswith("cudaEventSynchronize"))
+    assert last > max(i for i, x in enumerate(log) if x.startswith("launch"))
+    gpu.finalize()
+    assert len(f.calls("cudaFreeHost")) == 1
+    f.reset()
+    b = _batch(gpu, [(2, 1)])
+    _slices(gpu, b)
+    assert len(f.calls("cudaHostAlloc")) == 1  # nothing is kept past finalize
+
+
+def test_batches_beside_each_other_have_blocks_of_their_own(fake):
+    gpu, f = fake
+    f.reset()
+    bs = [_batch(gpu, [(2, 1)]) for _ in range(20)]
+    for b in bs:
+        _slices(gpu, b)
+    assert len(f.calls("cudaHostAlloc")) == 20
+    for b in bs:
+        b.close()
+    assert len(f.calls("cudaFreeHost")) == 4  # 16 are kept
+    gpu.finalize()
+    assert len(f.calls("cudaFreeHost")) == 20
+
+
+def test_the_kept_blocks_are_bounded_in_bytes(fake):
+    gpu, f = fake
+    f.reset()
+    nt, ntau, s = 300, 20, 8  # a slice of 638 kB
+    bs = [_batch(gpu, [(s, 1)], nt, ntau) for _ in range(15)]
+    for b in bs:
+        _slices(gpu, b, nt, ntau, s, 1)
+    sizes = [int(x.split()[1]) for x in f.calls("cudaHostAlloc")]
+    assert len(sizes) == 15 and sizes[0] >= 4 * 16 * s * s * (2 * (nt + 1) + ntau + 1)
+    for b in bs:
+        b.close()
+    assert 15 - len(f.calls("cudaFreeHost")) == (32 << 20) // sizes[0]
+    f.reset()
+    b = _batch(gpu, [(2, 1)])  # a block that is larger than needed serves too
+    _slices(gpu, b)
+    assert not f.calls("cudaHostAlloc")
+
+
+def test_a_failed_wait_keeps_a_block_from_the_next_batch(fake):
+    gpu, f = fake
+    b = _batch(gpu, [(2, 1)])
+    _slices(gpu, b, count=1)
+    f.reset()
+    f.fail("cudaEventSynchronize", 1, 1)
+    b.close()
+    assert len(f.calls("cudaFreeHost")) == 1
+
+
+def test_creation_makes_no_more_calls_than_it_needs(fake):
+    """A batch of one size has no second pair of streams, and its error word, descriptor table and their
+    upload are one allocation and one wait."""
+    gpu, f = fake
+    _batch(gpu, [(2, 1)])
+    f.reset()
+    _batch(gpu, [(2, 1)])
+    assert len(f.calls("cudaStreamSynchronize")) == 1 and not f.calls("cudaMemset")
+    assert len(f.calls("cudaEventCreate")) == 2 and len(f.calls("cudaStreamCreate")) == 2
+    assert len(f.calls("cudaMalloc")) == 7 + 1 + 16 + 1 + 1  # problem, scratch, group, problems' and groups' tables
