@@ -347,18 +347,19 @@ int find_group(nessi_batch *b, int user_id) {
 // ---- per-size kernel launch table ----------------------------------------------------
 // Dynamic shared memory of a kernel, with the SM's L1 / shared split set to all shared: kernels of
 // the two streams of a step can share an SM only when they ask for the same split.
-// The attributes only grow and are set once per kernel and size on a device.
+// The attributes only grow and are set once per kernel and size on a device, until nessi_gpu_finalize:
+// a context that is made after it starts without them.
+std::mutex g_shared_mutex;
+std::map<std::pair<int, const void *>, size_t> g_shared;  // (device, kernel) -> bytes set
 int share_sm(const void *kernel, size_t smem) {
-    static std::mutex m;
-    static std::map<std::pair<int, const void *>, size_t> done;
     int dev = 0;
     CK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(m);
-    auto it = done.find({dev, kernel});
-    if (it != done.end() && it->second >= smem) return NESSI_OK;
+    std::lock_guard<std::mutex> lock(g_shared_mutex);
+    auto it = g_shared.find({dev, kernel});
+    if (it != g_shared.end() && it->second >= smem) return NESSI_OK;
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    done[{dev, kernel}] = smem;
+    g_shared[{dev, kernel}] = smem;
     return NESSI_OK;
 }
 
@@ -1013,6 +1014,10 @@ int nessi_gpu_finalize(void) {
         CK(cudaDeviceSynchronize());
     }
     g_tables_ready.clear();  // the next init or batch uploads the integration tables again
+    {
+        std::lock_guard<std::mutex> lock(g_shared_mutex);
+        g_shared.clear();
+    }
     free_stages();
     return NESSI_OK;
 }

@@ -309,3 +309,21 @@ def test_creation_makes_no_more_calls_than_it_needs(fake):
     assert len(f.calls("cudaStreamSynchronize")) == 1 and not f.calls("cudaMemset")
     assert len(f.calls("cudaEventCreate")) == 2 and len(f.calls("cudaStreamCreate")) == 2
     assert len(f.calls("cudaMalloc")) == 7 + 1 + 16 + 1 + 1  # problem, scratch, group, problems' and groups' tables
+
+
+# ---- kernel attributes ----------------------------------------------------------------------------------------
+def test_kernel_attributes_are_set_again_after_finalize(fake):
+    gpu, f = fake
+
+    def step():
+        b = _batch(gpu, [(4, 2)])
+        f.reset()
+        b.dyson_timestep(30)
+        sets = f.calls("cudaFuncSetAttribute")
+        b.close()
+        return sets
+    first = step()
+    assert not step()  # once per kernel and size
+    gpu.finalize()     # a context that is made after it starts without them
+    again = step()
+    assert again and (not first or again == first)
