@@ -388,9 +388,20 @@ int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
 }
 
 // Products on the repo's DMMA GEMM (kernels_gemm.cuh).  Long K, or too few 32 x 32 tiles for the
-// 148 SMs: the k-split form; else the tiled one (both sides measured at the kernels).
-bool zgemm_use_split(long M, long N, long K, int count = 1) {
-    return K >= 256 || ((M + 31) / 32) * ((N + 31) / 32) * count < 148;
+// SMs: the k-split form; else the tiled one (both sides measured at the kernels).
+bool zgemm_use_split(const nessi_batch *b, long M, long N, long K, int count = 1) {
+    return K >= 256 || ((M + 31) / 32) * ((N + 31) / 32) * count < b->nsm;
+}
+// les*adv runs beside the tv stream.  At size1 1 and 2 the stream is most of the step, and with at least six
+// tiles per SM the tiled form, which reads each operand tile once, leaves it more of the memory path.
+// Steps with the k-split form over steps with the tiled one, on 148 SMs: size1 1, n 600, ntau 400: 0.85 (76
+// tiles), 1.00 (228), 1.03 (304 to 817), 1.05 (893 and more); n 1000, ntau 200: 0.98 (480), 1.01 (800); n
+// 1000, ntau 800: 1.03 to 1.06 (480 to 1024); size1 2, n 800: 0.91 (255), 0.99 (459), 1.01 (561 to 765),
+// 1.06 (867), 1.00 (969); n 300: 0.97 (304), 0.99 (760), 1.00 (1140).  At larger size1 the recursion is the longer
+// branch: size1 3 0.95 (342), 1.00 (456 to 1083), size1 4 0.96 (440), 0.99 (792), 0.98 (1056), size1 8 0.97
+// (606), 0.98 (909), 0.99 (1010).
+bool les_adv_tiled(const nessi_batch *b, int size1, long tiles) {
+    return size1 <= 2 && b->precision == NESSI_PREC_FP64 && tiles >= 6L * b->nsm;
 }
 // chained: not the first kernel after a wait for another stream
 template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n, bool chained, cudaStream_t st) {
@@ -402,12 +413,9 @@ template <int OP> int product_launch(nessi_batch *b, const GroupSel &sel, int n,
         m.N = std::max(m.N, d.N);
         m.K = std::max(m.K, d.K);
     }
-    // les*adv runs beside the tv stream: with enough tiles for an even spread the tiled form, which
-    // reads each operand tile once, leaves the stream more of the memory path (32 x 32 lattice step 9.95
-    // ms, k-split 10.5; 256 two-band k-points 15.9 and 16.4; with 490 to 604 tiles 1 to 2 % slower)
     const long tiles = (long)((m.M + 31) / 32) * ((m.N + 31) / 32) * sel.ng;
-    const bool beside = OP == PROD_LESADV && b->precision == NESSI_PREC_FP64 && tiles >= 6 * 148;
-    if (!beside && zgemm_use_split(m.M, m.N, m.K, sel.ng)) {
+    const bool beside = OP == PROD_LESADV && les_adv_tiled(b, b->groups[sel.gid[0]].s, tiles);
+    if (!beside && zgemm_use_split(b, m.M, m.N, m.K, sel.ng)) {
         const dim3 grid((unsigned)((m.N + 7) / 8), (unsigned)((m.M + 31) / 32), (unsigned)sel.ng);
         if (sel.ng == 1) {
             LdRowK la;
@@ -479,7 +487,7 @@ int volterra_class(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) 
         const int M = (n - kmin - (blk + 1) * C::NBT) * S;  // rows after the block (largest group)
         if (M <= 0) break;
         const unsigned rt = (unsigned)((M + 31) / 32), N = (unsigned)(maxact * S), z = (unsigned)sel.ng;
-        if (blk >= 0 && zgemm_use_split(M, N, C::NR, sel.ng))
+        if (blk >= 0 && zgemm_use_split(b, M, N, C::NR, sel.ng))
             CKR(launch_chained(k_vol_trail_split<S, RET>, dim3((N + 7) / 8, rt, z), 256, 0, st, gt, sel, n, blk));
         else
             CKR(launch_chained(k_vol_trail<S, RET>, dim3((N + 31) / 32, rt, z), 128, smt, st, gt, sel, n, blk));

@@ -327,3 +327,17 @@ def test_kernel_attributes_are_set_again_after_finalize(fake):
     gpu.finalize()     # a context that is made after it starts without them
     again = step()
     assert again and (not first or again == first)
+
+
+# ---- which form of a product a step takes -------------------------------------------------------------------
+@pytest.mark.parametrize("s,cnt,tiled", [(2, 896, True), (2, 880, False),  # 16 x 56 tiles of 32 x 32, 16 x 55; the line is 6 x 148
+                                         (3, 400, False), (4, 224, False), (8, 112, False)])
+def test_les_adv_is_tiled_for_small_blocks_only(fake, s, cnt, tiled):
+    gpu, f = fake
+    n = 255
+    b = _batch(gpu, [(s, cnt)], nt=n, ntau=8)
+    f.reset()
+    b.dyson_timestep(n)
+    products = [x for x in f.calls("launch") if "k_zgemm" in x]
+    assert len(products) == 3
+    assert [("k_zgemm<1>" in x) for x in products].count(True) == int(tiled)  # <1>: Sigma^< G^A, tiled
