@@ -354,6 +354,25 @@ def mixed_companion(b, W, nt, k, fp64_value, args, world, stream):
 FLOP_KERNELS = ("ret", "les", "gemm")
 
 
+# profile of the kernel that streams the tv history, by precision (none for the FP32 copy's kernel)
+TV_PROFILE = {"fp64": "k_tv_ring_config1-ncu.md"}
+
+
+def tv_traffic_ratio(precision):
+    """DRAM bytes per algorithmic byte of the tv kernel that runs, from its ncu capture under profiles/;
+    None where that kernel has none."""
+    name = TV_PROFILE.get(precision)
+    if name is None or os.environ.get("NESSI_TV_KERNEL") == "stream":
+        return None
+    path = os.path.join(ROOT, "profiles", name)
+    if os.path.exists(path):
+        with open(path) as f:
+            for line in f:
+                if line.startswith("traffic_ratio:"):
+                    return float(line.split(":")[1])
+    return None
+
+
 def kernel_roofline(prof, prof_steps, peak_hbm, hbm_kind, peak_fp64, traffic_ratio):
     """Breakdown per kernel class and the roofline of the dominant one (largest device time):
     HBM bytes against the measured copy peak for the streaming kernels, FP64 flops against the
@@ -385,8 +404,8 @@ def kernel_roofline(prof, prof_steps, peak_hbm, hbm_kind, peak_fp64, traffic_rat
                 "traffic": (traffic_ratio * work / launches) if (traffic_ratio and launches and dom == "tv") else None,
                 "algorithmic_bytes_per_launch": work / launches if launches else None, "avg_launch_ms": avg}
         if roof["traffic"] is not None:
-            roof["traffic_note"] = ("DRAM bytes per algorithmic byte from one ncu capture of k_tv, scaled to this "
-                                    "launch's algorithmic bytes")
+            roof["traffic_note"] = ("DRAM bytes per algorithmic byte from one ncu capture of k_tv_ring, scaled to "
+                                    "this launch's algorithmic bytes")
     return breakdown, roof
 
 
@@ -557,12 +576,7 @@ def main():
     # per-kernel device times and the roofline of the dominant kernel class
     peak, peak_kind = load_peaks()
     peak_fp64 = fp64_peak_tflops()
-    traffic_ratio = None
-    tpath = os.path.join(ROOT, "profiles", "k_tv_config1-ncu.md")
-    if os.path.exists(tpath):
-        for line in open(tpath):
-            if line.startswith("traffic_ratio:"):
-                traffic_ratio = float(line.split(":")[1])
+    traffic_ratio = tv_traffic_ratio(args.precision)
     breakdown, roofline = kernel_roofline(prof, prof_steps, peak, peak_kind, peak_fp64, traffic_ratio)
     # the whole step against the HBM peak: all algorithmic bytes of the propagation over its
     # time; low where the sequential Volterra recursions set the pace
