@@ -35,8 +35,8 @@
 // ret and les, 1024 problems, n 1000: 340 us; two that share the loads 475, their sums are longer than
 // the chain).  Size1 2: two at eight columns per CTA, else one (256 problems, n 1000: 687 us, 512
 // problems 1048; built for one only: 775 and 1004).
-// 128 scalar rows: the widest triangle that fits in shared memory beside the tv stream's ring, so
-// that a step of n rows is n s / 128 launch pairs.  The kernels of a recursion are launched with
+// 128 scalar rows: the widest triangle that fits in shared memory beside the tv stream's ring (size1 <= 4, see
+// vol_beside_tv), so that a step of n rows is n s / 128 launch pairs.  The kernels of a recursion are launched with
 // programmatic stream serialization: what does not depend on the solution (triangle, near block,
 // step inverses) is staged while the previous kernel still runs.
 //
@@ -70,6 +70,23 @@ template <int S> struct VbCfg {
     // packed column-major triangle: column l (s scalar columns) holds rows (l+1) s .. NR-1
     static __device__ __forceinline__ int off(int l) { return S * (l * NR - S * (l * (l + 1) / 2)); }
 };
+// Most columns per CTA with which k_vol_block and k_tv_ring share an SM (228 KB of shared memory, 1 KB of it
+// reserved per CTA): 8 for size1 1 (219 KB for the pair), 4 for 2 (224; with 8 240), 2 for 3 (206), 1 for 4
+// (218; with 2 228.4).  From size1 5 on the ring takes all registers of the SM and there is no limit.
+// The retarded recursion keeps to it in an FP64 step with ntau >= 75 size1: with more columns a CTA its SMs wait
+// for the stream's to finish, which costs more than a second wave of CTAs.  A step in ms, with the limit and
+// with 8 (size1 4: 2) columns: size1 2, 310 problems, n 200, ntau 150 0.50 and 0.53; 1000, n 500, ntau 150 3.18
+// and 3.35; 512, n 800, ntau 500 4.65 and 5.27; size1 4, 40 problems, n 200, ntau 300 0.70 and 0.71; 150, n 500,
+// ntau 300 5.00 and 5.31; 40, n 1200, ntau 800 6.46 and 7.16.  A shorter stream has less to lose: size1 2, 310
+// problems, n 900, ntau 40 2.51 and 2.41; size1 4, 45 problems, n 200, ntau 100 0.59 and 0.53.  The lesser
+// recursion runs alone and has no limit (size1 2, 300 problems, n 800, ntau 500 3.08, limited too 3.19), nor has
+// a mixed step, whose tv kernel does not leave room in any case (3.33 with it, 3.25 without).
+template <int S> constexpr int vol_beside_tv() {
+    int wc = VbCfg<S>::WMAX;
+    if (S <= 4)
+        while (wc > 1 && (VbCfg<S>::total(wc) + TvCfg<S>::total) * 16 + 2 * 1024 > 228 * 1024) wc /= 2;
+    return wc;
+}
 // T(i, l)[a][b]
 template <int S, bool RET>
 __device__ __forceinline__ const double2 *vol_t(const GroupDev &g, int n, int i, int l, int a, int b) {

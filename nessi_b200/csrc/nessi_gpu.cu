@@ -449,15 +449,17 @@ template <int S> size_t les_start_smem(int k) {
 
 // One Volterra recursion (ret or les) of a step for the selected groups (same size1 and kind): the
 // start rows, then per block of VbCfg<S>::NBT time rows the diagonal kernel and the GEMM into the
-// later rows.  Columns per CTA of the diagonal kernel: as many as put one CTA on every SM, at most 8.
+// later rows.  Columns per CTA of the diagonal kernel: as many as put one CTA on every SM, within the limits at
+// VbCfg and vol_beside_tv.
 template <int S, bool VIE, bool RET>
 int volterra_class(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) {
     using C = VbCfg<S>;
-    int kmin = NESSI_K1MAX, kmax = 0, maxact = 0;
+    int kmin = NESSI_K1MAX, kmax = 0, maxact = 0, ntau = 0;
     long cols = 0;
     for (int i = 0; i < sel.ng; i++) {
         kmin = std::min(kmin, b->groups[sel.gid[i]].k);
         kmax = std::max(kmax, b->groups[sel.gid[i]].k);
+        ntau = std::max(ntau, b->groups[sel.gid[i]].ntau);
         maxact = std::max(maxact, sel.nact[i]);
         cols += (long)sel.nact[i] * S;
     }
@@ -472,8 +474,11 @@ int volterra_class(nessi_batch *b, const GroupSel &sel, int n, cudaStream_t st) 
         CKR(share_sm((const void *)k_les_start<S, VIE>, sm));
         CKR(launch_chained(k_les_start<S, VIE>, dim3((unsigned)maxact, (unsigned)sel.ng), 256, sm, st, gt, sel, n));
     }
+    // the retarded recursion beside a long k_tv_ring: no more than leave room for it on an SM
+    const bool beside = RET && b->precision == NESSI_PREC_FP64 && b->tv_kernel == 1 && ntau >= 75 * S;
+    const int wmax = beside ? vol_beside_tv<S>() : C::WMAX;
     int wc = 1;
-    while (wc < C::WMAX && cols > (long)wc * b->nsm) wc *= 2;
+    while (wc < wmax && cols > (long)wc * b->nsm) wc *= 2;
     const dim3 gd((unsigned)((maxact * S + wc - 1) / wc), (unsigned)sel.ng);
     const size_t smb = (size_t)C::total(wc) * sizeof(double2);
     CKR(share_sm((const void *)k_vol_block<S, VIE, RET>, (size_t)C::total(C::WMAX) * sizeof(double2)));

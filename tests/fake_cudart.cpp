@@ -22,8 +22,7 @@ struct HostRange { char *p; size_t n; int access; };
 static std::vector<HostRange> g_host;  // pinned ranges
 static int g_next = 1;
 static cudaError_t g_last = cudaSuccess;
-static std::string g_pushed;
-static std::vector<cudaStream_t> g_push_stream;
+static std::vector<std::pair<cudaStream_t, dim3>> g_push;
 
 static int id_of(const void *p) { return p ? g_ids[(void *)p] : 0; }
 // a call that fails by plan has "failed" in front of its name in the log
@@ -72,21 +71,23 @@ void __cudaRegisterFunction(void **, const char *host, char *, const char *name,
     free(d);
 }
 void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
-unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, struct CUstream_st *st) { g_push_stream.push_back(st); return 0; }
-cudaError_t __cudaPopCallConfiguration(dim3 *, dim3 *, size_t *, void *st) {
-    *(cudaStream_t *)st = g_push_stream.back();
-    g_push_stream.pop_back();
+unsigned __cudaPushCallConfiguration(dim3 grid, dim3, size_t, struct CUstream_st *st) { g_push.push_back({st, grid}); return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *, size_t *, void *st) {
+    *(cudaStream_t *)st = g_push.back().first;
+    *grid = g_push.back().second;
+    g_push.pop_back();
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t st) {
-    return call("launch", num(id_of(st)) + " plain " + g_kernels[f]);
+static std::string shape(dim3 g) { return " grid " + num(g.x) + " " + num(g.y) + " " + num(g.z); }
+cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **, size_t, cudaStream_t st) {
+    return call("launch", num(id_of(st)) + " plain " + g_kernels[f] + shape(grid));
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) {
     bool chained = false;
     for (unsigned i = 0; i < c->numAttrs; i++)
         chained = chained || (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
                               c->attrs[i].val.programmaticStreamSerializationAllowed);
-    return call("launch", num(id_of(c->stream)) + (chained ? " chained " : " plain ") + g_kernels[f]);
+    return call("launch", num(id_of(c->stream)) + (chained ? " chained " : " plain ") + g_kernels[f] + shape(c->gridDim));
 }
 cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v) { return call("cudaFuncSetAttribute", num(a) + " " + num(v) + " " + g_kernels[f]); }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes *a, const void *) { memset(a, 0, sizeof *a); return call("cudaFuncGetAttributes"); }

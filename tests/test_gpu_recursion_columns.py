@@ -3,8 +3,9 @@ do not reach, against the oracle at the parity bar of the repository (1e-10 of t
 the rounding of the longest sum here).
 
 Columns: a CTA of the diagonal kernel takes wc = 1, 2, 4 or 8 columns, doubling while there are more than
-wc x 148 of them (size1 3 and 4: at most 2, larger: at most 4).  The counts here reach every wc, two columns per
-warp (size1 2, wc 8), CTAs whose columns belong to several problems, and a last CTA with columns missing."""
+wc x 148 of them (size1 3 and 4: at most 2, larger: at most 4; less for the retarded one beside a long tau grid).
+The counts here reach every wc, two columns per warp (size1 2, wc 8), CTAs whose columns belong to several
+problems, and a last CTA with columns missing; the long tau grid has a case of its own."""
 import numpy as np
 import pytest
 
@@ -13,7 +14,7 @@ from nessi_b200 import herm_matrix
 from test_gpu_recursion import _history
 
 pytestmark = pytest.mark.gpu
-TOL = 1e-10
+TOL, TOL_MIXED = 1e-10, 1e-8  # the repository's bars
 BETA, H_, NTAU = 4.0, 0.04, 8
 
 
@@ -21,7 +22,7 @@ def _rows(s):
     return 4 * (32 // s)  # time rows of a block
 
 
-def _run(oracle, s, k, n, cnt, check, vie2=False):
+def _run(oracle, s, k, n, cnt, check, vie2=False, mixed=False):
     """One late step n of cnt problems; the problems in `check` have data of their own, the others share
     one set."""
     from nessi_b200 import gpu
@@ -29,7 +30,8 @@ def _run(oracle, s, k, n, cnt, check, vie2=False):
     Sig = make_sigma(oracle, rng, n, NTAU, s, -1, BETA, H_)
     own = {p: (make_sigma(oracle, rng, n, NTAU, s, -1, BETA, H_) if vie2 else make_H(rng, n, s, H_), _history(rng, n, s))
            for p in list(check) + [-1]}
-    b = gpu.Batch([dict(nt=n, ntau=NTAU, size1=s, sig=-1, solve_order=k, beta=BETA, h=H_, mu=0.1)] * cnt)
+    b = gpu.Batch([dict(nt=n, ntau=NTAU, size1=s, sig=-1, solve_order=k, beta=BETA, h=H_, mu=0.1)] * cnt,
+                  gpu.PREC_MIXED if mixed else gpu.PREC_FP64)
     if vie2:
         b.set_F(0, Sig, Sig)  # hermitian: Fcc = F
     else:
@@ -56,7 +58,7 @@ def _run(oracle, s, k, n, cnt, check, vie2=False):
         got = herm_matrix(n, NTAU, s, -1)
         b.get_G(p, got)
         for comp, v in component_errors(got, ref, n, n).items():
-            assert v < TOL, (p, comp, v)
+            assert v < (TOL_MIXED if mixed else TOL), (p, comp, v)
     b.close()
 
 
@@ -80,6 +82,19 @@ def test_dyson_columns(oracle, s, cnt):
 @pytest.mark.parametrize("s,cnt", [(1, 603), (2, 299), (3, 101), (4, 75), (5, 61), (8, 38)])
 def test_vie2_columns(oracle, s, cnt):
     _run(oracle, s, 5, 5 + _rows(s) + 2, cnt, _some(s, cnt), vie2=True)
+
+
+@pytest.mark.parametrize("s,cnt,vie2", [(2, 299, False), (2, 299, True), (4, 75, False), (1, 603, False)])
+def test_columns_of_a_mixed_step(oracle, s, cnt, vie2):
+    _run(oracle, s, 5, 5 + _rows(s) + 2, cnt, _some(s, cnt), vie2, mixed=True)
+
+
+@pytest.mark.parametrize("s,ntau,cnt", [(2, 150, 299), (4, 300, 40)])  # wc 4 for ret and 8 for les, 1 and 2
+def test_columns_beside_a_long_tau_grid(oracle, monkeypatch, s, ntau, cnt):
+    import test_gpu_recursion
+    monkeypatch.setattr(test_gpu_recursion, "NTAU", ntau)
+    monkeypatch.setitem(globals(), "NTAU", ntau)
+    _run(oracle, s, 5, 5 + _rows(s) + 2, cnt, _some(s, cnt))
 
 
 @pytest.mark.parametrize("vie2", [False, True])

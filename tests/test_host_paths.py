@@ -341,3 +341,23 @@ def test_les_adv_is_tiled_for_small_blocks_only(fake, s, cnt, tiled):
     products = [x for x in f.calls("launch") if "k_zgemm" in x]
     assert len(products) == 3
     assert [("k_zgemm<1>" in x) for x in products].count(True) == int(tiled)  # <1>: Sigma^< G^A, tiled
+
+
+@pytest.mark.parametrize("s,ntau,cnt,mixed,ret,les", [
+    (1, 75, 1200, False, 150, 150),                  # 8 columns a CTA: 219 KB with the tv ring on an SM
+    (2, 150, 290, False, 145, 145), (2, 150, 300, False, 150, 75),  # 4 at most for ret, 8 for les
+    (2, 149, 300, False, 75, 75),                    # a short stream
+    (2, 150, 300, True, 75, 75),                     # no ring in a mixed step
+    (3, 225, 52, False, 78, 78),                     # 2
+    (4, 300, 37, False, 148, 148), (4, 300, 40, False, 160, 80), (4, 299, 40, False, 80, 80),  # 1 and 2
+    (5, 375, 61, False, 77, 77), (8, 600, 38, False, 76, 76)])      # 4: the ring has the SM to itself
+def test_the_retarded_recursion_leaves_room_for_the_tv_ring(fake, s, ntau, cnt, mixed, ret, les):
+    gpu, f = fake
+    b = gpu.Batch([dict(nt=30, ntau=ntau, size1=s, sig=-1, solve_order=5, beta=2.0, h=0.1)] * cnt,
+                  gpu.PREC_MIXED if mixed else gpu.PREC_FP64)
+    _open.append(b)
+    f.reset()
+    b.dyson_timestep(30)
+    grids = {kind: {int(x.split(" grid ")[1].split()[0]) for x in f.calls("launch")
+                    if "k_vol_block<%d, false, %s>" % (s, kind) in x} for kind in ("true", "false")}
+    assert grids == {"true": {ret}, "false": {les}}
