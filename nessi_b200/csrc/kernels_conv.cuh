@@ -17,7 +17,9 @@
 // the right-hand blocks are loaded once for the JW rows and a column access A^<(j.., m) is a whole
 // line.  Measured on a B200, 16 problems of size1 2, n 600, ntau 400 (ret / tv / les, us): a thread per
 // output element, each summing alone, took 333 / 453 / 987; this form 81 / 90 / 228 (3.0 TB/s of
-// operand bytes; one problem 137 us in all, before 1150).
+// operand bytes; one problem 137 us in all, before 1150).  The other sizes, 16 problems, n 200, ntau 100, all
+// three, before and now: size1 1 466, 86; 3 825, 168; 4 865, 290; 5 1151, 601; 6 1338, 913; 7 1972, 1269; 8 3659,
+// 2209; n 600, ntau 300: size1 5 5532, 5009 (16), size1 8 17947, 11300 (10 problems).
 #pragma once
 #include "device_common.cuh"
 

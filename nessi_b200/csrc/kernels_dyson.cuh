@@ -118,7 +118,6 @@ __device__ __forceinline__ void prep_group(const GroupDev &g, int n, int d_lo, i
     // tv coefficients, j = 0..n-1
     for (long e = tid; e < (long)n * s2; e += nth) {
         int j = (int)(e / s2), ab = (int)(e % s2), a = ab / S, b = ab % S;
-        (void)a; (void)b;
         double2 v = cscale(g.sret[(tri(n) + j) * s2 + ab], (VIE ? -h : h) * greg_w(k, n, j));
         if (!VIE && j >= n - k - 1 && a == b) v = csub(v, cmk(0.0, bd_w(k, n - j) / h));
         g.tvcoef[(long)j * s2 + ab] = v;

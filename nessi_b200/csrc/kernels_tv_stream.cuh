@@ -3,7 +3,7 @@
 // (cp.async.bulk global -> shared, completion counted in bytes on an mbarrier):
 //   Q(tau) = sum_{j<n} a_j G^tv(j, tau) + Cmat(tau) [+ Q^tv(n, tau) for VIE2]
 //   G^tv(n, tau) = Minv_les[n] Q(tau)
-// a_j = tvcoef (k_prep_group), Cmat = K_n Gmat_all (the Matsubara integral as one group GEMM).
+// a_j = tvcoef (k_prep), Cmat = K_n Gmat_all (the Matsubara integral as one group GEMM).
 //
 // The history stream is the HBM-bound part of a time step.  The default form (k_tv_ring) gives every
 // warp a ring of its own, filled by cp.async.  Here one persistent CTA per SM keeps up to five stages
